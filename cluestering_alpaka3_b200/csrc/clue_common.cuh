@@ -225,6 +225,23 @@ CLUE_HD int32_t get_bin(float coord, float mn, float mx, float size, bool wrappe
 template <int N, int MT>
 struct Metric;
 
+// Gap between a point and a box, and between two boxes, per dimension (0 where they overlap).
+CLUE_HD float gap1(float lo_minus, float minus_hi) { return fmaxf(fmaxf(lo_minus, minus_hi), 0.0f); }
+template <int N, class M>
+CLUE_HD float lower_point(const float* x, const float* lo, const float* hi, const float* par) {
+  float gap[N];
+#pragma unroll
+  for (int d = 0; d < N; ++d) gap[d] = gap1(fsub(lo[d], x[d]), fsub(x[d], hi[d]));
+  return M::lower_gap(gap, par);
+}
+template <int N, class M>
+CLUE_HD float lower_box(const float* alo, const float* ahi, const float* lo, const float* hi, const float* par) {
+  float gap[N];
+#pragma unroll
+  for (int d = 0; d < N; ++d) gap[d] = gap1(fsub(lo[d], ahi[d]), fsub(alo[d], hi[d]));
+  return M::lower_gap(gap, par);
+}
+
 template <int N>
 struct Metric<N, CLUE_METRIC_EUCLIDEAN> {
   static constexpr bool kRoot = true;
@@ -239,14 +256,14 @@ struct Metric<N, CLUE_METRIC_EUCLIDEAN> {
     }
     return acc;
   }
-  // Lower bound of partial(x, c) over every c in the box [lo, hi], with the same monotone
-  // rounded operations, so lower() > t implies partial(x, c) > t for every c in the box.
-  CLUE_HD static float lower(const float* x, const float* lo, const float* hi, const float*) {
+  // Lower bound of partial() from the per-dimension gaps of a point and a box or of two boxes
+  // (lower_point, lower_box), with the same monotone rounded operations: lower_gap() > t implies
+  // partial(x, c) > t for every pair of points they stand for.
+  CLUE_HD static float lower_gap(const float* gap, const float*) {
     float acc = 0.0f;
 #pragma unroll
     for (int d = N - 1; d >= 0; --d) {
-      const float gap = x[d] < lo[d] ? fsub(lo[d], x[d]) : (x[d] > hi[d] ? fsub(x[d], hi[d]) : 0.0f);
-      acc = fadd(fmul(gap, gap), acc);
+      acc = fadd(fmul(gap[d], gap[d]), acc);
     }
     return acc;
   }
@@ -265,12 +282,11 @@ struct Metric<N, CLUE_METRIC_WEIGHTED_EUCLIDEAN> {
     }
     return acc;
   }
-  CLUE_HD static float lower(const float* x, const float* lo, const float* hi, const float* w) {
+  CLUE_HD static float lower_gap(const float* gap, const float* w) {
     float acc = 0.0f;
 #pragma unroll
     for (int d = N - 1; d >= 0; --d) {
-      const float gap = x[d] < lo[d] ? fsub(lo[d], x[d]) : (x[d] > hi[d] ? fsub(x[d], hi[d]) : 0.0f);
-      acc = fadd(fmul(fmul(w[d], gap), gap), acc);
+      acc = fadd(fmul(fmul(w[d], gap[d]), gap[d]), acc);
     }
     return acc;
   }
@@ -295,12 +311,11 @@ struct Metric<N, CLUE_METRIC_PERIODIC_EUCLIDEAN> {
     return acc;
   }
   // Periodic dimensions contribute no bound; the others bound like the Euclidean metric.
-  CLUE_HD static float lower(const float* x, const float* lo, const float* hi, const float* period) {
+  CLUE_HD static float lower_gap(const float* gap, const float* period) {
     float acc = 0.0f;
 #pragma unroll
     for (int d = N - 1; d >= 0; --d) {
-      const float gap = x[d] < lo[d] ? fsub(lo[d], x[d]) : (x[d] > hi[d] ? fsub(x[d], hi[d]) : 0.0f);
-      acc = fadd(period[d] == 0.0f ? fmul(gap, gap) : 0.0f, acc);
+      acc = fadd(period[d] == 0.0f ? fmul(gap[d], gap[d]) : 0.0f, acc);
     }
     return acc;
   }
@@ -317,12 +332,11 @@ struct Metric<N, CLUE_METRIC_MANHATTAN> {
     for (int d = N - 2; d >= 0; --d) acc = fadd(fabsf(fsub(a[d], b[d])), acc);
     return acc;
   }
-  CLUE_HD static float lower(const float* x, const float* lo, const float* hi, const float*) {
+  CLUE_HD static float lower_gap(const float* gap, const float*) {
     float acc = 0.0f;
 #pragma unroll
     for (int d = N - 1; d >= 0; --d) {
-      const float gap = x[d] < lo[d] ? fsub(lo[d], x[d]) : (x[d] > hi[d] ? fsub(x[d], hi[d]) : 0.0f);
-      acc = fadd(gap, acc);
+      acc = fadd(gap[d], acc);
     }
     return acc;
   }
@@ -341,12 +355,11 @@ struct Metric<N, CLUE_METRIC_CHEBYSHEV> {
     }
     return m;
   }
-  CLUE_HD static float lower(const float* x, const float* lo, const float* hi, const float*) {
+  CLUE_HD static float lower_gap(const float* gap, const float*) {
     float m = 0.0f;
 #pragma unroll
     for (int d = 0; d < N; ++d) {
-      const float gap = x[d] < lo[d] ? fsub(lo[d], x[d]) : (x[d] > hi[d] ? fsub(x[d], hi[d]) : 0.0f);
-      m = (m < gap) ? gap : m;
+      m = (m < gap[d]) ? gap[d] : m;
     }
     return m;
   }
@@ -365,12 +378,11 @@ struct Metric<N, CLUE_METRIC_WEIGHTED_CHEBYSHEV> {
     }
     return m;
   }
-  CLUE_HD static float lower(const float* x, const float* lo, const float* hi, const float* w) {
+  CLUE_HD static float lower_gap(const float* gap, const float* w) {
     float m = 0.0f;
 #pragma unroll
     for (int d = 0; d < N; ++d) {
-      const float gap = x[d] < lo[d] ? fsub(lo[d], x[d]) : (x[d] > hi[d] ? fsub(x[d], hi[d]) : 0.0f);
-      const float t = fmul(w[d], gap);
+      const float t = fmul(w[d], gap[d]);
       m = (m < t) ? t : m;
     }
     return m;

@@ -61,25 +61,28 @@ struct Events {
 };
 constexpr int kEvChunkShift = 10;
 
-__device__ __forceinline__ int warp_min_i(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+// The lane's number, read once: left to itself the compiler reads the special register again at
+// every use in a long kernel.
+__device__ __forceinline__ int lane_id() {
+  int lane = threadIdx.x & 31;
+  asm volatile("" : "+r"(lane));
+  return lane;
 }
-__device__ __forceinline__ int warp_max_i(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+
+// Warp-wide minima and maxima, one instruction each (redux.sync; the float forms are sm_100a).
+__device__ __forceinline__ int warp_min_i(int v) { return __reduce_min_sync(0xffffffffu, v); }
+__device__ __forceinline__ int warp_max_i(int v) { return __reduce_max_sync(0xffffffffu, v); }
+__device__ __forceinline__ uint32_t warp_min_u(uint32_t v) { return __reduce_min_sync(0xffffffffu, v); }
+__device__ __forceinline__ uint32_t warp_max_u(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
+__device__ __forceinline__ float warp_min_f(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
-__device__ __forceinline__ uint32_t warp_min_u(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-__device__ __forceinline__ uint32_t warp_max_u(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+__device__ __forceinline__ float warp_max_f(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
 
 // Largest e in [0, E) with base[e] <= x.
@@ -173,10 +176,8 @@ __device__ __forceinline__ void home_bins(const EvGrid* __restrict__ g, int t, i
   for (int d = 0; d < N; ++d) hb[d] = (lt / g->stride[d]) % g->nperdim;
 }
 
-__device__ __forceinline__ int wrap_bin(int v, int npd) {
-  int b = v % npd;
-  return b < 0 ? b + npd : b;
-}
+// Tile bin of virtual bin v: lane_box keeps v within one period of the grid, [-npd, 2 npd).
+__device__ __forceinline__ int wrap_bin(int v, int npd) { return v < 0 ? v + npd : (v >= npd ? v - npd : v); }
 
 // Box of one warp's 32 records (lanes past the end repeat a record of the block): lo[N],
 // hi[N] and the largest payload, written as block b.
@@ -189,19 +190,10 @@ __device__ __forceinline__ void write_block_box(float4* __restrict__ blk, int b,
   for (int k = 0; k < 4 * BW; ++k) out[k] = 0.0f;
 #pragma unroll
   for (int d = 0; d < N; ++d) {
-    float a = x[d], z = x[d];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
-      z = fmaxf(z, __shfl_xor_sync(0xffffffffu, z, o));
-    }
-    out[d] = a;
-    out[N + d] = z;
+    out[d] = warp_min_f(x[d]);
+    out[N + d] = warp_max_f(x[d]);
   }
-  float pm = pl;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) pm = fmaxf(pm, __shfl_xor_sync(0xffffffffu, pm, o));
-  out[2 * N] = pm;
+  out[2 * N] = warp_max_f(pl);
   if (lane < BW) {
     float4 v;
 #pragma unroll
@@ -247,14 +239,10 @@ __global__ void __launch_bounds__(256) k_superblock_bbox(const float4* __restric
     }
 #pragma unroll
     for (int d = 0; d < N; ++d) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        v[d] = fminf(v[d], __shfl_xor_sync(0xffffffffu, v[d], o));
-        v[N + d] = fmaxf(v[N + d], __shfl_xor_sync(0xffffffffu, v[N + d], o));
-      }
+      v[d] = warp_min_f(v[d]);
+      v[N + d] = warp_max_f(v[N + d]);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[2 * N] = fmaxf(v[2 * N], __shfl_xor_sync(0xffffffffu, v[2 * N], o));
+    v[2 * N] = warp_max_f(v[2 * N]);
     if (lane < BW) {
       float4 out;
 #pragma unroll
@@ -312,137 +300,161 @@ __device__ __forceinline__ void smem_rec(const float4* sm, int j, float* c, floa
   payload = r[Rec<N>::kPayload];
 }
 
-// Spatial sweep of one warp over the Morton-ordered records of its search-box tiles (any
-// order: the own tile first, then the union of the warp's boxes lexicographically).  Super-blocks
-// and blocks whose bounding box lies beyond bound() for every lane, or whose largest payload is
-// below pmin for every lane, are skipped; vis(p0, p1, inbox, lexpos) gets the rest.  lexpos is
-// the tile's position in this lane's reference iteration order (lexicographic over its box).
-// With PREVISIT, p_home is the lane's own Morton position: the blocks around the warp's own
-// positions in the home tile are visited first (the nearest candidates are there, which tightens
-// bound() for the rest of the sweep) and skipped later.  Without it every tile's blocks are
-// visited in Morton order, so order-sensitive sums do not depend on how records are aligned to
-// blocks (a batch and a single event give identical results).
-template <int N, class M, bool PREVISIT, class Bound, class Visit>
+// Spatial sweep of one warp over the Morton-ordered records of its search-box tiles: the own tile
+// first, then the union of the warp's boxes.  vis(p0, p1, need, rank) gets every 32-record block that
+// some lane may need: the lane's box holds the tile, the block's box lower bound is within bound()
+// and its largest payload reaches pmin.  rank is the tile's position in the union of the boxes,
+// lexicographically: the order of two tiles of a lane's box in the reference's iteration.
+//
+// The tests are bound by instruction issue, so they are spread over the lanes: lane l looks up
+// tile l of the union (32 at a time) and tests block l of a super-block (1024 records) against the
+// warp's box, its largest bound and its smallest pmin; only blocks that pass get the test of every
+// lane against its own point.  (Testing every block by every lane took 30 tests of about 30
+// instructions per warp of the calorimeter batch's nearest-higher search, where 7.6 blocks are
+// visited.)
+//
+// With NEAREST, p_home is the lane's own Morton position: the blocks of the warp's own positions
+// come first, then the blocks of a super-block in the order of their distance from the warp's
+// box, and (up to three dimensions) the tiles next to the home tile before the others, so that
+// bound() shrinks early.  Without it every tile's blocks are visited in Morton order, so
+// order-sensitive sums do not depend on how records are aligned to blocks (a batch and a single
+// event give identical results).
+template <int N, class M, bool NEAREST, class Bound, class Visit>
 __device__ __forceinline__ void spatial_sweep(const KParams& kp, const EvGrid* __restrict__ g,
                                               const int32_t* __restrict__ off, const int* hb, const int* lo,
                                               const int* hi, bool valid, const float* x,
                                               const float4* __restrict__ blk, const float4* __restrict__ sblk,
                                               float pmin, int p_home, Bound&& bound, Visit&& vis) {
   constexpr int BW = Blk<N>::kWords;
-  const int ph_lo = warp_min_i(valid ? p_home : INT_MAX);
-  const int ph_hi = warp_max_i(valid ? p_home : INT_MIN);
-  int skip_lo = 1, skip_hi = 0;  // home-tile blocks already visited
+  const int lane = lane_id();
+  const int ph_lo = NEAREST ? warp_min_i(valid ? p_home : INT_MAX) : 0;
+  const int ph_hi = NEAREST ? warp_max_i(valid ? p_home : INT_MIN) : 0;
   int wl[N], wh[N];
+  float hlo[N], hhi[N];  // box of the warp's own points
 #pragma unroll
   for (int d = 0; d < N; ++d) {
     wl[d] = warp_min_i(valid ? lo[d] : INT_MAX);
     wh[d] = warp_max_i(valid ? hi[d] : INT_MIN);
+    hlo[d] = warp_min_f(valid ? x[d] : INFINITY);
+    hhi[d] = warp_max_f(valid ? x[d] : -INFINITY);
   }
-  int64_t ext[N];
-  {
-    int64_t m = 1;
-#pragma unroll
-    for (int d = N - 1; d >= 0; --d) {
-      ext[d] = m;
-      m *= (int64_t)(hi[d] - lo[d] + 1);
-    }
-  }
-  // one tile of the search boxes: its super-blocks and blocks that some lane may need
-  auto visit_tile = [&](const int* v, bool is_home_tile) {
+  // one non-empty tile [pb, pe): its super-blocks and blocks that some lane may need
+  auto visit_tile = [&](const int* v, int rank, int pb, int pe, bool home_tile) {
     bool inbox = valid;
-    int u = g->tile_base;
-    int64_t lexpos = 0;
 #pragma unroll
-    for (int d = 0; d < N; ++d) {
-      inbox = inbox && v[d] >= lo[d] && v[d] <= hi[d];
-      u += g->stride[d] * wrap_bin(v[d], g->nperdim);
-      lexpos += (int64_t)(v[d] - lo[d]) * ext[d];
-    }
+    for (int d = 0; d < N; ++d) inbox = inbox && v[d] >= lo[d] && v[d] <= hi[d];
     if (!__any_sync(0xffffffffu, inbox)) return;
-    const int pb = off[u], pe = off[u + 1];
-    if (pb >= pe) return;
-    const bool home_tile = PREVISIT && is_home_tile;
-    if (home_tile && ph_lo <= ph_hi) {
-      skip_lo = max(pb >> 5, (ph_lo >> 5) - 1);
-      skip_hi = min((pe - 1) >> 5, (ph_hi >> 5) + 1);
-      for (int b = skip_lo; b <= skip_hi; ++b) {
-        const int q0 = max(pb, b << 5), q1 = min(pe, (b + 1) << 5);
-        bool need = inbox;
-        if (kp.lb_ok) {
-          float bb[4 * BW];
-          load_box<N>(blk, b, bb);
-          need = need && M::lower(x, bb, bb + N, kp.mpar) <= bound() && bb[2 * N] >= pmin;
-        }
-        if (__any_sync(0xffffffffu, need)) vis(q0, q1, need, lexpos);
-      }
-    }
-    for (int sbk = pb >> 10; sbk <= (pe - 1) >> 10; ++sbk) {
-      if (kp.lb_ok) {
+    const float rmin = warp_min_f(inbox ? pmin : INFINITY);
+    const int bf = pb >> 5, bl = (pe - 1) >> 5;
+    const int sf = bf >> 5, ns = (bl >> 5) - sf + 1;
+    int s = NEAREST && home_tile ? ph_lo >> 10 : sf;  // the super-block of the own points first
+    for (int k = 0; k < ns; ++k, s = s + 1 == sf + ns ? sf : s + 1) {
+      const float bmax = warp_max_f(inbox ? bound() : -INFINITY);
+      if (kp.lb_ok && ns > 1) {
         float bb[4 * BW];
-        load_box<N>(sblk, sbk, bb);
-        const bool need = inbox && M::lower(x, bb, bb + N, kp.mpar) <= bound() && bb[2 * N] >= pmin;
-        if (!__any_sync(0xffffffffu, need)) continue;
+        load_box<N>(sblk, s, bb);
+        if (!(lower_box<N, M>(hlo, hhi, bb, bb + N, kp.mpar) <= bmax && bb[2 * N] >= rmin)) continue;
       }
-      const int sp0 = max(pb, sbk << 10), sp1 = min(pe, (sbk + 1) << 10);
-      for (int b = sp0 >> 5; b <= (sp1 - 1) >> 5; ++b) {
-        if (home_tile && b >= skip_lo && b <= skip_hi) continue;
+      const int bi = (s << 5) + lane;
+      bool c = bi >= bf && bi <= bl;
+      float lb = 0.0f;
+      if (kp.lb_ok && c) {
+        float bb[4 * BW];
+        load_box<N>(blk, bi, bb);
+        lb = lower_box<N, M>(hlo, hhi, bb, bb + N, kp.mpar);
+        c = lb <= bmax && bb[2 * N] >= rmin;
+      }
+      if (NEAREST && home_tile && bi >= ph_lo >> 5 && bi <= ph_hi >> 5) lb = -1.0f;
+      unsigned mask = __ballot_sync(0xffffffffu, c);
+      while (mask) {
+        int src;
+        if (NEAREST) {
+          const float near = warp_min_f(c ? lb : INFINITY);
+          if (kp.lb_ok && near > warp_max_f(inbox ? bound() : -INFINITY)) break;  // so are the rest
+          src = __ffs(__ballot_sync(0xffffffffu, c && lb == near)) - 1;
+          c = c && lane != src;
+          mask &= ~(1u << src);
+        } else {
+          src = __ffs(mask) - 1;
+          mask &= mask - 1;
+        }
+        const int b = (s << 5) + src;
         bool need = inbox;
         if (kp.lb_ok) {
           float bb[4 * BW];
           load_box<N>(blk, b, bb);
-          need = need && M::lower(x, bb, bb + N, kp.mpar) <= bound() && bb[2 * N] >= pmin;
+          need = need && lower_point<N, M>(x, bb, bb + N, kp.mpar) <= bound() && bb[2 * N] >= pmin;
         }
-        if (!__any_sync(0xffffffffu, need)) continue;
-        vis(max(sp0, b << 5), min(sp1, (b + 1) << 5), need, lexpos);
+        if (__any_sync(0xffffffffu, need)) vis(max(pb, b << 5), min(pe, (b + 1) << 5), need, rank);
       }
     }
   };
-  visit_tile(hb, true);
-  int v[N];
-  if (PREVISIT && N <= 3) {
-    // the other tiles ring by ring around the home tile (nearest first, so the bound shrinks
-    // early and far blocks are skipped), lexicographic inside a ring
-    int R = 0;
+  // Lane l's tile v (in_batch: whether it has one): looked up by all lanes at once, then visited in
+  // lane order.
+  auto visit_batch = [&](const int* v, bool in_batch, bool home_tile) {
+    int u = g->tile_base, rank = 0;
 #pragma unroll
-    for (int d = 0; d < N; ++d) R = max(R, max(hb[d] - wl[d], wh[d] - hb[d]));
-    for (int r = 1; r <= R; ++r) {
-#pragma unroll
-      for (int d = 0; d < N; ++d) v[d] = wl[d];
-      while (true) {
-        int ring = 0;
-#pragma unroll
-        for (int d = 0; d < N; ++d) ring = max(ring, abs(v[d] - hb[d]));
-        if (ring == r) visit_tile(v, false);
-        int d = N - 1;
-        for (; d >= 0; --d) {
-          if (v[d] < wh[d]) {
-            ++v[d];
-            break;
-          }
-          v[d] = wl[d];
-        }
-        if (d < 0) break;
-      }
+    for (int d = 0; d < N; ++d) {
+      u += g->stride[d] * wrap_bin(v[d], g->nperdim);
+      rank = rank * (wh[d] - wl[d] + 1) + (v[d] - wl[d]);
     }
-  } else {
-    // the other tiles of the union box lexicographically
-#pragma unroll
-    for (int d = 0; d < N; ++d) v[d] = wl[d];
-    while (true) {
-      bool is_home = true;
-#pragma unroll
-      for (int d = 0; d < N; ++d) is_home = is_home && v[d] == hb[d];
-      if (!is_home) visit_tile(v, false);
-      int d = N - 1;
-      for (; d >= 0; --d) {
-        if (v[d] < wh[d]) {
-          ++v[d];
-          break;
-        }
-        v[d] = wl[d];
-      }
-      if (d < 0) break;
+    int pb = 0, pe = 0;
+    if (in_batch) {
+      pb = off[u];
+      pe = off[u + 1];
     }
+    for (unsigned m = __ballot_sync(0xffffffffu, pb < pe); m; m &= m - 1) {
+      const int src = __ffs(m) - 1;
+      int tv[N];
+#pragma unroll
+      for (int d = 0; d < N; ++d) tv[d] = __shfl_sync(0xffffffffu, v[d], src);
+      visit_tile(tv, __shfl_sync(0xffffffffu, rank, src), __shfl_sync(0xffffffffu, pb, src),
+                 __shfl_sync(0xffffffffu, pe, src), home_tile);
+    }
+  };
+  visit_batch(hb, lane == 0, true);
+  int done_ring = 0;  // tiles up to this ring around the home tile are done
+  if (NEAREST && N <= 3) {
+    int v[N], id = lane;
+    bool in = true, home = true;
+#pragma unroll
+    for (int d = N - 1; d >= 0; --d) {
+      v[d] = hb[d] - 1 + id % 3;
+      id /= 3;
+      in = in && v[d] >= wl[d] && v[d] <= wh[d];
+      home = home && v[d] == hb[d];
+    }
+    visit_batch(v, in && id == 0 && !home, false);
+    done_ring = 1;
+  }
+  // the other tiles of the union box lexicographically, 32 at a time
+  int64_t total = 1;
+  bool rest = false;
+#pragma unroll
+  for (int d = 0; d < N; ++d) {
+    total *= wh[d] - wl[d] + 1;
+    rest = rest || hb[d] - wl[d] > done_ring || wh[d] - hb[d] > done_ring;
+  }
+  if (!rest) return;
+  for (int64_t base = 0; base < total; base += 32) {
+    int64_t id = base + lane;
+    const bool in = id < total;
+    int v[N], ring = 0;
+#pragma unroll
+    for (int d = N - 1; d >= 0; --d) {
+      const int ext = wh[d] - wl[d] + 1;
+      if (d == 0) {
+        v[d] = wl[d] + (int)(in ? id : 0);
+      } else if (total <= INT_MAX) {
+        v[d] = wl[d] + (int)((uint32_t)id % (uint32_t)ext);
+        id = (uint32_t)id / (uint32_t)ext;
+      } else {
+        v[d] = wl[d] + (int)(id % ext);
+        id /= ext;
+      }
+      ring = max(ring, abs(v[d] - hb[d]));
+    }
+    visit_batch(v, in && ring > done_ring, false);
   }
 }
 
@@ -470,7 +482,7 @@ __device__ __forceinline__ void scan_blocks(const KParams& kp, const float4* __r
         buf[4 * k + 2] = v.z;
         buf[4 * k + 3] = v.w;
       }
-      const float lb = M::lower(x, buf, buf + N, kp.mpar);
+      const float lb = lower_point<N, M>(x, buf, buf + N, kp.mpar);
       need = need && (strict ? lb < bound : lb <= bound) && buf[2 * N] >= pmin;
     }
     if (__any_sync(0xffffffffu, need)) inner(j, je);
@@ -1236,23 +1248,24 @@ __device__ bool staged_sweep(const EvGrid* __restrict__ g, const int32_t* __rest
 struct ChunkHome {
   int t;
   const EvGrid* g;
-  int pos;
+  int p;  // the thread's slot of the tile's home order (the chunk's first slot when not valid)
   bool valid;
 };
 
 __device__ __forceinline__ bool chunk_home(const KParams& kp, Events ev, const int32_t* __restrict__ off,
-                                           const int32_t* __restrict__ ord, const int32_t* __restrict__ chunk_tile,
+                                           const int32_t* __restrict__ chunk_tile,
                                            const uint32_t* __restrict__ chunk_off,
                                            const uint32_t* __restrict__ chunk_total, ChunkHome& h) {
   const int w = blockIdx.x;
   if (w >= (int)*chunk_total) return false;
   h.t = chunk_tile[w];
-  h.g = ev.eg + find_event(ev.tile, kp.n_events, h.t);
   const int beg = off[h.t];
+  // slots are event-major: the tile's first one lies among its event's points
+  h.g = ev.eg + event_of(ev.pt, ev.chunk_ev, kp.n_events, beg);
   const int start = (w - (int)chunk_off[h.t]) * kChunk;
   const int cnt = min(kChunk, off[h.t + 1] - beg - start);
   h.valid = (int)threadIdx.x < cnt;
-  h.pos = ord[beg + start + (h.valid ? (int)threadIdx.x : 0)];
+  h.p = beg + start + (h.valid ? (int)threadIdx.x : 0);
   return true;
 }
 
@@ -1274,8 +1287,8 @@ __global__ void __launch_bounds__(kTileThreads) k_density(const KParams kp, Even
   constexpr int W = Rec<N>::kWords;
   __shared__ StageSmem<N> sm;
   ChunkHome h;
-  if (!chunk_home(kp, ev, off, ord, chunk_tile, chunk_off, chunk_total, h)) return;
-  const int pos = h.pos;
+  if (!chunk_home(kp, ev, off, chunk_tile, chunk_off, chunk_total, h)) return;
+  const int pos = ord[h.p];
   const bool valid = h.valid;
   float x[N], wi;
   load_rec<N>(rec_w, pos, x, wi);
@@ -1328,79 +1341,72 @@ __global__ void __launch_bounds__(kTileThreads) k_density(const KParams kp, Even
 // (or than dm) or holds no density reaching the lane's.  TIE == CLUE_TIE_RHO_INDEX resolves equal
 // distances by higher rho, then lower index.
 
+// A block is visited in one of two forms.  Where few lanes need it, it is taken home by home with
+// a candidate per lane: one distance per lane, one vote, and the few candidates that pass settle
+// the home's update.  Otherwise it is taken candidate by candidate with a home per lane, without
+// branches: every lane keeps the two smallest keys of the block, a key being the metric value's
+// bits with the candidate's number in place of the lowest five.  The smallest key names the nearest
+// candidate unless the two are within one step of the shortened value (or the best so far is): such
+// lanes, and those whose nearest candidate has their own density, take the first form.
+// (On 512 events of the calorimeter batch a warp visits 3.3 blocks that 23 lanes need on average and
+// 4.4 that 2.6 lanes need.)
+// Bound by instruction issue (68% active).  A form with a vote and an update branch per candidate
+// pair and lane groups for the blocks few lanes need took 7000 instructions a warp, this one 3200:
+// 3.92 -> 2.00 ms on the 4096-event batch, 2.20 -> 1.10 ms on 4M 3-D points, 0.366 -> 0.193 ms on
+// 1M 2-D points.  split_lanes 4 / 8 / 12 / 16 gives 2.05 / 2.00 / 2.01 / 2.06 ms and 1.21 / 1.10 /
+// 1.08 / 1.09 ms on the first two.
 template <int N, int MT, int TIE>
 __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileThreads) k_nearest_higher(
-    const KParams kp, Events ev, const int32_t* __restrict__ off, const int32_t* __restrict__ ord,
-    const int32_t* __restrict__ chunk_tile, const uint32_t* __restrict__ chunk_off,
-    const uint32_t* __restrict__ chunk_total, const float4* __restrict__ rec_r, const float4* __restrict__ rec_m,
-    const int32_t* __restrict__ mq, const float4* __restrict__ blk, const float4* __restrict__ sblk,
-    const int32_t* __restrict__ minv, const int32_t* __restrict__ perm, int32_t* __restrict__ nh_s,
+    const KParams kp, Events ev, const int32_t* __restrict__ off, const int32_t* __restrict__ chunk_tile,
+    const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ chunk_total,
+    const float4* __restrict__ rec_m, const int32_t* __restrict__ mq, const float4* __restrict__ blk,
+    const float4* __restrict__ sblk, const int32_t* __restrict__ perm, int32_t* __restrict__ nh_s,
     float* __restrict__ delta_s, DevStatus* st, int split_lanes) {
   using M = Metric<N, MT>;
   ChunkHome h;
-  if (!chunk_home(kp, ev, off, ord, chunk_tile, chunk_off, chunk_total, h)) return;
-  const int pos = h.pos;
+  if (!chunk_home(kp, ev, off, chunk_tile, chunk_off, chunk_total, h)) return;
   const bool valid = h.valid;
+  if (!__any_sync(0xffffffffu, valid)) return;
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
   float x[N], rho_i;
-  load_rec<N>(rec_r, pos, x, rho_i);
-  const int orig_i = perm[pos];
+  load_rec<N>(rec_m, h.p, x, rho_i);
   int hb[N], lo[N], hi[N];
   home_bins<N>(h.g, h.t, hb);
   lane_box<N>(kp, h.g, x, kp.dm, hb, lo, hi);
-  if (!__any_sync(0xffffffffu, valid)) return;
   const float tdm = kp.t_dm;
-  __shared__ float4 s_rec[kTileThreads / 32][32 * Rec<N>::kWords];
-  __shared__ int32_t s_q[kTileThreads / 32][32];
-  float4* sm = s_rec[threadIdx.x >> 5];
-  int32_t* sq = s_q[threadIdx.x >> 5];
+  // per warp: the homes' records, and the visited block's coordinates and densities by dimension
+  __shared__ float4 s_home[kChunkWarps][32 * Rec<N>::kWords];
+  __shared__ float4 s_blk[kChunkWarps][N + 1][8];
+  store_rec<N>(s_home[warp], lane, x, rho_i);
+  __syncwarp();
   const float slack = M::kRoot ? 1.0f + 1.0f / 524288.0f : 1.0f;  // s range of one rounded distance
-  float s_best = INFINITY, rho_best = 0.0f;  // metric value of the nearest higher so far
+  float s_best = INFINITY;  // metric value of the nearest higher so far
   // Candidates beyond bnd cannot be nearer than the best so far (nor within dm): its distance
   // would round above delta.
   float bnd = tdm;
-  int nh = -1, orig_best = -1;
-  int lex_best = 0;  // search-box position of the best one's tile (below the tile count)
-  spatial_sweep<N, M, true>(kp, h.g, off, hb, lo, hi, valid, x, blk, sblk, rho_i, minv[pos],
-                      [&]() { return bnd; },
-                      [&](int p0, int p1, bool need, int64_t lexpos) {
+  int nh = -1;        // Morton position of the best so far
+  int rank_best = 0;  // position of its tile in the search boxes' iteration
+  const int pw = warp_min_i(valid ? h.p : INT_MAX);  // the warp's homes are pw + lane
+  spatial_sweep<N, M, true>(kp, h.g, off, hb, lo, hi, valid, x, blk, sblk, rho_i, h.p, [&]() { return bnd; },
+                            [&](int p0, int p1, bool need, int rank) {
     const int cnt = p1 - p0;
-    stage_block<N>(sm, rec_m, p0, cnt, sq, mq);
-    // Update of the lane's best by candidate j (called by the whole warp).  The common case, a
-    // strictly denser candidate whose distance rounds strictly below the best one's, is a
-    // predicated update; equal densities (index rule) and distances that may round to the best
-    // one's (rank rule) take the full test, entered only when some lane has such a case.
-    // Update of the lane's best by candidate j, in two parts.  consider_fast() takes the common
-    // case, a strictly denser candidate whose distance rounds strictly below the best one's, with
-    // selects, and returns whether the candidate needs the full test (equal densities: index
-    // rule; distances that may round to the best one's: rank rule).  consider_full() is that
-    // test; it may run after other candidates' updates, since the best is an exact minimum.
-    auto consider_fast = [&](int j, float s, float rho_j, bool in_block) -> bool {
-      // selects rather than a branch: the candidate's position is a shared-memory broadcast
-      const int qj = sq[j];
-      // The home point itself (equal density, never higher) is left out here: the full test
-      // would reject it only after a global load of its original index, and every pair of
-      // candidates holding some lane's own point would take that path (measured: nearest
-      // higher on calo4096 4.04 -> 3.79 ms, on the 4M 3-D points 2.40 -> 2.17 ms).
-      const bool c = need && in_block && s <= bnd && rho_j >= rho_i && qj != pos;
-      const bool fast = c && rho_j > rho_i && s * slack < s_best;
-      const float bj = fminf(tdm, s * slack);
-      s_best = fast ? s : s_best;
-      bnd = fast ? bj : bnd;
-      nh = fast ? qj : nh;
-      lex_best = fast ? (int)lexpos : lex_best;
-      if (TIE != CLUE_TIE_REFERENCE) {
-        rho_best = fast ? rho_j : rho_best;
-        orig_best = fast ? -1 : orig_best;  // -1: read from perm when a tie needs it
-      }
-      return c && !fast;
+    // candidate p0 + j becomes the lane's best
+    auto take = [&](int j, float s) {
+      s_best = s;
+      bnd = fminf(tdm, s * slack);
+      nh = p0 + j;
+      rank_best = rank;
     };
-    auto consider_full = [&](int j, float s, float rho_j) {
-      const int q = sq[j];
+    // Full test of candidate p0 + j, within bnd and not below the lane's density: equal densities
+    // are decided by the original indices, distances that may round to the best one's by the
+    // rank.  The order of the calls does not matter, since the best is an exact minimum.
+    auto consider = [&](int j, float s, float rho_j) {
+      const int p = p0 + j;
       int orig_j = -1;
       bool higher = rho_j > rho_i;
       if (!higher && rho_j > 0.0f) {
-        orig_j = __ldg(perm + q);
-        higher = orig_j > orig_i;
+        orig_j = __ldg(perm + __ldg(mq + p));
+        higher = orig_j > __ldg(perm + __ldg(mq + h.p));
       }
       if (!higher) return;
       bool better;
@@ -1413,127 +1419,114 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
         const float dist = M::finish(s), dbest = M::finish(s_best);
         if (dist != dbest || nh < 0) {
           better = dist < dbest;
-        } else if (TIE == CLUE_TIE_REFERENCE && (int)lexpos != lex_best) {
-          better = (int)lexpos < lex_best;
+        } else if (TIE == CLUE_TIE_REFERENCE && rank != rank_best) {
+          better = rank < rank_best;
         } else {
-          if (orig_j < 0) orig_j = __ldg(perm + q);
-          const int ob = TIE == CLUE_TIE_REFERENCE || orig_best < 0 ? __ldg(perm + nh) : orig_best;
-          better = TIE == CLUE_TIE_REFERENCE ? orig_j < ob
-                                             : rho_j > rho_best || (rho_j == rho_best && orig_j < ob);
+          if (orig_j < 0) orig_j = __ldg(perm + __ldg(mq + p));
+          const int orig_best = __ldg(perm + __ldg(mq + nh));
+          if (TIE == CLUE_TIE_REFERENCE) {
+            better = orig_j < orig_best;
+          } else {
+            float xb[N], rho_best;
+            load_rec<N>(rec_m, nh, xb, rho_best);
+            better = rho_j > rho_best || (rho_j == rho_best && orig_j < orig_best);
+          }
         }
       }
-      if (better) {
-        s_best = s;
-        bnd = fminf(tdm, s * slack);
-        nh = q;
-        lex_best = (int)lexpos;
-        if (TIE != CLUE_TIE_REFERENCE) {
-          rho_best = rho_j;
-          orig_best = orig_j;
-        }
-      }
+      if (better) take(j, s);
     };
-    // both parts for one candidate (called by the whole warp)
-    auto consider = [&](int j, float s, float rho_j, bool in_block) {
-      const bool slow = consider_fast(j, s, rho_j, in_block);
-      if (__any_sync(0xffffffffu, slow) && slow) consider_full(j, s, rho_j);
-    };
-    // Few lanes need this block: its candidates are split among all 32 lanes, G lanes per
-    // needing home (G = 32 / P, P >= the number of such homes, a power of two); each group finds
-    // its home's best candidate of the block, and the home lane takes it through consider().
-    // Inside one block every candidate has the same search-box position, so the best is the
-    // least (rounded distance, then [density, for TIE_RHO_INDEX] then original index), a strict
-    // total order that the group reduces exactly.
-    const unsigned nm = __ballot_sync(0xffffffffu, need);
+    // lane j's candidate; lanes past the block hold none (no density reaches theirs)
+    float c[N], r;
+    load_rec<N>(rec_m, lane < cnt ? p0 + lane : p0, c, r);
+    if (lane >= cnt) r = -INFINITY;
+    unsigned nm = __ballot_sync(0xffffffffu, need);
     const int k = __popc(nm);
-    if (k <= split_lanes) {
-      const int lg = k <= 1 ? 5 : (k <= 2 ? 4 : (k <= 4 ? 3 : (k <= 8 ? 2 : 1)));  // log2 G
-      const int lane = threadIdx.x & 31;
-      const int hs = lane >> lg;  // home slot of this lane's group
-      unsigned m = nm;
-      for (int i = 0; i < hs && m; ++i) m &= m - 1;
-      const bool gv = hs < k;
-      const int hl = gv ? __ffs(m) - 1 : 0;  // lane of the group's home
-      float xh[N];
+    // home by home: about 20 instructions a home against 10 a candidate in the other form
+    if (kp.lb_ok && k > split_lanes) {
+      __syncwarp();  // the previous block's readers are done
 #pragma unroll
-      for (int d = 0; d < N; ++d) xh[d] = __shfl_sync(0xffffffffu, x[d], hl);
-      const float rho_h = __shfl_sync(0xffffffffu, rho_i, hl);
-      const float bnd_h = __shfl_sync(0xffffffffu, bnd, hl);
-      const int orig_h = __shfl_sync(0xffffffffu, orig_i, hl);
-      const int pos_h = __shfl_sync(0xffffffffu, pos, hl);
-      // a before b (both higher than the home, same tile)
-      auto less = [&](float sa, float ra, int ja, float sb, float rb, int jb) -> bool {
-        if (sa * slack < sb) return true;
-        if (sb * slack < sa) return false;
-        const float da = M::finish(sa), db = M::finish(sb);
-        if (da != db) return da < db;
-        if (TIE != CLUE_TIE_REFERENCE && ra != rb) return ra > rb;
-        return __ldg(perm + sq[ja]) < __ldg(perm + sq[jb]);
-      };
-      float s_loc = INFINITY, r_loc = 0.0f;
-      int j_loc = -1;
-      const int G = 1 << lg;
-      for (int j = lane & (G - 1); j < cnt; j += G) {
-        float c[N], rj;
-        smem_rec<N>(sm, j, c, rj);
-        const float sj = M::partial(xh, c, kp.mpar);
-        if (gv && sj <= bnd_h && rj >= rho_h) {
-          bool higher = rj > rho_h;
-          if (!higher && rj > 0.0f) {  // (the home point itself needs no load: never higher)
-            const int qj = sq[j];
-            higher = qj != pos_h && __ldg(perm + qj) > orig_h;
-          }
-          if (higher && (j_loc < 0 || less(sj, rj, j, s_loc, r_loc, j_loc))) {
-            s_loc = sj;
-            r_loc = rj;
-            j_loc = j;
+      for (int d = 0; d < N; ++d) reinterpret_cast<float*>(s_blk[warp][d])[lane] = c[d];
+      reinterpret_cast<float*>(s_blk[warp][N])[lane] = r;
+      __syncwarp();
+      const int self = h.p - p0;  // the home point itself (equal density) is not a candidate
+      uint32_t k1 = 0xffffffffu, k2 = 0xffffffffu;
+      for (int q = 0; 4 * q < cnt; ++q) {
+        float cc[N][4], rr[4];
+#pragma unroll
+        for (int d = 0; d <= N; ++d) {
+          const float4 v = s_blk[warp][d][q];
+          float* to = d < N ? cc[d < N ? d : 0] : rr;
+          to[0] = v.x, to[1] = v.y, to[2] = v.z, to[3] = v.w;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          float ca[N], cb[N];
+#pragma unroll
+          for (int d = 0; d < N; ++d) ca[d] = cc[d][e], cb[d] = cc[d][e + 1];
+          const float2 s2 = partial_pair<N, MT>(x, ca, cb, kp.mpar);
+#pragma unroll
+          for (int f = 0; f < 2; ++f) {
+            const int j = 4 * q + e + f;
+            const uint32_t bits = (__float_as_uint(f ? s2.y : s2.x) & ~31u) | j;
+            const uint32_t key = rr[e + f] >= rho_i && j != self ? bits : 0xffffffffu;
+            k2 = min(k2, max(k1, key));
+            k1 = min(k1, key);
           }
         }
       }
-      for (int o = G >> 1; o > 0; o >>= 1) {
-        const float s_o = __shfl_xor_sync(0xffffffffu, s_loc, o);
-        const float r_o = __shfl_xor_sync(0xffffffffu, r_loc, o);
-        const int j_o = __shfl_xor_sync(0xffffffffu, j_loc, o);
-        if (j_o >= 0 && (j_loc < 0 || less(s_o, r_o, j_o, s_loc, r_loc, j_loc))) {
-          s_loc = s_o;
-          r_loc = r_o;
-          j_loc = j_o;
+      bool slow = false;
+      if (need && k1 != 0xffffffffu) {
+        const int j = k1 & 31u;
+        float cj[N];
+#pragma unroll
+        for (int d = 0; d < N; ++d) cj[d] = reinterpret_cast<const float*>(s_blk[warp][d])[j];
+        const float s = M::partial(x, cj, kp.mpar);
+        if ((k2 >> 5) - (k1 >> 5) <= 1u)
+          slow = true;
+        else if (s <= bnd) {
+          if (reinterpret_cast<const float*>(s_blk[warp][N])[j] > rho_i && s * slack < s_best)
+            take(j, s);
+          else
+            slow = true;
         }
       }
-      const int src = need ? __popc(nm & ((1u << lane) - 1u)) << lg : 0;
-      const float s_g = __shfl_sync(0xffffffffu, s_loc, src);
-      const float r_g = __shfl_sync(0xffffffffu, r_loc, src);
-      const int j_g = __shfl_sync(0xffffffffu, j_loc, src);
-      consider(j_g >= 0 ? j_g : 0, s_g, r_g, j_g >= 0);
-      return;
+      nm = __ballot_sync(0xffffffffu, slow);
     }
-    // two candidates at a time: their metric values and densities first, then the update,
-    // entered only when some lane holds a candidate that passes the bound (the bound only
-    // shrinks between the two, and consider() checks it again)
-    for (int j = 0; j < cnt; j += 2) {
-      float ca[N], cb[N], ra, rb;
-      smem_rec<N>(sm, j, ca, ra);
-      smem_rec<N>(sm, j + 1, cb, rb);
-      // paired differences and squares pay from three dimensions on (measured)
-      const float2 s2 = N >= 3 ? partial_pair<N, MT>(x, ca, cb, kp.mpar)
-                               : make_float2(M::partial(x, ca, kp.mpar), M::partial(x, cb, kp.mpar));
-      const bool any = (s2.x <= bnd && ra >= rho_i) || (j + 1 < cnt && s2.y <= bnd && rb >= rho_i);
-      if (__any_sync(0xffffffffu, need && any)) {
-        const bool slow_a = consider_fast(j, s2.x, ra, true);
-        const bool slow_b = consider_fast(j + 1, s2.y, rb, j + 1 < cnt);
-        if (__any_sync(0xffffffffu, slow_a || slow_b)) {  // one vote for both full tests
-          if (slow_a) consider_full(j, s2.x, ra);
-          if (slow_b) consider_full(j + 1, s2.y, rb);
-        }
+    while (nm) {
+      const int hl = __ffs(nm) - 1;
+      nm &= nm - 1;
+      float xh[N], rho_h;
+      smem_rec<N>(s_home[warp], hl, xh, rho_h);
+      const float bnd_h = __shfl_sync(0xffffffffu, bnd, hl);
+      const float s = M::partial(xh, c, kp.mpar);
+      const bool ok = s <= bnd_h && r >= rho_h && p0 + lane != pw + hl;
+      unsigned om = __ballot_sync(0xffffffffu, ok);
+      if (om == 0) continue;
+      if (om & (om - 1)) {
+        // of several, those that a strictly denser one is not strictly nearer than
+        const float near = warp_min_f(ok && r > rho_h ? s : INFINITY);
+        om = __ballot_sync(0xffffffffu, ok && s <= near * slack);
       }
+      do {
+        const int j = __ffs(om) - 1;
+        om &= om - 1;
+        const float sj = __shfl_sync(0xffffffffu, s, j), rj = __shfl_sync(0xffffffffu, r, j);
+        if (lane == hl) {
+          if (rj > rho_i && sj * slack < s_best)
+            take(j, sj);
+          else
+            consider(j, sj, rj);
+        }
+      } while (om);
     }
   });
   if (valid) {
-    nh_s[pos] = nh;
+    const int pos = mq[h.p];
+    nh_s[pos] = nh >= 0 ? mq[nh] : -1;
     delta_s[pos] = nh >= 0 ? M::finish(s_best) : FLT_MAX;
   }
   const uint32_t none = __ballot_sync(0xffffffffu, valid && nh < 0);
-  if ((threadIdx.x & 31) == 0 && none) {
+  if (lane == 0 && none) {
     atomicAdd(&st->seed_candidates, (uint32_t)__popc(none));
     atomicAdd(const_cast<uint32_t*>(&h.g->seed_candidates), (uint32_t)__popc(none));
   }
@@ -1559,8 +1552,8 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
   using M = Metric<N, MT>;
   __shared__ float4 s_rec[kTileThreads / 32][32 * Rec<N>::kWords];
   ChunkHome h;
-  if (!chunk_home(kp, ev, off, ord, chunk_tile, chunk_off, chunk_total, h)) return;
-  const int pos = h.pos;
+  if (!chunk_home(kp, ev, off, chunk_tile, chunk_off, chunk_total, h)) return;
+  const int pos = ord[h.p];
   const bool valid = h.valid;
   float x[N], wi;
   load_rec<N>(rec_w, pos, x, wi);
@@ -1697,7 +1690,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
   const int startA = off[t] + (a_loc << 5);
   const int cntA = min(32, off[t + 1] - startA);
   if (cntA <= 0) return;  // whole warp: this block of the chunk is past the tile's end
-  const EvGrid* g = ev.eg + find_event(ev.tile, kp.n_events, t);
+  const EvGrid* g = ev.eg + event_of(ev.pt, ev.chunk_ev, kp.n_events, off[t]);
   const bool hv = lane < cntA;
   const int pA = startA + (hv ? lane : 0);
   float x[N], wi;
@@ -1782,7 +1775,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
       for (int b = (u == t ? a_loc + 1 : 0); b < nb; ++b) {
         float bb[4 * BW];
         load_box<N>(tblk, (int)bo[u] + b, bb);
-        const bool need = hv && M::lower(x, bb, bb + N, kp.mpar) <= tdc;
+        const bool need = hv && lower_point<N, M>(x, bb, bb + N, kp.mpar) <= tdc;
         if (!__any_sync(0xffffffffu, need)) continue;
         const int first = pb + (b << 5);
         const int cntB = min(32, pe - first);
@@ -1943,8 +1936,8 @@ __global__ void __launch_bounds__(kTileThreads) k_near_ties(
     const int32_t* __restrict__ minv, const int32_t* __restrict__ nh_s, DevStatus* st) {
   using M = Metric<N, MT>;
   ChunkHome h;
-  if (!chunk_home(kp, ev, off, ord, chunk_tile, chunk_off, chunk_total, h)) return;
-  const int pos = h.pos;
+  if (!chunk_home(kp, ev, off, chunk_tile, chunk_off, chunk_total, h)) return;
+  const int pos = ord[h.p];
   const bool valid = h.valid;
   float x[N], rho_i;
   load_rec<N>(rec_r, pos, x, rho_i);
@@ -2185,19 +2178,16 @@ void launch_density(const KParams& kp, Workspace& ws, cudaStream_t s) {
 }
 template <int N, int MT>
 void launch_nh(const KParams& kp, Workspace& ws, cudaStream_t s) {
-  // a block needed by at most this many lanes is split among all lanes (at most 16: the split
-  // gives every needing lane a group of 2 lanes or more)
+  // a block needed by at most this many lanes is split among all lanes
   const int split_lanes = std::max(0, std::min(16, (int)ws.tune_nh_split));
   if (kp.tiebreak == CLUE_TIE_RHO_INDEX)
     k_nearest_higher<N, MT, CLUE_TIE_RHO_INDEX><<<chunk_grid(kp), kTileThreads, 0, s>>>(
-        kp, events_of(ws), ws.offsets, ws.mq, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_r,
-        ws.rec_m_cur, ws.mq, ws.blk, ws.sblk, ws.minv, ws.perm, ws.nh_s, ws.delta_s, ws.status,
-        split_lanes);
+        kp, events_of(ws), ws.offsets, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_m_cur, ws.mq, ws.blk,
+        ws.sblk, ws.perm, ws.nh_s, ws.delta_s, ws.status, split_lanes);
   else
     k_nearest_higher<N, MT, CLUE_TIE_REFERENCE><<<chunk_grid(kp), kTileThreads, 0, s>>>(
-        kp, events_of(ws), ws.offsets, ws.mq, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_r,
-        ws.rec_m_cur, ws.mq, ws.blk, ws.sblk, ws.minv, ws.perm, ws.nh_s, ws.delta_s, ws.status,
-        split_lanes);
+        kp, events_of(ws), ws.offsets, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_m_cur, ws.mq, ws.blk,
+        ws.sblk, ws.perm, ws.nh_s, ws.delta_s, ws.status, split_lanes);
 }
 template <int N, int MT, int FORM>
 void launch_density_spatial_form(const KParams& kp, Workspace& ws, cudaStream_t s, float kexp) {

@@ -1,0 +1,36 @@
+"""Edges of the neighbour sweeps against the oracle, bit for bit (flat kernel): blocks of 32, super-blocks
+of 1024 records, more than 32 tiles in a search box, boxes that wrap, and many equal distances."""
+import numpy as np
+import pytest
+
+from parity_util import assert_exact, random_blobs, run_both
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ndim,n,ppbin,dc,dm", [
+    (2, 1, 128, 1.0, 1.0), (2, 31, 128, 5.0, 9.0), (2, 33, 128, 5.0, 9.0), (2, 129, 128, 5.0, 9.0),
+    (2, 9000, 3000, 1.5, 3.0),    # tiles of several super-blocks
+    (1, 5000, 2500, 0.4, 0.9),
+    (2, 3001, 8, 2.0, 60.0),      # hundreds of tiles in a box, rings beyond the neighbours
+    (3, 2500, 6, 3.0, 45.0),
+    (4, 3000, 16, 4.0, 30.0),     # no ring order above three dimensions
+    (7, 900, 4, 6.0, 12.0),
+])
+@pytest.mark.parametrize("tiebreak", ["reference", "rho_index"])
+def test_nearest_higher_edges(gpu_context, ndim, n, ppbin, dc, dm, tiebreak):
+    rng = np.random.default_rng(n + ndim)
+    c, w = random_blobs(rng, n, ndim, nblobs=min(6, n), extent=60.0, sigma=1.5)
+    assert_exact(*run_both(gpu_context, c, w, dc=dc, rhoc=2.0, dm=dm, ppbin=ppbin, tiebreak=tiebreak))
+
+
+@pytest.mark.parametrize("n,ppbin", [(700, 128), (4000, 1500)])
+@pytest.mark.parametrize("wrapped", [(), (1, 0), (1, 1)])
+def test_nearest_higher_lattice(gpu_context, n, ppbin, wrapped):
+    """Integer coordinates and weights: equal distances and equal densities in every block."""
+    rng = np.random.default_rng(n)
+    c = rng.integers(0, 25, size=(2, n)).astype(np.float32)
+    w = rng.integers(1, 4, size=n).astype(np.float32)
+    for tiebreak in ("reference", "rho_index"):
+        assert_exact(*run_both(gpu_context, c, w, dc=1.0, rhoc=2.0, dm=4.0, ppbin=ppbin, wrapped=wrapped,
+                               tiebreak=tiebreak))

@@ -159,7 +159,6 @@ std::vector<ArenaItem> arena_items(Workspace& nw, void** evtab, size_t n, size_t
       {(void**)&nw.mkeys_alt, n * 4},
       {(void**)&nw.rec_m, n * w * 16},
       {(void**)&nw.sblk, (n / 1024 + 1) * 6 * 16},
-      {(void**)&nw.ord_rho, n * 4},
       {(void**)&nw.chunk_count, (ntiles + 1) * 4},
       {(void**)&nw.chunk_tile, (n / kChunkPoints + ntiles + 1) * 4},
       {(void**)&nw.chunk_total, 16},
@@ -761,10 +760,6 @@ static clue_status read_info(Workspace& ws, const KParams& kp, cudaStream_t s, c
     set_error(std::string("device bounds check failed in ") + check_site_name(h->check_site) + ": index " +
               std::to_string(h->check_index));
     return CLUE_ERR_CUDA;
-  }
-  if (h->stage_timeout) {
-    set_error("a bulk-copy wait in the density / nearest-higher sweep timed out");
-    return CLUE_ERR_TIMEOUT;
   }
   if (h->nonfinite) {
     set_error("coordinates or weights contain NaN or Inf");
@@ -1469,10 +1464,6 @@ static clue_status batch_host_overlapped(clue_context ctx, const clue_params* pa
       set_error(std::string("device bounds check failed in ") + check_site_name(hs[c].check_site) + ": index " +
                 std::to_string(hs[c].check_index));
       return CLUE_ERR_CUDA;
-    }
-    if (hs[c].stage_timeout) {
-      set_error("a bulk-copy wait in the density / nearest-higher sweep timed out");
-      return CLUE_ERR_TIMEOUT;
     }
     if (hs[c].nonfinite) {
       set_error("coordinates or weights contain NaN or Inf");

@@ -89,7 +89,6 @@ struct DevStatus {
   uint32_t n_seeds;
   uint32_t unresolved[64];   // label rounds that left an unresolved parent chain
   uint32_t label_rounds;
-  uint32_t stage_timeout;  // a bulk-copy wait in a staged sweep gave up
   uint32_t n_clusters;     // seeds kept in the seed lists, summed over events
   // near-threshold decisions (relative tolerance kNearTol, counted by k_seeds and k_near_ties)
   uint32_t near_rhoc;      // |rho - rhoc| <= tol * rhoc
@@ -442,6 +441,33 @@ __device__ __forceinline__ float2 partial_pair(const float* x, const float* a, c
     return acc;
   } else {
     return make_float2(Metric<N, MT>::partial(x, a, mpar), Metric<N, MT>::partial(x, b, mpar));
+  }
+}
+// The same for two points whose coordinates are already paired (c[d] holds both of dimension d, x[d]
+// the one point's coordinate twice), as they come from 64-bit loads: no moves to pair registers.
+template <int N, int MT>
+__device__ __forceinline__ float2 partial_packed(const unsigned long long* x, const unsigned long long* c,
+                                                 const float* mpar) {
+  if constexpr (MT == CLUE_METRIC_EUCLIDEAN) {
+    float2 acc;
+#pragma unroll
+    for (int d = N - 1; d >= 0; --d) {
+      unsigned long long df, sq;
+      asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(df) : "l"(x[d]), "l"(c[d]));
+      asm("mul.rn.f32x2 %0, %1, %1;" : "=l"(sq) : "l"(df));
+      const float2 t = upk2(sq);
+      acc = d == N - 1 ? t : make_float2(fadd(t.x, acc.x), fadd(t.y, acc.y));
+    }
+    return acc;
+  } else {
+    float xx[N], a[N], b[N];
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+      xx[d] = upk2(x[d]).x;
+      a[d] = upk2(c[d]).x;
+      b[d] = upk2(c[d]).y;
+    }
+    return make_float2(Metric<N, MT>::partial(xx, a, mpar), Metric<N, MT>::partial(xx, b, mpar));
   }
 }
 #endif

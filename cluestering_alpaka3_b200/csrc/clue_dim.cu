@@ -23,12 +23,11 @@
 // Layout in HBM: points are reordered by tile into float4 records {coords..., payload}: by
 // ascending index inside a tile for the reference-order density, by Morton code inside a tile
 // for the spatial sweeps.  A CTA processes a chunk of 128 home points of one tile (four warps
-// of 32).  The reference-order density stages whole candidate tiles into shared memory with
-// bulk copies; the spatial sweeps stage one 32-record Morton block per warp, skip blocks whose
-// bounding box is out of reach, and read every candidate as one broadcast 16-byte
-// shared-memory load (nearest higher) or from its owner lane by shuffle (symmetric density).
+// of 32).  The reference-order density reads whole candidate tiles and sums what lies within reach
+// of the warp's homes; the spatial sweeps take one 32-record Morton block at a time, skip blocks
+// whose bounding box is out of reach, and read the candidates from shared memory (nearest higher)
+// or from their owner lanes by shuffle (symmetric density).
 #include "clue_internal.h"
-#include "clue_tma.cuh"
 
 #ifndef CLUE_NDIM
 #error "CLUE_NDIM must be defined"
@@ -41,12 +40,6 @@ constexpr int kTileThreads = 128;
 constexpr int kChunkWarps = kTileThreads / 32;
 constexpr int kChunk = kChunkPoints;  // home points per CTA in the density / nearest-higher sweeps
 static_assert(kChunkPoints == kTileThreads, "one home point per thread");
-// float4 words per staging buffer (12 KiB).  Two 16 KiB buffers held the reference-order density
-// to six CTAs per SM by shared memory; at 12 KiB it runs eight (63 registers; measured on the 1M
-// 2-D points: 0.630 -> 0.587 ms, the same bits).
-constexpr int kStageWords = 768;
-constexpr int kMaxSeg = 32;        // tile segments per staged piece
-
 struct InPtrs {
   const float* c[kMaxDim];
   const float* w;
@@ -300,11 +293,67 @@ __device__ __forceinline__ void smem_rec(const float4* sm, int j, float* c, floa
   payload = r[Rec<N>::kPayload];
 }
 
+// Tiles of the union box [wl, wh] of a warp's search boxes, lane l's tile v (in_batch: whether it has
+// one) looked up by all lanes at once; f(v, rank, pb, pe) gets the non-empty ones in lane order with
+// their records [pb, pe).  rank is the tile's lexicographic position in the union, so it orders two
+// tiles of a lane's box as the reference's iteration does.
+template <int N, class F>
+__device__ __forceinline__ void batch_tiles(const EvGrid* __restrict__ g, const int32_t* __restrict__ off,
+                                            const int* wl, const int* wh, const int* v, bool in_batch, F&& f) {
+  int u = g->tile_base, rank = 0;
+#pragma unroll
+  for (int d = 0; d < N; ++d) {
+    u += g->stride[d] * wrap_bin(v[d], g->nperdim);
+    rank = rank * (wh[d] - wl[d] + 1) + (v[d] - wl[d]);
+  }
+  int pb = 0, pe = 0;
+  if (in_batch) {
+    pb = off[u];
+    pe = off[u + 1];
+  }
+  for (unsigned m = __ballot_sync(0xffffffffu, pb < pe); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    int tv[N];
+#pragma unroll
+    for (int d = 0; d < N; ++d) tv[d] = __shfl_sync(0xffffffffu, v[d], src);
+    f(tv, __shfl_sync(0xffffffffu, rank, src), __shfl_sync(0xffffffffu, pb, src), __shfl_sync(0xffffffffu, pe, src));
+  }
+}
+
+// All tiles of the union box more than done_ring tiles away from the home tile, lexicographically.
+template <int N, class F>
+__device__ __forceinline__ void box_tiles(const EvGrid* __restrict__ g, const int32_t* __restrict__ off,
+                                          const int* hb, const int* wl, const int* wh, int done_ring, int lane,
+                                          F&& f) {
+  int64_t total = 1;
+#pragma unroll
+  for (int d = 0; d < N; ++d) total *= wh[d] - wl[d] + 1;
+  for (int64_t base = 0; base < total; base += 32) {
+    int64_t id = base + lane;
+    const bool in = id < total;
+    int v[N], ring = 0;
+#pragma unroll
+    for (int d = N - 1; d >= 0; --d) {
+      const int ext = wh[d] - wl[d] + 1;
+      if (d == 0) {
+        v[d] = wl[d] + (int)(in ? id : 0);
+      } else if (total <= INT_MAX) {
+        v[d] = wl[d] + (int)((uint32_t)id % (uint32_t)ext);
+        id = (uint32_t)id / (uint32_t)ext;
+      } else {
+        v[d] = wl[d] + (int)(id % ext);
+        id /= ext;
+      }
+      ring = max(ring, abs(v[d] - hb[d]));
+    }
+    batch_tiles<N>(g, off, wl, wh, v, in && ring > done_ring, f);
+  }
+}
+
 // Spatial sweep of one warp over the Morton-ordered records of its search-box tiles: the own tile
 // first, then the union of the warp's boxes.  vis(p0, p1, need, rank) gets every 32-record block that
 // some lane may need: the lane's box holds the tile, the block's box lower bound is within bound()
-// and its largest payload reaches pmin.  rank is the tile's position in the union of the boxes,
-// lexicographically: the order of two tiles of a lane's box in the reference's iteration.
+// and its largest payload reaches pmin.  rank: see batch_tiles.
 //
 // The tests are bound by instruction issue, so they are spread over the lanes: lane l looks up
 // tile l of the union (32 at a time) and tests block l of a super-block (1024 records) against the
@@ -389,30 +438,10 @@ __device__ __forceinline__ void spatial_sweep(const KParams& kp, const EvGrid* _
       }
     }
   };
-  // Lane l's tile v (in_batch: whether it has one): looked up by all lanes at once, then visited in
-  // lane order.
-  auto visit_batch = [&](const int* v, bool in_batch, bool home_tile) {
-    int u = g->tile_base, rank = 0;
-#pragma unroll
-    for (int d = 0; d < N; ++d) {
-      u += g->stride[d] * wrap_bin(v[d], g->nperdim);
-      rank = rank * (wh[d] - wl[d] + 1) + (v[d] - wl[d]);
-    }
-    int pb = 0, pe = 0;
-    if (in_batch) {
-      pb = off[u];
-      pe = off[u + 1];
-    }
-    for (unsigned m = __ballot_sync(0xffffffffu, pb < pe); m; m &= m - 1) {
-      const int src = __ffs(m) - 1;
-      int tv[N];
-#pragma unroll
-      for (int d = 0; d < N; ++d) tv[d] = __shfl_sync(0xffffffffu, v[d], src);
-      visit_tile(tv, __shfl_sync(0xffffffffu, rank, src), __shfl_sync(0xffffffffu, pb, src),
-                 __shfl_sync(0xffffffffu, pe, src), home_tile);
-    }
-  };
-  visit_batch(hb, lane == 0, true);
+  batch_tiles<N>(g, off, wl, wh, hb, lane == 0, [&](const int* v, int rank, int pb, int pe) {
+    visit_tile(v, rank, pb, pe, true);
+  });
+  auto other = [&](const int* v, int rank, int pb, int pe) { visit_tile(v, rank, pb, pe, false); };
   int done_ring = 0;  // tiles up to this ring around the home tile are done
   if (NEAREST && N <= 3) {
     int v[N], id = lane;
@@ -424,70 +453,13 @@ __device__ __forceinline__ void spatial_sweep(const KParams& kp, const EvGrid* _
       in = in && v[d] >= wl[d] && v[d] <= wh[d];
       home = home && v[d] == hb[d];
     }
-    visit_batch(v, in && id == 0 && !home, false);
+    batch_tiles<N>(g, off, wl, wh, v, in && id == 0 && !home, other);
     done_ring = 1;
   }
-  // the other tiles of the union box lexicographically, 32 at a time
-  int64_t total = 1;
   bool rest = false;
 #pragma unroll
-  for (int d = 0; d < N; ++d) {
-    total *= wh[d] - wl[d] + 1;
-    rest = rest || hb[d] - wl[d] > done_ring || wh[d] - hb[d] > done_ring;
-  }
-  if (!rest) return;
-  for (int64_t base = 0; base < total; base += 32) {
-    int64_t id = base + lane;
-    const bool in = id < total;
-    int v[N], ring = 0;
-#pragma unroll
-    for (int d = N - 1; d >= 0; --d) {
-      const int ext = wh[d] - wl[d] + 1;
-      if (d == 0) {
-        v[d] = wl[d] + (int)(in ? id : 0);
-      } else if (total <= INT_MAX) {
-        v[d] = wl[d] + (int)((uint32_t)id % (uint32_t)ext);
-        id = (uint32_t)id / (uint32_t)ext;
-      } else {
-        v[d] = wl[d] + (int)(id % ext);
-        id /= ext;
-      }
-      ring = max(ring, abs(v[d] - hb[d]));
-    }
-    visit_batch(v, in && ring > done_ring, false);
-  }
-}
-
-// Walks the staged segment [qb, qb + n) block by block (blocks are 32 aligned records) and
-// calls inner(j0, j1) for the parts whose block some lane of the warp may need: the lane's
-// box holds the tile, the block's box lower bound is within `bound` (strictly below it when
-// `strict`) and the block's largest payload reaches `pmin`.
-template <int N, class M, class Inner>
-__device__ __forceinline__ void scan_blocks(const KParams& kp, const float4* __restrict__ blk, const float* x,
-                                            bool inbox, float bound, bool strict, float pmin, int qb, int n,
-                                            Inner&& inner) {
-  constexpr int BW = Blk<N>::kWords;
-  int j = 0;
-  while (j < n) {
-    const int b = (qb + j) >> 5;
-    const int je = min(n, ((b + 1) << 5) - qb);
-    bool need = inbox;
-    if (kp.lb_ok) {
-      float buf[4 * BW];
-#pragma unroll
-      for (int k = 0; k < BW; ++k) {
-        const float4 v = __ldg(blk + (size_t)b * BW + k);
-        buf[4 * k] = v.x;
-        buf[4 * k + 1] = v.y;
-        buf[4 * k + 2] = v.z;
-        buf[4 * k + 3] = v.w;
-      }
-      const float lb = lower_point<N, M>(x, buf, buf + N, kp.mpar);
-      need = need && (strict ? lb < bound : lb <= bound) && buf[2 * N] >= pmin;
-    }
-    if (__any_sync(0xffffffffu, need)) inner(j, je);
-    j = je;
-  }
+  for (int d = 0; d < N; ++d) rest = rest || hb[d] - wl[d] > done_ring || wh[d] - hb[d] > done_ring;
+  if (rest) box_tiles<N>(g, off, hb, wl, wh, done_ring, lane, other);
 }
 
 // ---- stage 1: bounding box, grid, bins --------------------------------------
@@ -954,85 +926,19 @@ __global__ void __launch_bounds__(256) k_gather_morton(const float4* __restrict_
   }
 }
 
-// ---- work orders and chunks --------------------------------------------------
-// Home points of every tile are taken in the fine Morton order of the tile (so 32 consecutive
-// points are close together at the data's own density scale).  For the one-sided density
-// sweeps they are also stably partitioned by search-box signature -- which neighbour tiles the
-// box of radius dc reaches, 2 bits per dimension -- so the 32 lanes of a warp share one box.
-// (The nearest-higher sweep and the symmetric density sweep take the Morton order as it is.)
-// The orders are cut into chunks of kChunk home points; one CTA processes one chunk, so a heavy
-// tile is spread over many CTAs.  One CTA per tile; warp w partitions the w-th quarter of the
-// tile and the quarters are concatenated per key, which keeps the partition stable.
-template <int N>
-__global__ void __launch_bounds__(kTileThreads) k_order(const KParams kp, Events ev,
-                                                        const int32_t* __restrict__ off,
-                                                        const float4* __restrict__ rec_w,
-                                                        const int32_t* __restrict__ mq,
-                                                        int32_t* __restrict__ ord_rho,
-                                                        uint32_t* __restrict__ chunk_count) {
-  constexpr int K = N <= 4 ? (1 << (2 * N)) : 1;
-  __shared__ uint32_t s_cnt[kChunkWarps][K];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
-  for (int t = blockIdx.x; t < kp.ntiles; t += gridDim.x) {
-    const int beg = off[t], end = off[t + 1];
-    if (threadIdx.x == 0) chunk_count[t] = (uint32_t)((end - beg + kChunk - 1) / kChunk);
-    if (beg == end) continue;
-    const EvGrid* g = ev.eg + find_event(ev.tile, kp.n_events, t);
-    int hb[N];
-    home_bins<N>(g, t, hb);
-    const int quarter = ((end - beg + kChunkWarps - 1) / kChunkWarps + 31) & ~31;
-    const int wb = min(end, beg + warp * quarter), we = min(end, wb + quarter);
-    for (int e = threadIdx.x; e < kChunkWarps * K; e += blockDim.x) (&s_cnt[0][0])[e] = 0;
-    __syncthreads();
-    for (int pass = 0; pass < 2; ++pass) {
-      for (int base = wb; base < we; base += 32) {
-        const int p = base + lane;
-        const bool valid = p < we;
-        const int q = valid ? mq[p] : mq[beg];
-        int key = 0;
-        if (K > 1) {
-          float x[N], pl;
-          load_rec<N>(rec_w, q, x, pl);
-          int lo[N], hi[N];
-          lane_box<N>(kp, g, x, kp.dc, hb, lo, hi);
-#pragma unroll
-          for (int d = 0; d < N; ++d) key |= ((lo[d] < hb[d] ? 1 : 0) | (hi[d] > hb[d] ? 2 : 0)) << (2 * d);
-        }
-        const uint32_t peers = __match_any_sync(0xffffffffu, valid ? key : -1);
-        const bool leader = valid && (peers & lt) == 0;
-        if (pass == 1 && valid) ord_rho[beg + s_cnt[warp][key] + __popc(peers & lt)] = q;
-        __syncwarp();
-        if (leader) s_cnt[warp][key] += __popc(peers);
-        __syncwarp();
-      }
-      if (pass == 0) {
-        __syncthreads();
-        // first slot of (warp, key): keys in order, warps in order inside a key
-        if (threadIdx.x == 0) {
-          uint32_t run = 0;
-          for (int k = 0; k < K; ++k)
-            for (int w = 0; w < kChunkWarps; ++w) {
-              const uint32_t c = s_cnt[w][k];
-              s_cnt[w][k] = run;
-              run += c;
-            }
-        }
-        __syncthreads();
-      }
-    }
-    __syncthreads();
-  }
-}
+// ---- chunks ---------------------------------------------------------------------
+// Home points of every tile are taken in the tile's fine Morton order (so 32 consecutive points are
+// close together at the data's own density scale), cut into chunks of kChunk points; one CTA
+// processes one chunk, so a heavy tile is spread over many CTAs.
 
-// Chunks of kChunk and blocks of 32 points of every tile (when no density home order is built).
+// Chunks of kChunk and blocks of 32 points of every tile.
 __global__ void k_tile_counts(int ntiles, const int32_t* __restrict__ off, uint32_t* __restrict__ chunk_count,
                               uint32_t* __restrict__ blk_count) {
   const int stride = gridDim.x * blockDim.x;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += stride) {
     const int cnt = off[t + 1] - off[t];
     chunk_count[t] = (uint32_t)((cnt + kChunk - 1) / kChunk);
-    blk_count[t] = (uint32_t)((cnt + 31) / 32);
+    if (blk_count) blk_count[t] = (uint32_t)((cnt + 31) / 32);
   }
 }
 
@@ -1044,204 +950,6 @@ __global__ void k_chunk_map(int ntiles, const int32_t* __restrict__ off, const u
     const uint32_t c0 = chunk_off[t];
     for (int c = 0; c < nch; ++c) chunk_tile[c0 + c] = t;
   }
-}
-
-// ---- staged sweep over the search-box tiles of one chunk ------------------------
-// The CTA's 4 warps (128 home points of one tile) walk the union of their search boxes
-// in the reference's lexicographic tile order.  Thread 0 packs consecutive tile segments
-// into pieces of at most kStageWords float4 words and copies each piece into shared memory
-// with bulk copies (TMA) completing on an mbarrier; two buffers alternate so the copy of
-// piece p + 1 overlaps the scan of piece p.  Each warp scans only the segments of tiles in
-// its own union; each lane only counts candidates of tiles inside its own box.
-
-template <int N>
-struct StageSmem {
-  float4 buf[2][kStageWords];
-  int32_t seg_v[2][kMaxSeg][N];
-  int32_t seg_qb[2][kMaxSeg];
-  int32_t seg_cnt[2][kMaxSeg];
-  int32_t seg_boff[2][kMaxSeg];
-  int32_t nseg[2];
-  int32_t wlo[kChunkWarps][N], whi[kChunkWarps][N];
-  int32_t ulo[N], uhi[N];
-  int32_t any_valid;
-  int32_t has[2];
-  alignas(8) uint64_t full[2];
-};
-
-// Thread-0 iterator over the tiles of the CTA union that some warp needs.
-template <int N>
-struct TileIter {
-  int v[N];
-  bool started = false;
-  int q = 0, qe = 0;
-
-  __device__ bool needed(const StageSmem<N>& sm) const {
-    for (int w = 0; w < kChunkWarps; ++w) {
-      bool in = true;
-#pragma unroll
-      for (int d = 0; d < N; ++d) in = in && v[d] >= sm.wlo[w][d] && v[d] <= sm.whi[w][d];
-      if (in) return true;
-    }
-    return false;
-  }
-
-  // Advances to the next needed, non-empty tile; false when the union is exhausted.
-  __device__ bool next(const EvGrid* __restrict__ g, const int32_t* __restrict__ off, const StageSmem<N>& sm) {
-    while (true) {
-      if (!started) {
-#pragma unroll
-        for (int d = 0; d < N; ++d) v[d] = sm.ulo[d];
-        started = true;
-      } else {
-        int d = N - 1;
-        for (; d >= 0; --d) {
-          if (v[d] < sm.uhi[d]) {
-            ++v[d];
-            break;
-          }
-          v[d] = sm.ulo[d];
-        }
-        if (d < 0) return false;
-      }
-      if (!needed(sm)) continue;
-      int u = g->tile_base;
-#pragma unroll
-      for (int d = 0; d < N; ++d) u += g->stride[d] * wrap_bin(v[d], g->nperdim);
-      q = off[u];
-      qe = off[u + 1];
-      if (qe > q) return true;
-    }
-  }
-};
-
-// Builds piece b (thread 0 only) and issues its bulk copies; returns the words staged.
-template <int N>
-__device__ int build_piece(const EvGrid* __restrict__ g, const int32_t* __restrict__ off,
-                           const float4* __restrict__ rec, StageSmem<N>& sm, TileIter<N>& it, bool& done,
-                           int b) {
-  constexpr int W = Rec<N>::kWords;
-  constexpr int cap = kStageWords / W;
-  int nseg = 0, fill = 0;
-  while (!done && nseg < kMaxSeg && fill < cap) {
-    if (it.q >= it.qe) {
-      if (!it.next(g, off, sm)) {
-        done = true;
-        break;
-      }
-    }
-    const int take = min(it.qe - it.q, cap - fill);
-#pragma unroll
-    for (int d = 0; d < N; ++d) sm.seg_v[b][nseg][d] = it.v[d];
-    sm.seg_qb[b][nseg] = it.q;
-    sm.seg_cnt[b][nseg] = take;
-    sm.seg_boff[b][nseg] = fill;
-    ++nseg;
-    fill += take;
-    it.q += take;
-  }
-  sm.nseg[b] = nseg;
-  if (fill > 0) {
-    mbar_arrive_expect_tx(&sm.full[b], (uint32_t)(fill * W * 16));
-    for (int s = 0; s < nseg; ++s)
-      bulk_g2s(&sm.buf[b][sm.seg_boff[b][s] * W], rec + (size_t)sm.seg_qb[b][s] * W,
-               (uint32_t)(sm.seg_cnt[b][s] * W * 16), &sm.full[b]);
-  }
-  return fill;
-}
-
-constexpr uint64_t kWaitLimitNs = 1000000000ull;  // 1 s per bulk-copy wait
-
-// Runs the staged sweep; `vis(inbox, staged_records, first_position, count)` is called for
-// every staged segment of a tile the warp needs.  Returns false if a bulk copy did not
-// complete within the wait limit (the caller reports it and the CTA exits).
-//
-// The give-up decision is made for the whole CTA: every thread waits on the piece's mbarrier
-// with its own time limit, a warp whose lanes did not all see the copy complete skips the
-// piece as a whole (no lane leaves the warp's shuffles and votes), and the barrier that ends
-// the piece is __syncthreads_or of the warps' give-ups, so every thread leaves the loop at the
-// same point and no thread passes a barrier that its siblings do not reach.  Before the CTA
-// returns, the copies it has issued (the timed-out piece and the one issued ahead of it) are
-// waited for once more, again with a time limit: a bulk copy cannot be cancelled, and shared
-// memory must not be released to the next CTA while one may still write into it.
-template <int N, class Visit>
-__device__ bool staged_sweep(const EvGrid* __restrict__ g, const int32_t* __restrict__ off,
-                             const float4* __restrict__ rec, StageSmem<N>& sm, const int* lo, const int* hi,
-                             bool valid, Visit&& vis) {
-  constexpr int W = Rec<N>::kWords;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int wl[N], wh[N];
-  const bool warp_valid = __any_sync(0xffffffffu, valid);
-#pragma unroll
-  for (int d = 0; d < N; ++d) {
-    wl[d] = warp_min_i(valid ? lo[d] : INT_MAX);
-    wh[d] = warp_max_i(valid ? hi[d] : INT_MIN);
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int d = 0; d < N; ++d) {
-      sm.wlo[warp][d] = wl[d];
-      sm.whi[warp][d] = wh[d];
-    }
-  }
-  if (threadIdx.x == 0) {
-    mbar_init(&sm.full[0], 1);
-    mbar_init(&sm.full[1], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int any = 0;
-#pragma unroll
-    for (int d = 0; d < N; ++d) {
-      int a = INT_MAX, z = INT_MIN;
-      for (int w = 0; w < kChunkWarps; ++w) {
-        a = min(a, sm.wlo[w][d]);
-        z = max(z, sm.whi[w][d]);
-      }
-      sm.ulo[d] = a;
-      sm.uhi[d] = z;
-    }
-    for (int w = 0; w < kChunkWarps; ++w) any |= sm.wlo[w][0] != INT_MAX;
-    sm.any_valid = any;
-  }
-  __syncthreads();
-  TileIter<N> it;
-  bool done = sm.any_valid == 0;
-  if (threadIdx.x == 0) sm.has[0] = build_piece<N>(g, off, rec, sm, it, done, 0) > 0;
-  __syncthreads();
-  for (int p = 0; sm.has[p & 1]; ++p) {
-    const int b = p & 1;
-    if (threadIdx.x == 0) sm.has[b ^ 1] = build_piece<N>(g, off, rec, sm, it, done, b ^ 1) > 0;
-    const bool arrived = mbar_wait_bounded(&sm.full[b], (uint32_t)((p >> 1) & 1), kWaitLimitNs);
-    // warp-uniform: a warp visits the piece only if all of its lanes saw the copy complete
-    const bool warp_gave_up = __any_sync(0xffffffffu, !arrived);
-    if (!warp_gave_up) {
-      const int nseg = sm.nseg[b];
-      for (int s = 0; s < nseg; ++s) {
-        bool wneed = warp_valid, inbox = valid;
-#pragma unroll
-        for (int d = 0; d < N; ++d) {
-          const int vd = sm.seg_v[b][s][d];
-          wneed = wneed && vd >= wl[d] && vd <= wh[d];
-          inbox = inbox && vd >= lo[d] && vd <= hi[d];
-        }
-        if (!wneed) continue;
-        vis(inbox, &sm.buf[b][sm.seg_boff[b][s] * W], sm.seg_qb[b][s], sm.seg_cnt[b][s]);
-      }
-    }
-    // CTA-uniform: every thread takes the same branch after this barrier
-    if (__syncthreads_or(warp_gave_up ? 1 : 0)) {
-      // drain what this CTA has issued: piece p (timed out) and piece p + 1 (issued above)
-      if (threadIdx.x == 0) {
-        mbar_wait_bounded(&sm.full[b], (uint32_t)((p >> 1) & 1), kWaitLimitNs);
-        if (sm.has[b ^ 1]) mbar_wait_bounded(&sm.full[b ^ 1], (uint32_t)(((p + 1) >> 1) & 1), kWaitLimitNs);
-      }
-      __syncthreads();
-      return false;
-    }
-  }
-  return true;
 }
 
 // Chunk of the CTA: tile, event grid and home position of this thread.
@@ -1273,60 +981,132 @@ __device__ __forceinline__ bool chunk_home(const KParams& kp, Events ev, const i
 // rho_i accumulates, in the reference's candidate order (search-box tiles
 // lexicographically, ascending index inside a tile), term = k(d, i, j) * w_j for every
 // candidate with d <= dc; candidates beyond dc contribute +-0 and are skipped.
+//
+// The homes of a warp are 32 neighbours of a tile's Morton order, so most candidates of its
+// search-box tiles are out of every lane's reach: the lanes read 32 candidates at a time (in index
+// order), keep those within dc of the box of the warp's homes, and append them to the warp's buffer
+// in shared memory, coordinates and terms by dimension.  What is kept is summed 32 at a time, four
+// candidates per load with paired differences and squares: 7 instructions a candidate, where staging
+// whole tiles by bulk copy and testing every candidate took about 12.  Bound by instruction issue on
+// large inputs and by the sums' own chain of additions where a scheduler has one warp: 0.66 -> 0.32 ms
+// on 1M 2-D points, 67 -> 36 us on 16k (homes in Morton order as they are; grouping them by the
+// tiles their search boxes reach, in a pass of 25 us, is not needed any more).
 template <int N, int MT>
-__global__ void __launch_bounds__(kTileThreads) k_density(const KParams kp, Events ev,
-                                                          const int32_t* __restrict__ off,
-                                                          const int32_t* __restrict__ ord,
-                                                          const int32_t* __restrict__ chunk_tile,
-                                                          const uint32_t* __restrict__ chunk_off,
-                                                          const uint32_t* __restrict__ chunk_total,
-                                                          const float4* __restrict__ rec_w,
-                                                          const float4* __restrict__ blk,
-                                                          float4* __restrict__ rec_r, DevStatus* st) {
+__global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4)) k_density(
+    const KParams kp, Events ev, const int32_t* __restrict__ off, const int32_t* __restrict__ chunk_tile,
+    const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ chunk_total,
+    const float4* __restrict__ rec_w, const int32_t* __restrict__ mq, float4* __restrict__ rec_r) {
   using M = Metric<N, MT>;
-  constexpr int W = Rec<N>::kWords;
-  __shared__ StageSmem<N> sm;
+  // coordinates and flat-kernel terms (or weights) of up to 64 kept candidates: two halves of 32
+  __shared__ ulonglong2 s_buf[kChunkWarps][N + 1][16];
   ChunkHome h;
   if (!chunk_home(kp, ev, off, chunk_tile, chunk_off, chunk_total, h)) return;
-  const int pos = ord[h.p];
   const bool valid = h.valid;
+  if (!__any_sync(0xffffffffu, valid)) return;
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  const int pos = mq[h.p];
   float x[N], wi;
   load_rec<N>(rec_w, pos, x, wi);
-  int hb[N], lo[N], hi[N];
+  int hb[N], lo[N], hi[N], wl[N], wh[N];
   home_bins<N>(h.g, h.t, hb);
   lane_box<N>(kp, h.g, x, kp.dc, hb, lo, hi);
+  float hlo[N], hhi[N];  // box of the warp's homes
+#pragma unroll
+  for (int d = 0; d < N; ++d) {
+    wl[d] = warp_min_i(valid ? lo[d] : INT_MAX);
+    wh[d] = warp_max_i(valid ? hi[d] : INT_MIN);
+    hlo[d] = warp_min_f(valid ? x[d] : INFINITY);
+    hhi[d] = warp_max_f(valid ? x[d] : -INFINITY);
+  }
   const bool flat = kp.kernel_type == CLUE_KERNEL_FLAT;
   const float kflat = kp.kpar[0];
   const float tdc = kp.t_dc;
+  const unsigned lt = (1u << lane) - 1u;
+  unsigned long long x2[N];
+#pragma unroll
+  for (int d = 0; d < N; ++d) x2[d] = pk2(make_float2(x[d], x[d]));
   float rho = 0.0f;
-  const bool ok = staged_sweep<N>(h.g, off, rec_w, sm, lo, hi, valid, [&](bool inbox, const float4* sb, int qb, int n_) {
-    scan_blocks<N, M>(kp, blk, x, inbox, tdc, false, -INFINITY, qb, n_, [&](int j0, int j1) {
-      if (flat) {
-#pragma unroll 4
-        for (int j = j0; j < j1; ++j) {
-          float c[N], wj;
-          unpack_rec<N>(sb + j * W, c, wj);
-          const float s = M::partial(x, c, kp.mpar);
-          const float term = (qb + j == pos) ? wj : fmul(kflat, wj);
-          if (inbox && s <= tdc) rho = fadd(rho, term);
+  box_tiles<N>(h.g, off, hb, wl, wh, -1, lane, [&](const int* v, int, int pb, int pe) {
+    bool inbox = valid;
+#pragma unroll
+    for (int d = 0; d < N; ++d) inbox = inbox && v[d] >= lo[d] && v[d] <= hi[d];
+    if (!__any_sync(0xffffffffu, inbox)) return;
+    const float thr = inbox ? tdc : -INFINITY;
+    int fill = 0;        // candidates appended so far
+    int self = INT_MIN;  // the home point's own number among them
+    // Sums candidates [f0, f1) of the buffer (f0 a multiple of 32, at most 32 of them).
+    auto sum = [&](int f0, int f1) {
+      // groups of four that hold some home's own point, whose term is its weight
+      const unsigned own = __reduce_or_sync(0xffffffffu, self >= f0 && self < f1 ? 1u << ((self - f0) >> 2) : 0u);
+      const int q0 = (f0 >> 2) & 15;
+      auto four = [&](int q, bool tail) {
+        float2 s2[2];
+        ulonglong2 c2[N];
+#pragma unroll
+        for (int d = 0; d < N; ++d) c2[d] = s_buf[warp][d][q0 + q];
+        {
+          unsigned long long ca[N], cb[N];
+#pragma unroll
+          for (int d = 0; d < N; ++d) ca[d] = c2[d].x, cb[d] = c2[d].y;
+          s2[0] = partial_packed<N, MT>(x2, ca, kp.mpar);
+          s2[1] = partial_packed<N, MT>(x2, cb, kp.mpar);
         }
-      } else {
-        for (int j = j0; j < j1; ++j) {
-          float c[N], wj;
-          unpack_rec<N>(sb + j * W, c, wj);
-          const float s = M::partial(x, c, kp.mpar);
-          if (inbox && s <= tdc) {
-            const float kv = (qb + j == pos) ? 1.0f : kernel_value(kp.kernel_type, kp.kpar, M::finish(s));
-            rho = fadd(rho, fmul(kv, wj));
+        const float4 tv = reinterpret_cast<const float4&>(s_buf[warp][N][q0 + q]);
+        float s[4] = {s2[0].x, s2[0].y, s2[1].x, s2[1].y}, tt[4] = {tv.x, tv.y, tv.z, tv.w};
+        if (tail) {  // the last group's empty places
+#pragma unroll
+          for (int e = 1; e < 4; ++e)
+            if (f0 + 4 * q + e >= f1) s[e] = INFINITY;
+        }
+        const bool any_own = (own >> q) & 1u;
+        if (flat) {
+          if (any_own) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) tt[e] = f0 + 4 * q + e == self ? wi : tt[e];
           }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) rho = s[e] <= thr ? fadd(rho, tt[e]) : rho;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (s[e] <= thr) {
+              const float kv = any_own && f0 + 4 * q + e == self
+                                   ? 1.0f
+                                   : kernel_value(kp.kernel_type, kp.kpar, M::finish(s[e]));
+              rho = fadd(rho, fmul(kv, tt[e]));
+            }
         }
+      };
+      if (flat && f1 - f0 == 32) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) four(q, false);
+      } else {
+        for (int q = 0; f0 + 4 * q < f1; ++q) four(q, f0 + 4 * q + 4 > f1);
       }
-    });
+    };
+    float c[N], w;
+    load_rec<N>(rec_w, min(pb + lane, pe - 1), c, w);
+    for (int base = pb; base < pe; base += 32) {
+      const bool last = base + 32 >= pe;
+      const bool keep = base + lane < pe && (!kp.lb_ok || lower_point<N, M>(c, hlo, hhi, kp.mpar) <= tdc);
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      const int was = fill;
+      if (keep) {
+        const int slot = (was + __popc(m & lt)) & 63;
+#pragma unroll
+        for (int d = 0; d < N; ++d) reinterpret_cast<float*>(s_buf[warp][d])[slot] = c[d];
+        reinterpret_cast<float*>(s_buf[warp][N])[slot] = flat ? fmul(kflat, w) : w;
+      }
+      fill += __popc(m);
+      const int o = pos - base;  // (a home always lies within its warp's box)
+      if (o >= 0 && o < 32) self = was + __popc(m & ((1u << o) - 1u));
+      if (!last) load_rec<N>(rec_w, min(base + 32 + lane, pe - 1), c, w);  // while the kept ones are summed
+      __syncwarp();
+      if ((was ^ fill) & ~31) sum(was & ~31, (was & ~31) + 32);
+      if (last && (fill & 31)) sum(fill & ~31, fill);
+      __syncwarp();
+    }
   });
-  if (!ok) {
-    if (threadIdx.x == 0) atomicOr(&st->stage_timeout, 1u);
-    return;
-  }
   if (valid) store_rec<N>(rec_r, pos, x, rho);
 }
 
@@ -1376,9 +1156,12 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
   const float tdm = kp.t_dm;
   // per warp: the homes' records, and the visited block's coordinates and densities by dimension
   __shared__ float4 s_home[kChunkWarps][32 * Rec<N>::kWords];
-  __shared__ float4 s_blk[kChunkWarps][N + 1][8];
+  __shared__ ulonglong2 s_blk[kChunkWarps][N + 1][8];
   store_rec<N>(s_home[warp], lane, x, rho_i);
   __syncwarp();
+  unsigned long long x2[N];
+#pragma unroll
+  for (int d = 0; d < N; ++d) x2[d] = pk2(make_float2(x[d], x[d]));
   const float slack = M::kRoot ? 1.0f + 1.0f / 524288.0f : 1.0f;  // s range of one rounded distance
   float s_best = INFINITY;  // metric value of the nearest higher so far
   // Candidates beyond bnd cannot be nearer than the best so far (nor within dm): its distance
@@ -1451,19 +1234,17 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
       const int self = h.p - p0;  // the home point itself (equal density) is not a candidate
       uint32_t k1 = 0xffffffffu, k2 = 0xffffffffu;
       for (int q = 0; 4 * q < cnt; ++q) {
-        float cc[N][4], rr[4];
+        ulonglong2 c2[N];
 #pragma unroll
-        for (int d = 0; d <= N; ++d) {
-          const float4 v = s_blk[warp][d][q];
-          float* to = d < N ? cc[d < N ? d : 0] : rr;
-          to[0] = v.x, to[1] = v.y, to[2] = v.z, to[3] = v.w;
-        }
+        for (int d = 0; d < N; ++d) c2[d] = s_blk[warp][d][q];
+        const float4 rv = reinterpret_cast<const float4&>(s_blk[warp][N][q]);
+        const float rr[4] = {rv.x, rv.y, rv.z, rv.w};
 #pragma unroll
         for (int e = 0; e < 4; e += 2) {
-          float ca[N], cb[N];
+          unsigned long long cp[N];
 #pragma unroll
-          for (int d = 0; d < N; ++d) ca[d] = cc[d][e], cb[d] = cc[d][e + 1];
-          const float2 s2 = partial_pair<N, MT>(x, ca, cb, kp.mpar);
+          for (int d = 0; d < N; ++d) cp[d] = e ? c2[d].y : c2[d].x;
+          const float2 s2 = partial_packed<N, MT>(x2, cp, kp.mpar);
 #pragma unroll
           for (int f = 0; f < 2; ++f) {
             const int j = 4 * q + e + f;
@@ -2172,9 +1953,9 @@ inline Events events_of(Workspace& ws) { return Events{ws.ev, ws.ev_pt, ws.ev_ti
 
 template <int N, int MT>
 void launch_density(const KParams& kp, Workspace& ws, cudaStream_t s) {
-  k_density<N, MT><<<chunk_grid(kp), kTileThreads, 0, s>>>(kp, events_of(ws), ws.offsets, ws.ord_rho,
-                                                            ws.chunk_tile, ws.chunk_count, ws.chunk_total,
-                                                            ws.rec_w, ws.blk, ws.rec_r, ws.status);
+  k_density<N, MT><<<chunk_grid(kp), kTileThreads, 0, s>>>(kp, events_of(ws), ws.offsets, ws.chunk_tile,
+                                                            ws.chunk_count, ws.chunk_total, ws.rec_w, ws.mq,
+                                                            ws.rec_r);
 }
 template <int N, int MT>
 void launch_nh(const KParams& kp, Workspace& ws, cudaStream_t s) {
@@ -2192,7 +1973,7 @@ void launch_nh(const KParams& kp, Workspace& ws, cudaStream_t s) {
 template <int N, int MT, int FORM>
 void launch_density_spatial_form(const KParams& kp, Workspace& ws, cudaStream_t s, float kexp) {
   k_density_spatial<N, MT, FORM><<<chunk_grid(kp), kTileThreads, 0, s>>>(
-      kp, events_of(ws), ws.offsets, ws.ord_rho, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_w,
+      kp, events_of(ws), ws.offsets, ws.mq, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_w,
       ws.rec_m_cur, ws.mq, ws.blk, ws.sblk, ws.rec_r, ws.minv, kexp);
 }
 template <int N, int MT>
@@ -2379,10 +2160,8 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
     launches += radix_sort_launches(bits) + 2 + 1 + radix_sort_launches(MortonSortBits<N>::kBits) + 1 +
                 radix_sort_launches(bits) + 1;
   }
-  if (symmetric)
-    k_tile_counts<<<grid_for(kp.ntiles, 256), 256, 0, s>>>(kp.ntiles, ws.offsets, ws.chunk_count, ws.tblk_off);
-  else
-    k_order<N><<<kp.ntiles, kTileThreads, 0, s>>>(kp, ev, ws.offsets, ws.rec_w, ws.mq, ws.ord_rho, ws.chunk_count);
+  k_tile_counts<<<grid_for(kp.ntiles, 256), 256, 0, s>>>(kp.ntiles, ws.offsets, ws.chunk_count,
+                                                         symmetric ? ws.tblk_off : nullptr);
   exclusive_scan(ws.chunk_count, ws.chunk_count, (size_t)kp.ntiles, ws.scan_scratch, ws.chunk_total, s);
   if (symmetric) exclusive_scan(ws.tblk_off, ws.tblk_off, (size_t)kp.ntiles, ws.scan_scratch, nullptr, s);
   k_chunk_map<<<grid_for(kp.ntiles, 256), 256, 0, s>>>(kp.ntiles, ws.offsets, ws.chunk_count, ws.chunk_tile);
@@ -2404,9 +2183,6 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
     k_block_bbox<N><<<grid_for(nblk_threads, 256), 256, 0, s>>>(ws.rec_m, n, ws.blk);
     k_superblock_bbox<N><<<grid_for(nsb_threads, 256), 256, 0, s>>>(ws.blk, n, ws.sblk);
     launches += 3;
-  } else {
-    k_block_bbox<N><<<grid_for(nblk_threads, 256), 256, 0, s>>>(ws.rec_w, n, ws.blk);
-    ++launches;
   }
 
   stage_mark(ws, 1, s);

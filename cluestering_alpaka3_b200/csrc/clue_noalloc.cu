@@ -70,7 +70,7 @@ size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 // included (so a call takes the same sweeps, and gives the same bits, as clue_make_clusters);
 // false if they do not fit.  With base null nothing is carved: the call only checks the fit.
 bool carve(Workspace& ws, void* base, int ndim, size_t n, size_t ntiles) {
-  void* evtab = nullptr;
+  void *evtab = nullptr, *spare = nullptr;
   const size_t w = (size_t)((ndim + 1 + 3) / 4);
   const size_t nb = (size_t)sort_blocks((int)n);
   const size_t hist_len = hist_words(nb);
@@ -101,7 +101,7 @@ bool carve(Workspace& ws, void* base, int ndim, size_t n, size_t ntiles) {
       {(void**)&ws.mkeys_alt, n * 4},
       {(void**)&ws.rec_m, n * w * 16},
       {(void**)&ws.sblk, (n / 1024 + 1) * 6 * 16},
-      {(void**)&ws.ord_rho, n * 4},
+      {&spare, n * 4},  // (unused: the limits on a request stay as documented)
       {(void**)&ws.chunk_count, (ntiles + 1) * 4},
       {(void**)&ws.chunk_tile, (n / kChunkPoints + ntiles + 1) * 4},
       {(void**)&ws.chunk_total, 16},
@@ -264,10 +264,6 @@ extern "C" clue_status clue_make_clusters_noalloc(const clue_params* params, con
       set_error(std::string("device bounds check failed in ") + check_site_name(h.check_site) + ": index " +
                 std::to_string(h.check_index));
       return CLUE_ERR_CUDA;
-    }
-    if (h.stage_timeout) {
-      set_error("a bulk-copy wait in the density / nearest-higher sweep timed out");
-      return CLUE_ERR_TIMEOUT;
     }
     if (h.nonfinite) {
       set_error("coordinates or weights contain NaN or Inf");

@@ -34,3 +34,17 @@ def test_nearest_higher_lattice(gpu_context, n, ppbin, wrapped):
     for tiebreak in ("reference", "rho_index"):
         assert_exact(*run_both(gpu_context, c, w, dc=1.0, rhoc=2.0, dm=4.0, ppbin=ppbin, wrapped=wrapped,
                                tiebreak=tiebreak))
+
+
+@pytest.mark.parametrize("n", [1, 4, 31, 32, 33, 63, 64, 65, 127, 130, 1021])
+@pytest.mark.parametrize("ndim,metric,wrapped", [
+    (1, ("euclidean", ()), ()), (2, ("euclidean", ()), ()), (2, ("periodic_euclidean", (0.0, 40.0)), (0, 1)),
+    (3, ("weighted_euclidean", (0.5, 2.0, 1.0)), ()), (4, ("chebyshev", ()), ()), (9, ("manhattan", ()), ()),
+])
+def test_reference_order_density_edges(gpu_context, n, ndim, metric, wrapped):
+    """Sums of whole and partial buffers of 32 kept candidates; all candidates kept, few, one."""
+    rng = np.random.default_rng(7 * n + ndim)
+    c, w = random_blobs(rng, n, ndim, nblobs=min(3, n), extent=40.0, sigma=1.0)
+    w -= np.float32(0.8)  # negative weights too
+    for dc, ppbin in ((0.4, 128), (2.5, 128), (200.0, 128), (3.0, 16)):
+        assert_exact(*run_both(gpu_context, c, w, dc=dc, rhoc=0.5, dm=dc, ppbin=ppbin, metric=metric, wrapped=wrapped))

@@ -148,11 +148,11 @@ std::vector<ArenaItem> arena_items(Workspace& nw, void** evtab, size_t n, size_t
       {(void**)&nw.offsets, (ntiles + 1) * 4},
       {(void**)&nw.rec_w, n * w * 16},
       {(void**)&nw.rec_r, n * w * 16},
-      {(void**)&nw.delta_s, n * 4},
       {(void**)&nw.nh_s, n * 4},
       {(void**)&nw.par, n * 4},
-      {(void**)&nw.is_seed_s, n * 4},
-      {(void**)&nw.seed_flag, n * 4},
+      {(void**)&nw.seed_bits, (n + 31) / 32 * 4},
+      {(void**)&nw.seed_rank, (n + 31) / 32 * 4},
+      {(void**)&nw.seed_list, n * 4},
       {(void**)&nw.seed_total, 16},
       {(void**)&nw.blk, (n / 32 + 1) * 6 * 16},
       {(void**)&nw.mq_alt, n * 4},
@@ -744,6 +744,7 @@ static clue_status prepare(clue_context ctx, const clue_params* params, const cl
   a.out = *out;
   a.ev_n_seeds = nullptr;
   a.ev_n_clusters = nullptr;
+  a.blocking = false;
   ctx->ws.last_kp = kp;
   return workspace_reserve(ctx->ws, ndim, (size_t)n, (size_t)nt);
 }
@@ -755,7 +756,7 @@ static clue_status read_info(Workspace& ws, const KParams& kp, cudaStream_t s, c
   CLUE_CUDA_TRY(cudaMemcpyAsync(h, ws.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
   CLUE_CUDA_TRY(cudaMemcpyAsync(total, ws.seed_total, 4, cudaMemcpyDeviceToHost, s));
   CLUE_CUDA_TRY(cudaStreamSynchronize(s));
-  unresolved = h->unresolved[3] != 0;
+  unresolved = labels_unresolved(*h);
   if (h->check_site) {
     set_error(std::string("device bounds check failed in ") + check_site_name(h->check_site) + ": index " +
               std::to_string(h->check_index));
@@ -819,11 +820,12 @@ clue_status clue_make_clusters(clue_context ctx, const clue_params* params, cons
     dev_out.delta = out->delta ? reinterpret_cast<float*>(o + 4 * nn) : nullptr;
     a.out = dev_out;
   }
+  a.blocking = true;
   st = run_pipeline_graph(ctx, a, s);
   bool unresolved = false;
   if (st == CLUE_OK) st = read_info(ws, a.kp, s, info, unresolved);
   if (st == CLUE_OK && unresolved) {
-    st = finish_labels_dispatch(ws, a, s, 4);
+    st = finish_labels_dispatch(ws, a, s, 1);
     if (st == CLUE_OK) st = read_info(ws, a.kp, s, info, unresolved);
   }
   if (st == CLUE_OK && memory == CLUE_MEM_HOST) {
@@ -1078,6 +1080,7 @@ static clue_status prepare_batch(clue_context ctx, const clue_params* params, co
   a.metric = metric->type;
   a.out = *out;
   a.ev_n_seeds = nullptr;
+  a.blocking = false;
   a.ev_n_clusters = nullptr;
   ws.last_kp = kp;
   return CLUE_OK;
@@ -1141,12 +1144,13 @@ static clue_status batch_plain(clue_context ctx, const clue_params* params, cons
   }
   a.out = dev_out;
   a.ev_n_clusters = dev_ncl;
+  a.blocking = true;
   st = upload_events(ws, n_events, s);
   if (st == CLUE_OK) st = run_pipeline_graph(ctx, a, s);
   bool unresolved = false;
   if (st == CLUE_OK) st = read_info(ws, a.kp, s, info, unresolved);
   if (st == CLUE_OK && unresolved) {
-    st = finish_labels_dispatch(ws, a, s, 4);
+    st = finish_labels_dispatch(ws, a, s, 1);
     if (st == CLUE_OK) st = read_info(ws, a.kp, s, info, unresolved);
   }
   if (st == CLUE_OK && memory == CLUE_MEM_HOST) {
@@ -1473,7 +1477,7 @@ static clue_status batch_host_overlapped(clue_context ctx, const clue_params* pa
   int64_t seeds = 0, clusters = 0, rounds = 0, tiles = 0;
   for (int c = 0; c < K; ++c) {
     int64_t cs = ht[c], cc = hs[c].n_clusters, cr = hs[c].label_rounds;
-    if (hs[c].unresolved[3] != 0) {
+    if (labels_unresolved(hs[c])) {
       // label chains beyond the fixed rounds: this chunk again, alone, with the plain path
       const int e0 = cut[c], E = cut[c + 1] - e0;
       const size_t a0 = (size_t)ev_off[e0], cnt = (size_t)ev_off[cut[c + 1]] - a0;

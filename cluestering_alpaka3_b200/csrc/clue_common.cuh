@@ -89,8 +89,9 @@ struct DevStatus {
   uint32_t n_seeds;
   uint32_t unresolved[64];   // label rounds that left an unresolved parent chain
   uint32_t label_rounds;
+  uint32_t label_enqueued;   // label rounds the run enqueued
   uint32_t n_clusters;     // seeds kept in the seed lists, summed over events
-  // near-threshold decisions (relative tolerance kNearTol, counted by k_seeds and k_near_ties)
+  // near-threshold decisions (relative tolerance kNearTol, counted by k_nearest_higher and k_near_ties)
   uint32_t near_rhoc;      // |rho - rhoc| <= tol * rhoc
   uint32_t near_seed_dc;   // nearest higher found and |delta - seed_dc| <= tol * seed_dc
   uint32_t near_dm;        // nearest higher found and |delta - dm| <= tol * dm
@@ -99,6 +100,11 @@ struct DevStatus {
   uint32_t check_site;   // device bounds checks (CLUE_DEVICE_CHECKS builds): first failing site
   int32_t check_index;   // and the index it rejected
 };
+
+// Whether the last enqueued label round left a chain unresolved.
+inline bool labels_unresolved(const DevStatus& st) {
+  return st.label_enqueued > 0 && st.unresolved[st.label_enqueued - 1] != 0;
+}
 
 // Relative tolerance of the near-threshold counts: the tolerance rho is held to against FP64.
 constexpr float kNearTol = 1e-5f;
@@ -114,10 +120,10 @@ constexpr float kNearTol = 1e-5f;
 #endif
 enum : uint32_t {
   kChkGatherPerm = 1,    // k_gather: the tile sort's permutation
-  kChkSeedsPerm = 2,     // k_seeds: the permutation
+  kChkSeedsPerm = 2,     // k_nearest_higher: the permutation
   kChkJumpParent = 3,    // k_jump: a parent pointer
-  kChkFinalizeRoot = 4,  // k_finalize: a label root and its original index
-  kChkFinalizeNh = 5,    // k_finalize: a nearest higher
+  kChkFinalizeRoot = 4,  // k_seed_labels, k_labels_again: a label root, an original index
+  kChkFinalizeNh = 5,    // k_nearest_higher: a nearest higher
   kChkDensityTile = 6,   // k_density_sym: a tile of the search box
   kChkDensityMirror = 7, // k_density_sym: the mirrored term's point
 };

@@ -53,12 +53,16 @@ int radix_sort_pairs(uint32_t* keys[2], int32_t* vals[2], bool vals_identity, in
                      uint32_t* hist, uint32_t* scan_scratch, cudaStream_t s);
 // Kernel launches made by radix_sort_pairs / exclusive_scan for the given sizes.
 inline int radix_sort_launches(int bits) { return (bits <= 0 ? 1 : (bits + kRadixBits - 1) / kRadixBits) * 3; }
-constexpr int kScanLaunches = 3;
+constexpr size_t kScanOneBlock = 8192;  // up to this length one block scans all (see exclusive_scan)
+inline int scan_launches(size_t len) { return len <= kScanOneBlock ? 1 : 3; }
 
 // Exclusive scan of len uint32 values (in may alias out).  Writes the total to *total
 // (device pointer) when non-null.
 void exclusive_scan(const uint32_t* in, uint32_t* out, size_t len, uint32_t* scratch,
                     uint32_t* total, cudaStream_t s);
+// The same over the number of bits set in every word (in and out must not alias).
+void exclusive_scan_bits(const uint32_t* in, uint32_t* out, size_t len, uint32_t* scratch,
+                         uint32_t* total, cudaStream_t s);
 
 // offsets[b] = first position of key b in sorted keys (b = 0..nkeys), n at the end; the key of
 // an entry is its value shifted right by `shift` bits.
@@ -78,6 +82,9 @@ struct RunArgs {
   int32_t metric;
   int32_t* ev_n_seeds;           // device [n_events] or null (batched calls)
   int32_t* ev_n_clusters;        // device [n_events] or null (batched calls)
+  // The caller reads the status back and continues label chains the first round left unresolved
+  // (finish_labels); otherwise all rounds are enqueued.
+  bool blocking;
 };
 
 template <int N>
@@ -109,11 +116,11 @@ struct Workspace {
   int32_t* offsets = nullptr;
   float4* rec_w = nullptr;  // coords + weight, tile-sorted
   float4* rec_r = nullptr;  // coords + rho, tile-sorted
-  float* delta_s = nullptr;
-  int32_t* nh_s = nullptr;
-  int32_t* par = nullptr;
-  int32_t* is_seed_s = nullptr;
-  uint32_t* seed_flag = nullptr;  // original order, then exclusive-scanned to ranks
+  int32_t* nh_s = nullptr;        // nearest highers, kept for the near-tie count
+  int32_t* par = nullptr;         // label parents: >= 0 a tile-sorted position, < 0 a root (see k_seed_labels)
+  uint32_t* seed_bits = nullptr;  // one bit per point in original order
+  uint32_t* seed_rank = nullptr;  // seeds before every 32-point word of seed_bits
+  int32_t* seed_list = nullptr;   // positions of the seeds, in no particular order
   uint32_t* seed_total = nullptr;
   float4* blk = nullptr;          // bounding boxes of 32-record blocks of the sorted records
   int32_t* mq_alt = nullptr;      // second value buffer of the Morton sort

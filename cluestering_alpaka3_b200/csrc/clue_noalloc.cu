@@ -90,18 +90,18 @@ bool carve(Workspace& ws, void* base, int ndim, size_t n, size_t ntiles) {
       {(void**)&ws.offsets, (ntiles + 1) * 4},
       {(void**)&ws.rec_w, n * w * 16},
       {(void**)&ws.rec_r, n * w * 16},
-      {(void**)&ws.delta_s, n * 4},
+      {(void**)&ws.seed_rank, n * 4},
       {(void**)&ws.nh_s, n * 4},
       {(void**)&ws.par, n * 4},
-      {(void**)&ws.is_seed_s, n * 4},
-      {(void**)&ws.seed_flag, n * 4},
+      {(void**)&ws.seed_list, n * 4},
+      {(void**)&ws.seed_bits, n * 4},
       {(void**)&ws.seed_total, 16},
       {(void**)&ws.blk, (n / 32 + 1) * 6 * 16},
       {(void**)&ws.mq_alt, n * 4},
       {(void**)&ws.mkeys_alt, n * 4},
       {(void**)&ws.rec_m, n * w * 16},
       {(void**)&ws.sblk, (n / 1024 + 1) * 6 * 16},
-      {&spare, n * 4},  // (unused: the limits on a request stay as documented)
+      {&spare, n * 4},  // (the limits on a request are documented: the items' sizes stay as they are)
       {(void**)&ws.chunk_count, (ntiles + 1) * 4},
       {(void**)&ws.chunk_tile, (n / kChunkPoints + ntiles + 1) * 4},
       {(void**)&ws.chunk_total, 16},
@@ -250,6 +250,7 @@ extern "C" clue_status clue_make_clusters_noalloc(const clue_params* params, con
   for (int d = 0; d < ndim; ++d) a.coords[d] = coords + (size_t)d * n;
   a.weight = weight;
   a.out = *out;
+  a.blocking = true;
 
   cudaStream_t s = (cudaStream_t)stream;
   if ((st = run_pipeline_dispatch(ws, a, s)) != CLUE_OK) return st;
@@ -269,8 +270,8 @@ extern "C" clue_status clue_make_clusters_noalloc(const clue_params* params, con
       set_error("coordinates or weights contain NaN or Inf");
       return CLUE_ERR_NONFINITE;
     }
-    if (h.unresolved[3] == 0 || attempt == 1) break;
-    if ((st = finish_dispatch(ws, a, s, 4)) != CLUE_OK) return st;
+    if (!labels_unresolved(h) || attempt == 1) break;
+    if ((st = finish_dispatch(ws, a, s, 1)) != CLUE_OK) return st;
   }
   if (info) {
     const int64_t nseeds = total;

@@ -194,13 +194,43 @@ __global__ void __launch_bounds__(1024) k_scan_rows(uint32_t* __restrict__ hist,
   if (threadIdx.x == 0) tot[blockIdx.x] = total;
 }
 
+// What a word counts in a scan: its value, or (BITS) the number of bits set in it.
+template <bool BITS>
+__device__ __forceinline__ uint32_t scan_value(uint32_t w) {
+  return BITS ? (uint32_t)__popc(w) : w;
+}
+
+// Short arrays: one block scans everything, so one launch takes the place of three (a launch costs
+// 2-3 us in a graph, and small events are bound by their launches).
+template <bool BITS>
+__global__ void __launch_bounds__(1024) k_scan_one(const uint32_t* in, int len, uint32_t* out, uint32_t* total) {
+  constexpr int kPer = (int)(kScanOneBlock / 1024);
+  const int base = threadIdx.x * kPer;
+  uint32_t v[kPer];
+  uint32_t s = 0;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    v[k] = base + k < len ? scan_value<BITS>(in[base + k]) : 0u;
+    s += v[k];
+  }
+  uint32_t tot;
+  uint32_t run = block_excl_scan(s, &tot);
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    if (base + k < len) out[base + k] = run;
+    run += v[k];
+  }
+  if (threadIdx.x == 0 && total) *total = tot;
+}
+
+template <bool BITS>
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* __restrict__ in, size_t len,
                                                               uint32_t* __restrict__ partial) {
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
   uint32_t s = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k)
-    if (base + k < len) s += in[base + k];
+    if (base + k < len) s += scan_value<BITS>(in[base + k]);
   uint32_t tot;
   block_excl_scan(s, &tot);
   if (threadIdx.x == 0) partial[blockIdx.x] = tot;
@@ -221,6 +251,7 @@ __global__ void __launch_bounds__(1024) k_scan_partials(uint32_t* partial, int n
 }
 
 // `in` and `out` may alias (in-place scan): every thread reads its items before writing them.
+template <bool BITS>
 __global__ void __launch_bounds__(kScanThreads) k_scan_down(const uint32_t* in, size_t len,
                                                             const uint32_t* __restrict__ partial,
                                                             uint32_t* out) {
@@ -229,7 +260,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const uint32_t* in, 
   uint32_t s = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    v[k] = base + k < len ? in[base + k] : 0u;
+    v[k] = base + k < len ? scan_value<BITS>(in[base + k]) : 0u;
     s += v[k];
   }
   uint32_t run = partial[blockIdx.x] + block_excl_scan(s, nullptr);
@@ -251,16 +282,29 @@ __global__ void k_offsets(const uint32_t* __restrict__ keys, int n, int nkeys, i
 
 }  // namespace
 
-void exclusive_scan(const uint32_t* in, uint32_t* out, size_t len, uint32_t* scratch, uint32_t* total,
-                    cudaStream_t s) {
-  const int nb = (int)((len + kScanTile - 1) / kScanTile);
-  if (nb == 0) {
+template <bool BITS>
+static void scan(const uint32_t* in, uint32_t* out, size_t len, uint32_t* scratch, uint32_t* total, cudaStream_t s) {
+  if (len == 0) {
     if (total) cudaMemsetAsync(total, 0, sizeof(uint32_t), s);
     return;
   }
-  k_scan_reduce<<<nb, kScanThreads, 0, s>>>(in, len, scratch);
+  if (len <= kScanOneBlock) {
+    k_scan_one<BITS><<<1, 1024, 0, s>>>(in, (int)len, out, total);
+    return;
+  }
+  const int nb = (int)((len + kScanTile - 1) / kScanTile);
+  k_scan_reduce<BITS><<<nb, kScanThreads, 0, s>>>(in, len, scratch);
   k_scan_partials<<<1, 1024, 0, s>>>(scratch, nb, total);
-  k_scan_down<<<nb, kScanThreads, 0, s>>>(in, len, scratch, out);
+  k_scan_down<BITS><<<nb, kScanThreads, 0, s>>>(in, len, scratch, out);
+}
+
+void exclusive_scan(const uint32_t* in, uint32_t* out, size_t len, uint32_t* scratch, uint32_t* total,
+                    cudaStream_t s) {
+  scan<false>(in, out, len, scratch, total, s);
+}
+void exclusive_scan_bits(const uint32_t* in, uint32_t* out, size_t len, uint32_t* scratch, uint32_t* total,
+                         cudaStream_t s) {
+  scan<true>(in, out, len, scratch, total, s);
 }
 
 int radix_sort_pairs(uint32_t* keys[2], int32_t* vals[2], bool vals_identity, int n, int bits,

@@ -48,3 +48,27 @@ def test_reference_order_density_edges(gpu_context, n, ndim, metric, wrapped):
     w -= np.float32(0.8)  # negative weights too
     for dc, ppbin in ((0.4, 128), (2.5, 128), (200.0, 128), (3.0, 16)):
         assert_exact(*run_both(gpu_context, c, w, dc=dc, rhoc=0.5, dm=dc, ppbin=ppbin, metric=metric, wrapped=wrapped))
+
+
+@pytest.mark.parametrize("n,fall", [(33, 0), (3000, 0), (100000, 0), (100000, 97)])
+@pytest.mark.parametrize("blocking", [True, False])
+def test_label_chains(gpu_context, n, fall, blocking):
+    """One chain through all points (each point's nearest higher is the next one), whole or cut into
+    pieces of `fall` points: one label round, several enqueued rounds, rounds from the host."""
+    import torch
+    from cluestering_alpaka3_b200 import capi
+    from oracle import oracle as O
+    from parity_util import gpu_args, oracle_cfg
+    c = np.arange(n, dtype=np.float32)[None]
+    w = (1.0 + np.arange(n) % fall if fall else 1.0 + np.arange(n)).astype(np.float32)
+    kw = dict(dc=0.5, rhoc=1.5, dm=1.5)
+    ref = O.run(c, w, oracle_cfg(**kw))
+    dc, dw = torch.from_numpy(c).cuda(), torch.from_numpy(w).cuda()
+    out = {k: torch.empty(n, dtype=torch.int32, device="cuda") for k in ("cluster_index", "is_seed", "nearest_higher")}
+    torch.cuda.synchronize()
+    gpu_context.make_clusters_device(dc.data_ptr(), dw.data_ptr(), 1, n, {k: t.data_ptr() for k, t in out.items()},
+                                     *gpu_args(**kw), blocking=blocking)
+    info = gpu_context.read_info()
+    assert isinstance(info, capi.RunInfo) and info.n_clusters == ref.stats["n_clusters"]
+    for k, t in out.items():
+        np.testing.assert_array_equal(t.cpu().numpy(), getattr(ref, k), err_msg=k)

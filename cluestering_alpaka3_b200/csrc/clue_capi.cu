@@ -277,6 +277,8 @@ void workspace_release(Workspace& ws) {
   if (ws.pipe_pinned) cudaFreeHost(ws.pipe_pinned);
   if (ws.arena) cudaFree(ws.arena);
   if (ws.dstage) cudaFree(ws.dstage);
+  if (ws.post) cudaFree(ws.post);
+  if (ws.post_host) cudaFreeHost(ws.post_host);
   if (ws.status_host) cudaFreeHost(ws.status_host);
   if (ws.pinned) cudaFreeHost(ws.pinned);
   ws = Workspace{};
@@ -324,27 +326,89 @@ float metric_eval_n(int32_t type, const float* a, const float* b, const float* p
 
 namespace clue_b200 {
 
-// keys[i] = cluster_index[i] + 1 (0 for outliers); labels outside [-1, n) raise *bad and count
-// as outliers so that every key stays inside the offsets table.
-__global__ void k_label_keys(const int32_t* __restrict__ label, int n, uint32_t* __restrict__ keys,
-                             int32_t* __restrict__ bad) {
+// keys[i] = cluster_index[i] + 1 (0 for outliers), the largest of them to info->n_clusters; labels
+// outside [-1, n) raise info->bad and count as outliers so that every key stays inside the offsets
+// table.
+__global__ void __launch_bounds__(256) k_label_keys(const int32_t* __restrict__ label, int n,
+                                                    uint32_t* __restrict__ keys, CsrInfo* info) {
+  uint32_t top = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int l = label[i];
     const bool ok = l >= -1 && l < n;
-    if (!ok) atomicOr(bad, 1);
-    keys[i] = ok ? (uint32_t)(l + 1) : 0u;
+    if (!ok) atomicOr(&info->bad, 1u);
+    const uint32_t k = ok ? (uint32_t)(l + 1) : 0u;
+    keys[i] = k;
+    top = max(top, k);
   }
+  __shared__ uint32_t s_top;
+  if (threadIdx.x == 0) s_top = 0u;
+  __syncthreads();
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_top, top);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_top > 0) atomicMax(&info->n_clusters, s_top);  // one per block
 }
 
-// off[k] = first sorted position of key k (k = 0..n+1); key 0 holds the outliers, so cluster c
-// owns sorted positions [off[c + 1], off[c + 2]).  Writes offsets[0..n] and the clustered points.
+// off[k] = first sorted position of key k (up to one above the largest key); key 0 holds the outliers,
+// so cluster c owns sorted positions [off[c + 1], off[c + 2]).  Writes offsets[0..n] (the total past
+// the last cluster) and the clustered points.
 __global__ void k_cluster_csr(const int32_t* __restrict__ off, const int32_t* __restrict__ vals, int n,
-                              int32_t* __restrict__ offsets, int32_t* __restrict__ points) {
-  const int first = off[1];
+                              int32_t* __restrict__ offsets, int32_t* __restrict__ points, CsrInfo* info) {
+  const int first = off[1], nc = (int)info->n_clusters;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
-    offsets[i] = off[i + 1] - first;
+    offsets[i] = i <= nc ? off[i + 1] - first : n - first;
     if (i < n - first) points[i] = vals[first + i];
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) info->n_clustered = n - first;
+}
+
+clue_status post_reserve(Workspace& ws, size_t device_bytes, size_t host_bytes) {
+  int prev = 0;
+  cudaGetDevice(&prev);
+  cudaSetDevice(ws.device);
+  cudaError_t e = cudaSuccess;
+  if (device_bytes > ws.post_bytes) {
+    if (ws.post) {
+      cudaDeviceSynchronize();
+      cudaFree(ws.post);
+    }
+    ws.post = nullptr;
+    ws.post_bytes = 0;
+    e = cudaMalloc(&ws.post, device_bytes);
+    if (e == cudaSuccess) ws.post_bytes = device_bytes;
+  }
+  if (e == cudaSuccess && host_bytes > ws.post_host_bytes) {
+    if (ws.post_host) cudaFreeHost(ws.post_host);
+    ws.post_host = nullptr;
+    ws.post_host_bytes = 0;
+    e = cudaMallocHost(&ws.post_host, host_bytes);
+    if (e == cudaSuccess) ws.post_host_bytes = host_bytes;
+  }
+  cudaSetDevice(prev);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    set_error(std::string("temporaries of a post-processing call: ") + cudaGetErrorString(e));
+    return CLUE_ERR_OUT_OF_MEMORY;
+  }
+  return CLUE_OK;
+}
+
+clue_status clusters_csr(Workspace& ws, int n, const int32_t* cluster_index, int32_t* offsets, int32_t* points,
+                         CsrInfo* info, cudaStream_t s) {
+  // keys = label + 1 in [0, n]; offsets_from_sorted needs n + 2 entries
+  clue_status st = workspace_reserve(ws, 1, (size_t)n, (size_t)n + 2, 1);
+  if (st != CLUE_OK) return st;
+  CLUE_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(CsrInfo), s));
+  const int threads = 256;
+  const int blocks = std::min((n + threads - 1) / threads, 148 * 16);
+  k_label_keys<<<blocks, threads, 0, s>>>(cluster_index, n, ws.keys[0], info);
+  const int bits = bits_for((uint32_t)n);
+  const int cur = radix_sort_pairs(ws.keys, ws.vals, true, n, bits, ws.hist, ws.scan_scratch, s, &info->n_clusters);
+  offsets_from_sorted(ws.keys[cur], n, n + 1, ws.offsets, s, 0, &info->n_clusters);
+  k_cluster_csr<<<blocks, threads, 0, s>>>(ws.offsets, ws.vals[cur], n, offsets, points, info);
+  ws.launches += 3 + radix_sort_launches(bits);
+  CLUE_CUDA_TRY(cudaGetLastError());
+  return CLUE_OK;
 }
 
 }  // namespace clue_b200
@@ -366,6 +430,10 @@ struct clue_context_s {
   cudaGraphExec_t plain_exec = nullptr;
   cudaEvent_t plain_ev[2] = {};
 };
+
+namespace clue_b200 {
+Workspace& context_workspace(clue_context ctx) { return ctx->ws; }
+}  // namespace clue_b200
 
 // Captures the pipeline enqueued by run_pipeline_dispatch on `g` into a graph and launches it
 // there, keeping the executable in *exec (updated in place when the captured graph has the same
@@ -677,7 +745,7 @@ clue_status clue_context_reserve_batch(clue_context ctx, int32_t ndim, int64_t n
   return workspace_reserve(ctx->ws, ndim, (size_t)n_points, (size_t)n_tiles, (size_t)n_events);
 }
 
-size_t clue_context_workspace_bytes(clue_context ctx) { return ctx ? ctx->ws.arena_bytes + ctx->ws.dstage_bytes : 0; }
+size_t clue_context_workspace_bytes(clue_context ctx) { return ctx ? ctx->ws.arena_bytes + ctx->ws.dstage_bytes + ctx->ws.post_bytes : 0; }
 
 }  // extern "C"
 
@@ -942,36 +1010,27 @@ clue_status clue_get_clusters(clue_context ctx, int32_t n, const int32_t* cluste
     return CLUE_ERR_INVALID_ARG;
   }
   Workspace& ws = ctx->ws;
-  // keys = label + 1 in [0, n]; offsets_from_sorted needs n + 2 entries, one more word holds
-  // the invalid-label flag.
-  clue_status st = workspace_reserve(ws, 1, (size_t)n, (size_t)n + 2, 1);
+  clue_status st = post_reserve(ws, sizeof(CsrInfo), sizeof(CsrInfo));
   if (st != CLUE_OK) return st;
   cudaStream_t s = (cudaStream_t)stream;
   int prev = 0;
   cudaGetDevice(&prev);
   cudaSetDevice(ws.device);
-  int32_t* bad = ws.offsets + (n + 2);
-  CLUE_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int32_t), s));
-  const int threads = 256;
-  const int blocks = std::min((n + threads - 1) / threads, 148 * 16);
-  k_label_keys<<<blocks, threads, 0, s>>>(cluster_index, n, ws.keys[0], bad);
-  const int cur = radix_sort_pairs(ws.keys, ws.vals, true, n, bits_for((uint32_t)n), ws.hist, ws.scan_scratch, s);
-  offsets_from_sorted(ws.keys[cur], n, n + 1, ws.offsets, s);
-  k_cluster_csr<<<blocks, threads, 0, s>>>(ws.offsets, ws.vals[cur], n, offsets, points);
-  ws.launches += 3 + radix_sort_launches(bits_for((uint32_t)n));
-  int32_t h[2] = {0, 0};
-  uint32_t last = 0;
-  CLUE_CUDA_TRY(cudaMemcpyAsync(h, ws.offsets + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  CLUE_CUDA_TRY(cudaMemcpyAsync(h + 1, bad, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  CLUE_CUDA_TRY(cudaMemcpyAsync(&last, ws.keys[cur] + (n - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  CLUE_CUDA_TRY(cudaStreamSynchronize(s));
+  CsrInfo* info = static_cast<CsrInfo*>(ws.post);
+  const CsrInfo* h = static_cast<const CsrInfo*>(ws.post_host);
+  st = clusters_csr(ws, n, cluster_index, offsets, points, info, s);
+  cudaError_t e = cudaSuccess;
+  if (st == CLUE_OK) e = cudaMemcpyAsync(ws.post_host, info, sizeof(CsrInfo), cudaMemcpyDeviceToHost, s);
+  if (st == CLUE_OK && e == cudaSuccess) e = cudaStreamSynchronize(s);
   cudaSetDevice(prev);
-  if (h[1]) {
+  if (st != CLUE_OK) return st;
+  CLUE_CUDA_TRY(e);
+  if (h->bad) {
     set_error("clue_get_clusters: cluster index outside [-1, n)");
     return CLUE_ERR_OUT_OF_RANGE;
   }
-  if (n_clusters_out) *n_clusters_out = (int32_t)last;  // max label + 1 (0 when all are -1)
-  if (n_clustered_out) *n_clustered_out = n - h[0];
+  if (n_clusters_out) *n_clusters_out = (int32_t)h->n_clusters;  // max label + 1 (0 when all are -1)
+  if (n_clustered_out) *n_clustered_out = h->n_clustered;
   return CLUE_OK;
 }
 

@@ -48,9 +48,10 @@ inline size_t scan_scratch_words(size_t len) { return (len + kScanTile - 1) / kS
 
 // Stable LSD radix sort of (key, value) pairs by the low `bits` bits of key.  Values
 // start as the identity (0..n-1) when vals_in is null.  Ping-pongs between buffer 0
-// and 1 of keys/vals; returns the index (0 or 1) holding the result.
+// and 1 of keys/vals; returns the index (0 or 1) holding the result.  With max_key (device, no key is
+// larger) the passes above its top digit only copy.
 int radix_sort_pairs(uint32_t* keys[2], int32_t* vals[2], bool vals_identity, int n, int bits,
-                     uint32_t* hist, uint32_t* scan_scratch, cudaStream_t s);
+                     uint32_t* hist, uint32_t* scan_scratch, cudaStream_t s, const uint32_t* max_key = nullptr);
 // Kernel launches made by radix_sort_pairs / exclusive_scan for the given sizes.
 inline int radix_sort_launches(int bits) { return (bits <= 0 ? 1 : (bits + kRadixBits - 1) / kRadixBits) * 3; }
 constexpr size_t kScanOneBlock = 8192;  // up to this length one block scans all (see exclusive_scan)
@@ -65,9 +66,10 @@ void exclusive_scan_bits(const uint32_t* in, uint32_t* out, size_t len, uint32_t
                          uint32_t* total, cudaStream_t s);
 
 // offsets[b] = first position of key b in sorted keys (b = 0..nkeys), n at the end; the key of
-// an entry is its value shifted right by `shift` bits.
+// an entry is its value shifted right by `shift` bits.  With max_key (device, the largest key) only
+// b = 0..*max_key + 1 are written.
 void offsets_from_sorted(const uint32_t* sorted_keys, int n, int nkeys, int32_t* offsets,
-                         cudaStream_t s, int shift = 0);
+                         cudaStream_t s, int shift = 0, const uint32_t* max_key = nullptr);
 
 // ---- per-dimension pipeline (clue_dim.cu, one instantiation per N) ----------
 struct Workspace;
@@ -147,6 +149,12 @@ struct Workspace {
   void* dstage = nullptr;
   size_t dstage_bytes = 0;
 
+  // device and pinned temporaries of the post-processing calls (grown on demand, post_reserve)
+  void* post = nullptr;
+  size_t post_bytes = 0;
+  void* post_host = nullptr;
+  size_t post_host_bytes = 0;
+
   // runtime choices (clue_context_set_tuning; clue_autotune_batch measures and picks them)
   int32_t tune_symmetric = 1;                  // symmetric density sweep where it applies
   int32_t tune_nh_split = 8;                   // nearest higher: split a block needed by <= this many lanes
@@ -190,6 +198,21 @@ inline void stage_mark(Workspace& ws, int k, cudaStream_t s) {
   if (k < CLUE_N_STAGES) nvtxRangePushA(kNames[k]);
   if (ws.timing && ws.tev[k]) cudaEventRecord(ws.tev[k], s);
 }
+
+Workspace& context_workspace(clue_context ctx);
+
+// Grows the post-processing temporaries to at least these sizes.
+clue_status post_reserve(Workspace& ws, size_t device_bytes, size_t host_bytes);
+
+// What clusters_csr leaves on the device.
+struct CsrInfo {
+  uint32_t n_clusters;   // max label + 1
+  uint32_t bad;          // a label outside [-1, n)
+  int32_t n_clustered;
+};
+// The association map of clue_get_clusters enqueued on s, without waiting; *info is device memory.
+clue_status clusters_csr(Workspace& ws, int n, const int32_t* cluster_index, int32_t* offsets, int32_t* points,
+                         CsrInfo* info, cudaStream_t s);
 
 clue_status workspace_reserve(Workspace& ws, int ndim, size_t n, size_t ntiles, size_t n_events = 1);
 

@@ -23,7 +23,8 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 // the end; keys are read four at a time where the tile is complete.
 __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const uint32_t* __restrict__ keys, int n,
                                                              int shift, uint32_t* __restrict__ hist,
-                                                             int nblocks) {
+                                                             int nblocks, const uint32_t* __restrict__ max_key) {
+  if (max_key && shift > 0 && (*max_key >> shift) == 0) return;  // nothing to order by
   constexpr int kWarps = kSortThreads / 32;
   __shared__ uint32_t h[kWarps][kRadix];
   const int warp = threadIdx.x >> 5;
@@ -96,7 +97,15 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* tot) {
 __global__ void __launch_bounds__(kSortThreads, 4) k_radix_scatter(
     const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     int32_t* __restrict__ vout, int n, int shift, const uint32_t* __restrict__ scanned,
-    const uint32_t* __restrict__ tot, int nblocks) {
+    const uint32_t* __restrict__ tot, int nblocks, const uint32_t* __restrict__ max_key) {
+  if (max_key && shift > 0 && (*max_key >> shift) == 0) {
+    const int end = min(n, (int)(blockIdx.x + 1) * kSortTile);
+    for (int i = blockIdx.x * kSortTile + threadIdx.x; i < end; i += kSortThreads) {
+      kout[i] = kin[i];
+      vout[i] = vin ? vin[i] : i;
+    }
+    return;
+  }
   static_assert(kSortThreads == kRadix, "one thread per digit");
   constexpr int kWarps = kSortThreads / 32;
   constexpr int kSlice = kSortItems * 32;  // items per warp
@@ -178,7 +187,9 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_radix_scatter(
 // Exclusive scan of every digit's row of the digit-major histogram, one CTA per digit (rows are
 // contiguous); the row's total goes to tot[d].
 __global__ void __launch_bounds__(1024) k_scan_rows(uint32_t* __restrict__ hist, int nblocks,
-                                                    uint32_t* __restrict__ tot) {
+                                                    uint32_t* __restrict__ tot, int shift,
+                                                    const uint32_t* __restrict__ max_key) {
+  if (max_key && shift > 0 && (*max_key >> shift) == 0) return;
   uint32_t* row = hist + (size_t)blockIdx.x * nblocks;
   const int per = (nblocks + 1023) / 1024;
   const int beg = min(nblocks, (int)threadIdx.x * per), end = min(nblocks, beg + per);
@@ -271,12 +282,28 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const uint32_t* in, 
   }
 }
 
-__global__ void k_offsets(const uint32_t* __restrict__ keys, int n, int nkeys, int shift, int32_t* __restrict__ off) {
-  const int stride = gridDim.x * blockDim.x;
-  for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos <= n; pos += stride) {
-    const int prev = pos > 0 ? (int)(keys[pos - 1] >> shift) : -1;
-    const int cur = pos < n ? (int)(keys[pos] >> shift) : nkeys;
-    for (int b = prev + 1; b <= cur; ++b) off[b] = pos;
+// Every position writes the offsets of the keys after its predecessor's up to its own.  A long run of
+// absent keys is written by the whole warp (one thread alone took 3.5 ms for the million keys above
+// the last cluster of a million labels).
+__global__ void __launch_bounds__(256) k_offsets(const uint32_t* __restrict__ keys, int n, int nkeys, int shift,
+                                                 int32_t* __restrict__ off, const uint32_t* __restrict__ max_key) {
+  const int stride = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
+  const int last = max_key ? min(nkeys, (int)*max_key + 1) : nkeys;
+  for (int base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; base <= n; base += stride) {
+    const int pos = base + lane;
+    int prev = 0, cur = -1;  // nothing to write
+    if (pos <= n) {
+      prev = pos > 0 ? (int)(keys[pos - 1] >> shift) : -1;
+      cur = pos < n ? (int)(keys[pos] >> shift) : last;
+    }
+    const bool far = cur - prev > 32;
+    if (!far)
+      for (int b = prev + 1; b <= cur; ++b) off[b] = pos;
+    for (unsigned m = __ballot_sync(0xffffffffu, far); m; m &= m - 1) {
+      const int src = __ffs(m) - 1;
+      const int p = __shfl_sync(0xffffffffu, prev, src), c = __shfl_sync(0xffffffffu, cur, src);
+      for (int b = p + 1 + lane; b <= c; b += 32) off[b] = base + src;
+    }
   }
 }
 
@@ -308,29 +335,29 @@ void exclusive_scan_bits(const uint32_t* in, uint32_t* out, size_t len, uint32_t
 }
 
 int radix_sort_pairs(uint32_t* keys[2], int32_t* vals[2], bool vals_identity, int n, int bits,
-                     uint32_t* hist, uint32_t* scan_scratch, cudaStream_t s) {
+                     uint32_t* hist, uint32_t* scan_scratch, cudaStream_t s, const uint32_t* max_key) {
   const int nb = sort_blocks(n);
   int cur = 0;
   const int passes = bits <= 0 ? 1 : (bits + kRadixBits - 1) / kRadixBits;
   for (int p = 0; p < passes; ++p) {
     const int shift = p * kRadixBits;
     uint32_t* tot = hist + (size_t)kRadix * nb;
-    k_radix_hist<<<nb, kSortThreads, 0, s>>>(keys[cur], n, shift, hist, nb);
-    k_scan_rows<<<kRadix, 1024, 0, s>>>(hist, nb, tot);
+    k_radix_hist<<<nb, kSortThreads, 0, s>>>(keys[cur], n, shift, hist, nb, max_key);
+    k_scan_rows<<<kRadix, 1024, 0, s>>>(hist, nb, tot, shift, max_key);
     const int32_t* vin = (p == 0 && vals_identity) ? nullptr : vals[cur];
     k_radix_scatter<<<nb, kSortThreads, 0, s>>>(keys[cur], vin, keys[cur ^ 1], vals[cur ^ 1], n, shift,
-                                                hist, tot, nb);
+                                                hist, tot, nb, max_key);
     cur ^= 1;
   }
   return cur;
 }
 
 void offsets_from_sorted(const uint32_t* sorted_keys, int n, int nkeys, int32_t* offsets, cudaStream_t s,
-                         int shift) {
+                         int shift, const uint32_t* max_key) {
   const int threads = 256;
   int blocks = (n + 1 + threads - 1) / threads;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  k_offsets<<<blocks, threads, 0, s>>>(sorted_keys, n, nkeys, shift, offsets);
+  k_offsets<<<blocks, threads, 0, s>>>(sorted_keys, n, nkeys, shift, offsets, max_key);
 }
 
 }  // namespace clue_b200

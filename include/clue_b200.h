@@ -375,8 +375,8 @@ clue_status clue_get_clusters(clue_context ctx, int32_t n, const int32_t* cluste
  * ascending point order as the reference's association map gives them.  coords (SoA) and
  * cluster_index are device arrays of n points (-1 = not clustered).  per_point (device, n
  * floats, optional) receives every point's score, NaN for points not scored; *mean (host,
- * optional) the average over the scored points.  n x (clustered points) distances; allocates
- * its temporaries and synchronises `stream`.
+ * optional) the average over the scored points.  (clustered points)^2 distances; its temporaries
+ * stay with the context (they grow on demand), and the call synchronises `stream`.
  */
 clue_status clue_silhouette(clue_context ctx, int32_t ndim, int32_t n, const float* coords,
                             const int32_t* cluster_index, float* per_point, float* mean, void* stream);
@@ -391,8 +391,8 @@ clue_status clue_silhouette(clue_context ctx, int32_t ndim, int32_t n, const flo
  * point count (the reference's ClusterProperties::cluster sizes,
  * data_structures/ClusterProperties.hpp:19-51).  *n_clusters_out (host, optional) = max label
  * + 1; more clusters than `capacity` gives CLUE_ERR_CAPACITY with *n_clusters_out set
- * (capacity 0 with centroids NULL asks for the count alone).  Allocates its temporaries and
- * synchronises `stream`.
+ * (capacity 0 with centroids NULL asks for the count alone).  Its temporaries stay with the
+ * context (they grow on demand); the call synchronises `stream`.
  */
 clue_status clue_cluster_centroids(clue_context ctx, int32_t ndim, int32_t n, const float* coords,
                                    const int32_t* cluster_index, int32_t capacity, float* centroids,

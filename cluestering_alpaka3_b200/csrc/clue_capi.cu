@@ -415,6 +415,18 @@ clue_status clusters_csr(Workspace& ws, int n, const int32_t* cluster_index, int
 
 using namespace clue_b200;
 
+// An executable graph kept for the next call's pipeline, and the cluster size of its k_build launch:
+// an update in place keeps a kernel node's cluster size, so each size has an executable of its own.
+struct GraphSlot {
+  static constexpr int kSizes = 5;  // none, 1, 2, 4, 8 CTAs
+  cudaGraphExec_t exec[kSizes] = {};
+  cudaGraphExec_t& at(int ranks) { return exec[ranks >= 8 ? 4 : (ranks >= 4 ? 3 : ranks)]; }
+  void destroy() {
+    for (auto& e : exec)
+      if (e) cudaGraphExecDestroy(e);
+  }
+};
+
 struct clue_context_s {
   Workspace ws;
   // A second workspace and stream for the odd chunks of an overlapped host-memory batch, so that
@@ -424,10 +436,10 @@ struct clue_context_s {
   // The overlapped host batch's even chunks run on chunk_stream (a stream of the context, so a
   // caller's legacy default stream never has to be captured), and every chunk's pipeline is
   // captured into a graph whose executable is kept here and updated in place on the next call.
-  cudaGraphExec_t chunk_exec[Workspace::kPipeMaxChunks] = {};
+  GraphSlot chunk_exec[Workspace::kPipeMaxChunks];
   cudaStream_t chunk_stream = nullptr;
   // the same for the pipeline of a blocking call (run_pipeline_graph)
-  cudaGraphExec_t plain_exec = nullptr;
+  GraphSlot plain_exec;
   cudaEvent_t plain_ev[2] = {};
 };
 
@@ -436,9 +448,9 @@ Workspace& context_workspace(clue_context ctx) { return ctx->ws; }
 }  // namespace clue_b200
 
 // Captures the pipeline enqueued by run_pipeline_dispatch on `g` into a graph and launches it
-// there, keeping the executable in *exec (updated in place when the captured graph has the same
+// there, keeping the executable in *slot (updated in place when the captured graph has the same
 // shape, else instantiated again).
-static clue_status capture_and_launch(Workspace& w, const RunArgs& a, cudaStream_t g, cudaGraphExec_t* exec) {
+static clue_status capture_and_launch(Workspace& w, const RunArgs& a, cudaStream_t g, GraphSlot* slot) {
   const bool timing = w.timing;
   w.timing = false;
   cudaGraph_t cg = nullptr;
@@ -450,6 +462,7 @@ static clue_status capture_and_launch(Workspace& w, const RunArgs& a, cudaStream
   }
   w.timing = timing;
   if (ce == cudaSuccess && st == CLUE_OK) {
+    cudaGraphExec_t* exec = &slot->at(w.build_ranks);
     cudaGraphExecUpdateResultInfo ui;
     if (!*exec || cudaGraphExecUpdate(*exec, cg, &ui) != cudaSuccess) {
       cudaGetLastError();
@@ -715,9 +728,8 @@ clue_status clue_context_destroy(clue_context ctx) {
   }
   if (ctx->alt_stream) cudaStreamDestroy(ctx->alt_stream);
   if (ctx->chunk_stream) cudaStreamDestroy(ctx->chunk_stream);
-  for (auto& ge : ctx->chunk_exec)
-    if (ge) cudaGraphExecDestroy(ge);
-  if (ctx->plain_exec) cudaGraphExecDestroy(ctx->plain_exec);
+  for (auto& slot : ctx->chunk_exec) slot.destroy();
+  ctx->plain_exec.destroy();
   for (auto& e : ctx->plain_ev)
     if (e) cudaEventDestroy(e);
   cudaSetDevice(prev);
@@ -1061,6 +1073,7 @@ static clue_status prepare_batch(clue_context ctx, const clue_params* params, co
     return CLUE_ERR_INVALID_ARG;
   }
   int64_t tiles = 0;
+  a.max_points = a.max_tiles = 0;
   for (int e = 0; e < n_events; ++e) {
     const int64_t ne = (int64_t)ev_off[e + 1] - ev_off[e];
     if (ne <= 0) {
@@ -1074,6 +1087,8 @@ static clue_status prepare_batch(clue_context ctx, const clue_params* params, co
       return CLUE_ERR_CAPACITY;
     }
     tiles += nt;
+    a.max_points = std::max(a.max_points, (int32_t)ne);
+    a.max_tiles = std::max(a.max_tiles, nt);
   }
   const int64_t n = ev_off[n_events];
   if (tiles > 2147483000ll || n > 2147483000ll) {

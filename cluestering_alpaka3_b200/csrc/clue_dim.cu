@@ -86,6 +86,11 @@ __device__ __forceinline__ float warp_max_f(float v) {
   return r;
 }
 
+// Entry p of an order; a null order is the identity.
+__device__ __forceinline__ int order_at(const int32_t* __restrict__ order, int p) {
+  return order ? __ldg(order + p) : p;
+}
+
 // Largest e in [0, E) with base[e] <= x.
 __device__ __forceinline__ int find_event(const int32_t* __restrict__ base, int E, int x) {
   int lo = 0, hi = E - 1;
@@ -204,56 +209,6 @@ __device__ __forceinline__ void write_block_box(float4* __restrict__ blk, int b,
   }
 }
 
-// Bounding box (and largest payload) of every 32 consecutive tile-sorted records.
-template <int N>
-__global__ void __launch_bounds__(256) k_block_bbox(const float4* __restrict__ rec, int n, float4* __restrict__ blk) {
-  const int lane = threadIdx.x & 31;
-  const int nblk = (n + 31) >> 5;
-  const int wstride = (gridDim.x * blockDim.x) >> 5;
-  for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nblk; b += wstride) {
-    const int q = (b << 5) + lane;
-    float x[N], pl;
-    load_rec<N>(rec, q < n ? q : b << 5, x, pl);  // lanes past the end duplicate the first record
-    write_block_box<N>(blk, b, x, pl);
-  }
-}
-
-// Bounding boxes of super-blocks (32 consecutive blocks = 1024 records) from the block boxes.
-template <int N>
-__global__ void __launch_bounds__(256) k_superblock_bbox(const float4* __restrict__ blk, int n,
-                                                         float4* __restrict__ sblk) {
-  constexpr int BW = Blk<N>::kWords;
-  const int lane = threadIdx.x & 31;
-  const int nblk = (n + 31) >> 5;
-  const int nsb = (nblk + 31) >> 5;
-  const int wstride = (gridDim.x * blockDim.x) >> 5;
-  for (int sb = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; sb < nsb; sb += wstride) {
-    const int b = min((sb << 5) + lane, nblk - 1);
-    float v[4 * BW];
-#pragma unroll
-    for (int k = 0; k < BW; ++k) {
-      const float4 t4 = __ldg(blk + (size_t)b * BW + k);
-      v[4 * k] = t4.x;
-      v[4 * k + 1] = t4.y;
-      v[4 * k + 2] = t4.z;
-      v[4 * k + 3] = t4.w;
-    }
-#pragma unroll
-    for (int d = 0; d < N; ++d) {
-      v[d] = warp_min_f(v[d]);
-      v[N + d] = warp_max_f(v[N + d]);
-    }
-    v[2 * N] = warp_max_f(v[2 * N]);
-    if (lane < BW) {
-      float4 out;
-#pragma unroll
-      for (int k = 0; k < BW; ++k)
-        if (k == lane) out = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-      sblk[(size_t)sb * BW + lane] = out;
-    }
-  }
-}
-
 template <int N>
 __device__ __forceinline__ void load_box(const float4* __restrict__ a, int i, float* bb) {
   constexpr int BW = Blk<N>::kWords;
@@ -280,7 +235,7 @@ __device__ __forceinline__ void stage_block(float4* sm, const float4* __restrict
   if (lane < cnt) {
 #pragma unroll
     for (int k = 0; k < W; ++k) sm[lane * W + k] = __ldg(rec + (size_t)(p0 + lane) * W + k);
-    if (sq) sq[lane] = __ldg(mq + p0 + lane);
+    if (sq) sq[lane] = order_at(mq, p0 + lane);
   }
   __syncwarp();
 }
@@ -475,10 +430,11 @@ __device__ __forceinline__ void spatial_sweep(const KParams& kp, const EvGrid* _
 // Resets the per-call state; for a plain call also writes the event table of its one event.
 template <int N>
 __global__ void k_init(const KParams kp, Events ev, int32_t* ev_pt, int32_t* ev_tile, uint32_t* seed_bits,
-                       DevStatus* st) {
+                       uint32_t* chunk_total, DevStatus* st) {
   if (blockIdx.x == 0) {
     uint32_t* s = reinterpret_cast<uint32_t*>(st);
     for (int k = threadIdx.x; k < (int)(sizeof(DevStatus) / 4); k += blockDim.x) s[k] = 0u;
+    if (chunk_total && threadIdx.x == 0) *chunk_total = (uint32_t)(kp.n / kChunk + kp.ntiles + 1);
   }
   const int stride = gridDim.x * blockDim.x;
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < (kp.n + 31) / 32; w += stride) seed_bits[w] = 0u;
@@ -790,11 +746,9 @@ __global__ void __launch_bounds__(256) k_bin(const KParams kp, InPtrs in, Events
 
 template <int N>
 __global__ void __launch_bounds__(256) k_gather(InPtrs in, int n, const int32_t* __restrict__ perm,
-                                                float4* __restrict__ rec_w, DevStatus* st,
-                                                int32_t* __restrict__ ida, int32_t* __restrict__ idb) {
+                                                float4* __restrict__ rec_w, DevStatus* st) {
   const int stride = gridDim.x * blockDim.x;
   for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < n; pos += stride) {
-    if (ida) ida[pos] = idb[pos] = pos;  // identity orders, when asked for
     const int i = perm[pos];
     if (dcheck_bad(st, i, n, kChkGatherPerm)) continue;
     float x[N];
@@ -918,12 +872,6 @@ __global__ void __launch_bounds__(256) k_bin_composite(const KParams kp, InPtrs 
   }
 }
 
-// Inverse permutation: minv[mq[p]] = p.
-__global__ void __launch_bounds__(256) k_invert(const int32_t* __restrict__ mq, int n, int32_t* __restrict__ minv) {
-  const int stride = gridDim.x * blockDim.x;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride) minv[mq[p]] = p;
-}
-
 template <int N>
 __global__ void __launch_bounds__(256) k_gather_morton(const float4* __restrict__ rec_r, int n,
                                                        const int32_t* __restrict__ mq, float4* __restrict__ rec_m) {
@@ -934,6 +882,412 @@ __global__ void __launch_bounds__(256) k_gather_morton(const float4* __restrict_
 #pragma unroll
     for (int k = 0; k < W; ++k) rec_m[(size_t)p * W + k] = __ldg(rec_r + (size_t)q * W + k);
   }
+}
+
+// ---- stage 1 in one launch: events of up to kBuildPoints points -----------------
+// A cluster of CTAs takes one event through the whole stage: bounding box, grid, tile and Morton keys,
+// the stable radix sorts, records, tile offsets, chunks and the symmetric density's block boxes.
+// Its CTAs exchange digit counts through distributed shared memory and the keys through L2, with a
+// cluster barrier between steps.  Bound by the latency of its steps (a radix pass of 16k points takes
+// about 5 us, one of 1000 points 2 us), where a launch takes 2 to 3 us: stage 1 of a flat event was
+// 24 launches, 125 us of direct launches for 16k points against 42 us, 180 against 92 us for 50k.
+
+// Shared memory of one CTA of a build cluster.
+template <int N, int W>
+struct BuildSmem {
+  uint32_t cnt[W][kRadix];  // digit counters of every warp, then its next positions
+  uint32_t tot[2][kRadix];  // digit counts of the CTA, read by the other CTAs (two passes in turn)
+  uint32_t scan[33];
+  uint32_t red[W][2 * N + 2];
+  uint32_t box[2 * N + 2];  // the CTA's part of the bounding box
+  float mn[N], size[N], mx[N];
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// The address of a shared-memory word of the cluster's CTA `rank`, and a load from it.
+__device__ __forceinline__ uint32_t load_remote(const uint32_t* p, uint32_t rank) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r, v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(r) : "memory");
+  return v;
+}
+
+// Block-wide exclusive scan of one value per thread over W warps; the total goes to *tot.
+template <int W>
+__device__ __forceinline__ uint32_t build_scan(uint32_t* s, uint32_t v, int lane, int warp, uint32_t* tot) {
+  uint32_t inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31) s[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t x = lane < W ? s[lane] : 0u;
+    uint32_t xi = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, xi, o);
+      if (lane >= o) xi += t;
+    }
+    s[lane] = xi - x;
+    if (lane == 31) s[32] = xi;
+  }
+  __syncthreads();
+  const uint32_t r = s[warp] + inc - v;
+  *tot = s[32];
+  __syncthreads();
+  return r;
+}
+
+// One stable radix pass over the event's n (key, value) pairs by the digit at `shift`; a null vin
+// stands for the points pt..pt+n-1.  Warp w of the cluster takes the pairs [w L, w L + L) in order.
+template <int N, int W>
+__device__ void build_pass(BuildSmem<N, W>& sm, int pass, const uint32_t* kin, const int32_t* vin, uint32_t* kout,
+                           int32_t* vout, int n, int pt, int shift, uint32_t rank, uint32_t ranks, int lane, int warp) {
+  constexpr int K = 4;  // loads in flight per lane
+  const int L = ((n + (int)ranks * W - 1) / ((int)ranks * W) + 31) & ~31;
+  const int b = min(n, ((int)rank * W + warp) * L), e = min(n, b + L);
+  uint32_t* cnt = sm.cnt[warp];
+  for (int d = lane; d < kRadix; d += 32) cnt[d] = 0u;
+  __syncwarp();
+  for (int i0 = b + lane; i0 < e; i0 += 32 * K) {
+    uint32_t k[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) k[j] = i0 + 32 * j < e ? __ldcg(kin + i0 + 32 * j) : 0u;
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+      if (i0 + 32 * j < e) atomicAdd(&cnt[(k[j] >> shift) & (kRadix - 1)], 1u);
+  }
+  __syncthreads();
+  const int t = threadIdx.x;
+  uint32_t* tot = sm.tot[pass & 1];
+  if (t < kRadix) {
+    uint32_t run = 0;
+#pragma unroll 8
+    for (int w = 0; w < W; ++w) {
+      const uint32_t c = sm.cnt[w][t];
+      sm.cnt[w][t] = run;
+      run += c;
+    }
+    tot[t] = run;
+  }
+  cluster_barrier();
+  uint32_t before = 0, all = 0;
+  if (t < kRadix) {
+    for (uint32_t r = 0; r < ranks; ++r) {
+      const uint32_t v = load_remote(tot + t, r);
+      before += r < rank ? v : 0u;
+      all += v;
+    }
+  }
+  uint32_t sum;
+  const uint32_t base = build_scan<W>(sm.scan, t < kRadix ? all : 0u, lane, warp, &sum) + before;
+  if (t < kRadix) {
+#pragma unroll 8
+    for (int w = 0; w < W; ++w) sm.cnt[w][t] += base;
+  }
+  __syncthreads();
+  const uint32_t lt = (1u << lane) - 1u;
+  for (int i0 = b; i0 < e; i0 += 32 * K) {
+    uint32_t k[K];
+    int32_t v[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const int i = i0 + 32 * j + lane;
+      k[j] = i < e ? __ldcg(kin + i) : 0u;
+      v[j] = i < e ? (vin ? __ldcg(vin + i) : pt + i) : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      if (i0 + 32 * j >= e) break;
+      const bool valid = i0 + 32 * j + lane < e;
+      const uint32_t d = (k[j] >> shift) & (kRadix - 1);
+      uint32_t peers = __ballot_sync(0xffffffffu, valid);
+      peers = valid ? peers : ~peers;
+#pragma unroll
+      for (int bit = 0; bit < kRadixBits; ++bit) {
+        const bool one = (d >> bit) & 1u;
+        const uint32_t bb = __ballot_sync(0xffffffffu, one);
+        peers &= one ? bb : ~bb;
+      }
+      const uint32_t place = valid ? cnt[d] + (uint32_t)__popc(peers & lt) : 0u;
+      __syncwarp();
+      if (valid) {
+        if ((peers & lt) == 0) cnt[d] += (uint32_t)__popc(peers);
+        kout[place] = k[j];
+        vout[place] = v[j];
+      }
+      __syncwarp();
+    }
+  }
+  cluster_barrier();
+}
+
+// Records of a build cluster's arrays, written by other CTAs of the cluster in this launch.
+template <int N>
+__device__ __forceinline__ void load_rec_cg(const float4* rec, int pos, float* x, float& payload) {
+  constexpr int WD = Rec<N>::kWords;
+  float buf[4 * WD];
+#pragma unroll
+  for (int k = 0; k < WD; ++k) {
+    const float4 v = __ldcg(rec + (size_t)pos * WD + k);
+    buf[4 * k] = v.x, buf[4 * k + 1] = v.y, buf[4 * k + 2] = v.z, buf[4 * k + 3] = v.w;
+  }
+#pragma unroll
+  for (int d = 0; d < N; ++d) x[d] = buf[d];
+  payload = buf[Rec<N>::kPayload];
+}
+
+// The buffers of k_build; `two` sorts give the tile order by index and the Morton order, one the
+// (tile, Morton) order alone (the symmetric density's).
+struct BuildBufs {
+  uint32_t *k0, *k1, *k2;   // keys: composite keys, the other buffer of their sort, first pass of the tile sort
+  int32_t *va, *vb;         // values of the composite sort, pass by pass
+  int32_t *perm, *vt;       // result of the tile sort, its first pass
+  int32_t* inv;             // tile-sorted position of every point
+  float4* rec_w;
+  int32_t* off;
+  uint32_t *chunk_off, *tblk_off;
+  int32_t* chunk_tile;
+  uint32_t* chunk_total;
+  float4* tblk;
+  int64_t* rho_fix;
+  uint32_t* seed_bits;
+  int32_t *ev_pt, *ev_tile, *ev_chunk;
+  DevStatus* st;
+};
+
+template <int N, int W>
+__global__ void __launch_bounds__(32 * W) k_build(const KParams kp, InPtrs in, EvGrid* eg, BuildBufs o, bool two,
+                                                  int mbits, int tile_passes, int passes, int want_ranks) {
+  __shared__ BuildSmem<N, W> sm;
+  uint32_t rank, ranks;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+  if ((int)ranks != want_ranks) {  // not the launch that was asked for: nothing is touched
+    if (blockIdx.x == 0 && threadIdx.x == 0) o.st->check_site = kChkBuildCluster, o.st->check_index = (int)ranks;
+    return;
+  }
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  const int e = blockIdx.x / ranks;
+  EvGrid* g = eg + e;
+  const bool single = kp.n_events == 1;
+  const int n = single ? kp.n : g->pt_count, pt = single ? 0 : g->pt_base;
+  const int ntiles = single ? kp.ntiles : g->ntiles, tile_base = single ? 0 : g->tile_base;
+  const int npd = single ? kp.nperdim0 : g->nperdim;
+  const int tid = rank * (32 * W) + threadIdx.x, step = ranks * (32 * W);
+  // the call's state (k_init's work; a batch runs k_init before)
+  if (single) {
+    if (rank == 0)
+      for (int k = threadIdx.x; k < (int)(sizeof(DevStatus) / 4); k += 32 * W) reinterpret_cast<uint32_t*>(o.st)[k] = 0u;
+    for (int k = tid; k < (n + 31) / 32; k += step) o.seed_bits[k] = 0u;
+    if (tid == 0) {
+      g->nperdim = npd;
+      g->ntiles = ntiles;
+      g->tile_base = 0;
+      g->pt_base = 0;
+      g->pt_count = n;
+      for (int d = 0; d < kMaxDim; ++d) g->stride[d] = kp.stride0[d];
+      o.ev_pt[0] = 0;
+      o.ev_pt[1] = n;
+      o.ev_tile[0] = 0;
+      o.ev_tile[1] = ntiles;
+    }
+  } else if (o.ev_chunk) {
+    for (int c = ((pt + (1 << kEvChunkShift) - 1) >> kEvChunkShift) + tid; c <= (pt + n - 1) >> kEvChunkShift; c += step)
+      o.ev_chunk[c] = e;
+  }
+  if (o.rho_fix)
+    for (int k = tid; k < n; k += step) o.rho_fix[pt + k] = 0;
+  // bounding box, largest |weight|, finite values
+  {
+    uint32_t emn[N], emx[N], wmax = 0u;
+    bool bad = false;
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+      emn[d] = 0xffffffffu;
+      emx[d] = 0u;
+    }
+#pragma unroll 2
+    for (int i = tid; i < n; i += step) {
+#pragma unroll
+      for (int d = 0; d < N; ++d) {
+        const float x = in.c[d][pt + i];
+        bad |= !isfinite(x);
+        const uint32_t u = enc_float(x);
+        emn[d] = min(emn[d], u);
+        emx[d] = max(emx[d], u);
+      }
+      const float w = in.w[pt + i];
+      bad |= !isfinite(w);
+      wmax = max(wmax, __float_as_uint(fabsf(w)));
+    }
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+      const uint32_t a = warp_min_u(emn[d]), z = warp_max_u(emx[d]);
+      if (lane == 0) {
+        sm.red[warp][d] = ~a;  // every entry is combined by maximum
+        sm.red[warp][N + d] = z;
+      }
+    }
+    wmax = warp_max_u(wmax);
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) {
+      sm.red[warp][2 * N] = wmax;
+      sm.red[warp][2 * N + 1] = bad ? 1u : 0u;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * N + 2) {
+      uint32_t v = 0u;
+      for (int w = 0; w < W; ++w) v = max(v, sm.red[w][threadIdx.x]);
+      sm.box[threadIdx.x] = v;
+    }
+    cluster_barrier();
+    if (threadIdx.x < 2 * N + 2) {
+      uint32_t v = 0u;
+      for (uint32_t r = 0; r < ranks; ++r) v = max(v, load_remote(sm.box + threadIdx.x, r));
+      sm.red[0][threadIdx.x] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+      const int d = threadIdx.x;
+      // tile size (max - min) / nperdim in FP32 (ComputeTiles.hpp:20-23)
+      const float mn = dec_float(~sm.red[0][d]), mx = dec_float(sm.red[0][N + d]);
+      const float size = fdiv(fsub(mx, mn), (float)npd);
+      sm.mn[d] = mn;
+      sm.mx[d] = mx;
+      sm.size[d] = size;
+      if (rank == 0) {
+        g->mn[d] = mn;
+        g->mx[d] = mx;
+        g->size[d] = size;
+      }
+    }
+    if (rank == 0 && threadIdx.x == 32) {
+      g->seed_candidates = 0;
+      g->wmax_bits = sm.red[0][2 * N];
+      if (sm.red[0][2 * N + 1]) atomicOr(&o.st->nonfinite, 1u);
+    }
+    __syncthreads();
+  }
+  // composite keys: tile of the event's grid, then the Morton code inside the tile
+  {
+    constexpr int bpd = MortonBits<N>::kPerDim;
+    const float scale = (float)(1u << bpd);
+    for (int i = tid; i < n; i += step) {
+      int gb = 0;
+      uint32_t m = 0;
+#pragma unroll
+      for (int d = 0; d < N; ++d) {
+        float x = in.c[d][pt + i];
+        if (kp.wrapped[d]) x = normalize_coord(x, sm.mn[d], sm.mx[d]);
+        const float q = fdiv(fsub(x, sm.mn[d]), sm.size[d]);
+        int b = cvt_i32(q);
+        b = b < npd - 1 ? b : npd - 1;
+        b = b > 0 ? b : 0;
+        gb = gb * npd + b;
+        int c = sm.size[d] > 0.0f ? (int)((q - (float)b) * scale) : 0;
+        c = c < 0 ? 0 : (c > (1 << bpd) - 1 ? (1 << bpd) - 1 : c);
+        m |= spread_bits<N>((uint32_t)c) << d;
+      }
+      o.k0[pt + i] = ((uint32_t)gb << mbits) | (m >> (MortonBits<N>::kBits - mbits));
+    }
+  }
+  cluster_barrier();
+  int pass = 0;
+  if (two) {
+    for (int p = 0; p < tile_passes; ++p, ++pass) {
+      const bool last = p + 1 == tile_passes;
+      build_pass<N, W>(sm, pass, p == 0 ? o.k0 + pt : o.k2 + pt, p == 0 ? nullptr : o.vt + pt, last ? o.k1 + pt : o.k2 + pt,
+                       last ? o.perm + pt : o.vt + pt, n, pt, mbits + 8 * p, rank, ranks, lane, warp);
+    }
+  }
+  for (int p = 0; p < passes; ++p, ++pass)
+    build_pass<N, W>(sm, pass, (p & 1 ? o.k1 : o.k0) + pt, p == 0 ? nullptr : (p & 1 ? o.va : o.vb) + pt,
+                     (p & 1 ? o.k0 : o.k1) + pt, (p & 1 ? o.vb : o.va) + pt, n, pt, 8 * p, rank, ranks, lane, warp);
+  const uint32_t* sorted = (passes & 1 ? o.k1 : o.k0) + pt;
+  const int32_t* by_morton = (passes & 1 ? o.va : o.vb) + pt;
+  int32_t* mq = (passes & 1 ? o.vb : o.va) + pt;
+  // records, tile offsets
+  for (int base = tid & ~31; base <= n; base += step) {
+    const int q = base + lane;
+    int prev = 0, cur = -1;  // tiles that start at q: prev + 1 .. cur
+    if (q <= n) {
+      prev = q > 0 ? (int)(__ldcg(sorted + q - 1) >> mbits) : -1;
+      cur = q < n ? (int)(__ldcg(sorted + q) >> mbits) : ntiles;
+    }
+    const bool far = cur - prev > 32;
+    if (!far)
+      for (int t = prev + 1; t <= cur; ++t) o.off[tile_base + t] = pt + q;
+    for (unsigned m = __ballot_sync(0xffffffffu, far); m; m &= m - 1) {
+      const int src = __ffs(m) - 1;
+      const int p = __shfl_sync(0xffffffffu, prev, src), c = __shfl_sync(0xffffffffu, cur, src);
+      for (int t = p + 1 + lane; t <= c; t += 32) o.off[tile_base + t] = pt + base + src;
+    }
+    if (q < n) {
+      const int i = __ldcg(two ? o.perm + pt + q : by_morton + q);
+      if (!dcheck_bad(o.st, i, kp.n, kChkGatherPerm)) {
+        float x[N];
+#pragma unroll
+        for (int d = 0; d < N; ++d) x[d] = in.c[d][i];
+        store_rec<N>(o.rec_w, pt + q, x, in.w[i]);
+        if (two) o.inv[i] = pt + q;
+      }
+    }
+  }
+  cluster_barrier();
+  if (two)
+    for (int p = tid; p < n; p += step) {
+      const int i = __ldcg(by_morton + p);
+      if (!dcheck_bad(o.st, i, kp.n, kChkGatherPerm)) mq[p] = __ldcg(o.inv + i);
+    }
+  // chunks of kChunk home points and blocks of 32 points of every tile; an event of a batch has the
+  // slots that its points and tiles can need at most, the unused ones are marked
+  const int slot0 = single ? 0 : pt / kChunk + tile_base, blk0 = single ? 0 : pt / 32 + tile_base;
+  if (rank == 0) {
+    uint32_t chunks = 0, blocks = 0;
+    for (int t0 = 0; t0 < ntiles; t0 += 32 * W) {
+      const int t = t0 + (int)threadIdx.x;
+      const int cnt = t < ntiles ? __ldcg(o.off + tile_base + t + 1) - __ldcg(o.off + tile_base + t) : 0;
+      const uint32_t nch = (uint32_t)((cnt + kChunk - 1) / kChunk), nbl = (uint32_t)((cnt + 31) / 32);
+      uint32_t sum;
+      const uint32_t ce = chunks + build_scan<W>(sm.scan, nch, lane, warp, &sum);
+      chunks += sum;
+      const uint32_t be = blocks + build_scan<W>(sm.scan, nbl, lane, warp, &sum);
+      blocks += sum;
+      if (t < ntiles) {
+        o.chunk_off[tile_base + t] = (uint32_t)slot0 + ce;
+        if (o.tblk_off) o.tblk_off[tile_base + t] = (uint32_t)blk0 + be;
+        for (uint32_t c = 0; c < nch; ++c) o.chunk_tile[slot0 + ce + c] = tile_base + t;
+      }
+    }
+    if (single) {
+      if (threadIdx.x == 0) *o.chunk_total = chunks;
+    } else {
+      const int end = e + 1 < kp.n_events ? (pt + n) / kChunk + tile_base + ntiles : kp.n / kChunk + kp.ntiles + 1;
+      for (int c = slot0 + (int)chunks + (int)threadIdx.x; c < end; c += 32 * W) o.chunk_tile[c] = -1;
+    }
+    if (threadIdx.x == 0) sm.scan[0] = chunks;
+  }
+  if (!o.tblk) return;  // (no CTA reads another's shared memory any more)
+  cluster_barrier();
+  const int nblocks = kChunkWarps * (int)load_remote(sm.scan, 0);
+  for (int sl = rank * W + warp; sl < nblocks; sl += ranks * W) {
+    const int t = __ldcg(o.chunk_tile + slot0 + sl / kChunkWarps);
+    const int b = (slot0 + sl / kChunkWarps - (int)__ldcg(o.chunk_off + t)) * kChunkWarps + sl % kChunkWarps;
+    const int first = __ldcg(o.off + t) + (b << 5);
+    const int cnt = min(32, __ldcg(o.off + t + 1) - first);
+    if (cnt <= 0) continue;
+    float x[N], w;
+    load_rec_cg<N>(o.rec_w, first + min(lane, cnt - 1), x, w);
+    write_block_box<N>(o.tblk, (int)__ldcg(o.tblk_off + t) + b, x, w);
+  }
+  cluster_barrier();  // sm.scan[0] of the first CTA is read by all
 }
 
 // ---- chunks ---------------------------------------------------------------------
@@ -977,6 +1331,7 @@ __device__ __forceinline__ bool chunk_home(const KParams& kp, Events ev, const i
   const int w = blockIdx.x;
   if (w >= (int)*chunk_total) return false;
   h.t = chunk_tile[w];
+  if (h.t < 0) return false;  // a slot that its event does not need (k_build)
   const int beg = off[h.t];
   // slots are event-major: the tile's first one lies among its event's points
   h.g = ev.eg + event_of(ev.pt, ev.chunk_ev, kp.n_events, beg);
@@ -1014,7 +1369,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4)) k_density(
   const bool valid = h.valid;
   if (!__any_sync(0xffffffffu, valid)) return;
   const int lane = lane_id(), warp = threadIdx.x >> 5;
-  const int pos = mq[h.p];
+  const int pos = order_at(mq, h.p);
   float x[N], wi;
   load_rec<N>(rec_w, pos, x, wi);
   int hb[N], lo[N], hi[N], wl[N], wh[N];
@@ -1198,8 +1553,8 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
       int orig_j = -1;
       bool higher = rho_j > rho_i;
       if (!higher && rho_j > 0.0f) {
-        orig_j = __ldg(perm + __ldg(mq + p));
-        higher = orig_j > __ldg(perm + __ldg(mq + h.p));
+        orig_j = __ldg(perm + order_at(mq, p));
+        higher = orig_j > __ldg(perm + order_at(mq, h.p));
       }
       if (!higher) return;
       bool better;
@@ -1215,8 +1570,8 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
         } else if (TIE == CLUE_TIE_REFERENCE && rank != rank_best) {
           better = rank < rank_best;
         } else {
-          if (orig_j < 0) orig_j = __ldg(perm + __ldg(mq + p));
-          const int orig_best = __ldg(perm + __ldg(mq + nh));
+          if (orig_j < 0) orig_j = __ldg(perm + order_at(mq, p));
+          const int orig_best = __ldg(perm + order_at(mq, nh));
           if (TIE == CLUE_TIE_REFERENCE) {
             better = orig_j < orig_best;
           } else {
@@ -1318,9 +1673,9 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
   // which +inf decides the same way.
   const float dist = nh >= 0 ? M::finish(s_best) : INFINITY;
   const bool seed = valid && dist > kp.seed_dc && rho_i >= kp.rhoc;
-  const int pos = mq[h.p];
+  const int pos = order_at(mq, h.p);
   if (valid) {
-    const int nhq = nh >= 0 ? mq[nh] : -1;
+    const int nhq = nh >= 0 ? order_at(mq, nh) : -1;
     sb.par[pos] = seed ? -1 : nhq;
     if (sb.nh) sb.nh[pos] = nhq;
     const int i = perm[pos];
@@ -1369,20 +1724,20 @@ enum { kDensGeneric = 0, kDensExpUnit = 1, kDensGauss0Unit = 2 };
 // that no lane of the warp holds within dc skip the kernel evaluation.
 template <int N, int MT, int FORM>
 __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileThreads) k_density_spatial(
-    const KParams kp, Events ev, const int32_t* __restrict__ off, const int32_t* __restrict__ ord,
-    const int32_t* __restrict__ chunk_tile, const uint32_t* __restrict__ chunk_off,
-    const uint32_t* __restrict__ chunk_total, const float4* __restrict__ rec_w, const float4* __restrict__ rec_m,
+    const KParams kp, Events ev, const int32_t* __restrict__ off, const int32_t* __restrict__ chunk_tile,
+    const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ chunk_total,
+    const float4* __restrict__ rec_m,
     const int32_t* __restrict__ mq, const float4* __restrict__ blk, const float4* __restrict__ sblk,
-    float4* __restrict__ rec_r, const int32_t* __restrict__ minv, float kexp) {
+    float4* __restrict__ rec_r, float kexp) {
   using M = Metric<N, MT>;
   __shared__ float4 s_rec[kTileThreads / 32][32 * Rec<N>::kWords];
   ChunkHome h;
   if (!chunk_home(kp, ev, off, chunk_tile, chunk_off, chunk_total, h)) return;
-  const int pos = ord[h.p];
+  const int pos = order_at(mq, h.p);
   const bool valid = h.valid;
   float x[N], wi;
-  load_rec<N>(rec_w, pos, x, wi);
-  const int p_home = minv[pos];
+  load_rec<N>(rec_m, h.p, x, wi);
+  const int p_home = h.p;
   int hb[N], lo[N], hi[N];
   home_bins<N>(h.g, h.t, hb);
   lane_box<N>(kp, h.g, x, kp.dc, hb, lo, hi);
@@ -1511,6 +1866,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
   if (c >= (int)*chunk_total) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = chunk_tile[c];
+  if (t < 0) return;  // a slot that its event does not need (k_build)
   const int a_loc = (c - (int)chunk_off[t]) * kChunkWarps + warp;  // block of the tile
   const int startA = off[t] + (a_loc << 5);
   const int cntA = min(32, off[t + 1] - startA);
@@ -1643,7 +1999,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
         acc = fadd(acc, fadd(acc2.x, acc2.y));
         const float cacc = fadd(cacc2.x, cacc2.y);
         if (cv && cacc != 0.0f) {
-          const int mi = mq[first + lane];
+          const int mi = order_at(mq, first + lane);
           if (!dcheck_bad(st, mi, kp.n, kChkDensityMirror))
             atomicAdd(reinterpret_cast<unsigned long long*>(rho_fix + mi), (unsigned long long)__float2ll_rn(cacc * scale));
         }
@@ -1659,7 +2015,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
     }
     if (d < 0) break;
   }
-  if (hv) store_rec<N>(rec_r, mq[pA], x, acc);
+  if (hv) store_rec<N>(rec_r, order_at(mq, pA), x, acc);
 }
 
 // rho = own-side sum + the fixed-point sum of the contributions received as a candidate.
@@ -1678,28 +2034,70 @@ __global__ void __launch_bounds__(256) k_density_combine(const KParams kp, Event
   }
 }
 
-// The symmetric density's fixed-point sums added in (as k_density_combine) and the block
-// boxes with the final densities (as k_block_bbox) in one pass over the records, for the
-// composite sort whose tile-ordered records are also the Morton-ordered ones.
-template <int N>
-__global__ void __launch_bounds__(256) k_combine_block_bbox(const KParams kp, Events ev, int n,
-                                                            const int64_t* __restrict__ rho_fix,
-                                                            float4* __restrict__ rec_r, float kmax,
-                                                            float4* __restrict__ blk) {
-  const int lane = threadIdx.x & 31;
-  const int nblk = (n + 31) >> 5;
-  const int wstride = (gridDim.x * blockDim.x) >> 5;
-  for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nblk; b += wstride) {
+// Boxes (and largest payloads) of every block of 32 and every super-block of 1024 Morton-ordered
+// records, one CTA per super-block.  GATHER takes the records through the order mq into rec_m
+// first; otherwise rec is in Morton order (a composite sort) and its densities get the symmetric
+// sweep's fixed-point sums added in (as k_density_combine does).
+template <int N, bool GATHER>
+__global__ void __launch_bounds__(1024) k_boxes(const KParams kp, Events ev, const int32_t* __restrict__ mq,
+                                                float4* rec, float4* __restrict__ rec_m,
+                                                const int64_t* __restrict__ rho_fix, float kmax,
+                                                float4* __restrict__ blk, float4* __restrict__ sblk) {
+  constexpr int BW = Blk<N>::kWords;
+  __shared__ float s_box[32][2 * N + 1];
+  const int lane = lane_id(), warp = threadIdx.x >> 5, n = kp.n;
+  const int b = blockIdx.x * 32 + warp, nblk = (n + 31) >> 5;
+  if (b < nblk) {
     const int q = (b << 5) + lane;
     const bool valid = q < n;
-    const int qq = valid ? q : b << 5;
-    bool uniform;
-    const EvGrid* g = ev.eg + warp_event(ev.pt, ev.chunk_ev, kp.n_events, qq, true, uniform);
-    float x[N], acc;
-    load_rec<N>(rec_r, qq, x, acc);
-    const float rho = fadd(acc, (float)((double)rho_fix[qq] * ldexp(1.0, -fix_exponent(g, kmax))));
-    if (valid) store_rec<N>(rec_r, q, x, rho);
-    write_block_box<N>(blk, b, x, rho);
+    const int qq = valid ? q : b << 5;  // lanes past the end repeat the first record
+    float x[N], pl;
+    if (GATHER) {
+      load_rec<N>(rec, mq[qq], x, pl);
+      if (valid) store_rec<N>(rec_m, q, x, pl);
+    } else {
+      bool uniform;
+      const EvGrid* g = ev.eg + warp_event(ev.pt, ev.chunk_ev, kp.n_events, qq, true, uniform);
+      load_rec<N>(rec, qq, x, pl);
+      pl = fadd(pl, (float)((double)rho_fix[qq] * ldexp(1.0, -fix_exponent(g, kmax))));
+      if (valid) store_rec<N>(rec, q, x, pl);
+    }
+    write_block_box<N>(blk, b, x, pl);
+    float lo[N], hi[N];
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+      lo[d] = warp_min_f(x[d]);
+      hi[d] = warp_max_f(x[d]);
+    }
+    pl = warp_max_f(pl);
+    if (lane == 0) {
+#pragma unroll
+      for (int d = 0; d < N; ++d) {
+        s_box[warp][d] = lo[d];
+        s_box[warp][N + d] = hi[d];
+      }
+      s_box[warp][2 * N] = pl;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int w = min(lane, nblk - 1 - (int)blockIdx.x * 32);  // blocks past the end repeat the last one
+    float v[4 * BW];
+#pragma unroll
+    for (int k = 0; k < 4 * BW; ++k) v[k] = 0.0f;
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+      v[d] = warp_min_f(s_box[w][d]);
+      v[N + d] = warp_max_f(s_box[w][N + d]);
+    }
+    v[2 * N] = warp_max_f(s_box[w][2 * N]);
+    if (lane < BW) {
+      float4 out;
+#pragma unroll
+      for (int k = 0; k < BW; ++k)
+        if (k == lane) out = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+      sblk[(size_t)blockIdx.x * BW + lane] = out;
+    }
   }
 }
 
@@ -1712,15 +2110,15 @@ __global__ void __launch_bounds__(256) k_combine_block_bbox(const KParams kp, Ev
 // rho_i - tol |rho_i|, are skipped.
 template <int N, int MT>
 __global__ void __launch_bounds__(kTileThreads) k_near_ties(
-    const KParams kp, Events ev, const int32_t* __restrict__ off, const int32_t* __restrict__ ord,
+    const KParams kp, Events ev, const int32_t* __restrict__ off,
     const int32_t* __restrict__ chunk_tile, const uint32_t* __restrict__ chunk_off,
     const uint32_t* __restrict__ chunk_total, const float4* __restrict__ rec_r, const float4* __restrict__ rec_m,
     const int32_t* __restrict__ mq, const float4* __restrict__ blk, const float4* __restrict__ sblk,
-    const int32_t* __restrict__ minv, const int32_t* __restrict__ nh_s, DevStatus* st) {
+    const int32_t* __restrict__ nh_s, DevStatus* st) {
   using M = Metric<N, MT>;
   ChunkHome h;
   if (!chunk_home(kp, ev, off, chunk_tile, chunk_off, chunk_total, h)) return;
-  const int pos = ord[h.p];
+  const int pos = order_at(mq, h.p);
   const bool valid = h.valid;
   float x[N], rho_i;
   load_rec<N>(rec_r, pos, x, rho_i);
@@ -1746,7 +2144,7 @@ __global__ void __launch_bounds__(kTileThreads) k_near_ties(
     flag = near(rho_nh);
   }
   const float pmin = rho_i - kNearTol * fabsf(rho_i);
-  spatial_sweep<N, M, false>(kp, h.g, off, hb, lo, hi, valid, x, blk, sblk, pmin, minv[pos], [&]() { return bnd; },
+  spatial_sweep<N, M, false>(kp, h.g, off, hb, lo, hi, valid, x, blk, sblk, pmin, h.p, [&]() { return bnd; },
                              [&](int p0, int p1, bool need, int64_t) {
     const int cnt = p1 - p0;
     stage_block<N>(sm, rec_m, p0, cnt, sq, mq);
@@ -1780,20 +2178,16 @@ __device__ __forceinline__ int64_t seed_cap(const KParams& kp, const EvGrid* g) 
 // search.
 
 // Seeds before point i of the original order.
-__device__ __forceinline__ uint32_t seed_rank_of(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ rank,
+__device__ __forceinline__ uint32_t seed_rank_of(const uint32_t* bits, const uint32_t* rank,
                                                  int i) {
   return rank[i >> 5] + (uint32_t)__popc(bits[i >> 5] & ((1u << (i & 31)) - 1u));
 }
 
 // The label of every seed (its rank by index inside its event) written as its root value, and per
 // event the seeds and clusters (optional outputs) with their total in st->n_clusters.
-__global__ void __launch_bounds__(256) k_seed_labels(const KParams kp, Events ev, const uint32_t* __restrict__ bits,
-                                                     const uint32_t* __restrict__ rank,
-                                                     const uint32_t* __restrict__ total,
-                                                     const int32_t* __restrict__ list,
-                                                     const int32_t* __restrict__ perm, int32_t* __restrict__ par,
-                                                     int32_t* __restrict__ n_seeds, int32_t* __restrict__ n_clusters,
-                                                     DevStatus* st) {
+__device__ __forceinline__ void seed_labels(const KParams& kp, Events ev, const uint32_t* bits, const uint32_t* rank,
+                                            const uint32_t* total, const int32_t* list, const int32_t* perm,
+                                            int32_t* par, int32_t* n_seeds, int32_t* n_clusters, DevStatus* st) {
   const int stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
   const int ns = (int)st->n_seeds;
   for (int k = first; k < ns; k += stride) {
@@ -1812,6 +2206,42 @@ __global__ void __launch_bounds__(256) k_seed_labels(const KParams kp, Events ev
     if (n_clusters) n_clusters[e] = (int32_t)nc;
     atomicAdd(&st->n_clusters, (uint32_t)nc);
   }
+}
+
+__global__ void __launch_bounds__(256) k_seed_labels(const KParams kp, Events ev, const uint32_t* __restrict__ bits,
+                                                     const uint32_t* __restrict__ rank,
+                                                     const uint32_t* __restrict__ total,
+                                                     const int32_t* __restrict__ list,
+                                                     const int32_t* __restrict__ perm, int32_t* __restrict__ par,
+                                                     int32_t* __restrict__ n_seeds, int32_t* __restrict__ n_clusters,
+                                                     DevStatus* st) {
+  seed_labels(kp, ev, bits, rank, total, list, perm, par, n_seeds, n_clusters, st);
+}
+
+// The same behind the scan of the seed bits in one block, for calls of up to kScanOneBlock words (a
+// launch less).
+__global__ void __launch_bounds__(1024) k_seed_labels_one(const KParams kp, Events ev, const uint32_t* bits,
+                                                          uint32_t* rank, uint32_t* total, int words,
+                                                          const int32_t* list, const int32_t* perm, int32_t* par,
+                                                          int32_t* n_seeds, int32_t* n_clusters, DevStatus* st) {
+  constexpr int kPer = (int)(kScanOneBlock / 1024);
+  __shared__ uint32_t s_scan[33];
+  const int base = threadIdx.x * kPer;
+  uint32_t c[kPer], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    c[k] = base + k < words ? (uint32_t)__popc(bits[base + k]) : 0u;
+    sum += c[k];
+  }
+  uint32_t all, run = build_scan<32>(s_scan, sum, threadIdx.x & 31, threadIdx.x >> 5, &all);
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    if (base + k < words) rank[base + k] = run;
+    run += c[k];
+  }
+  if (threadIdx.x == 0) *total = all;
+  __syncthreads();
+  seed_labels(kp, ev, bits, rank, total, list, perm, par, n_seeds, n_clusters, st);
 }
 
 // Pointer jumping on the forest: every parent pointer is replaced by its grandparent until it
@@ -1994,8 +2424,8 @@ void launch_nh(const KParams& kp, Workspace& ws, const clue_outputs& out, cudaSt
 template <int N, int MT, int FORM>
 void launch_density_spatial_form(const KParams& kp, Workspace& ws, cudaStream_t s, float kexp) {
   k_density_spatial<N, MT, FORM><<<chunk_grid(kp), kTileThreads, 0, s>>>(
-      kp, events_of(ws), ws.offsets, ws.mq, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_w,
-      ws.rec_m_cur, ws.mq, ws.blk, ws.sblk, ws.rec_r, ws.minv, kexp);
+      kp, events_of(ws), ws.offsets, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_m_cur, ws.mq,
+      ws.blk, ws.sblk, ws.rec_r, kexp);
 }
 template <int N, int MT>
 void launch_density_spatial(const KParams& kp, Workspace& ws, cudaStream_t s) {
@@ -2036,7 +2466,6 @@ void launch_density_sym(const KParams& kp, Workspace& ws, cudaStream_t s, bool f
   if (kp.kernel_type == CLUE_KERNEL_FLAT) kmax = fmaxf(1.0f, fabsf(kp.kpar[0]));
   if (kp.kernel_type == CLUE_KERNEL_EXPONENTIAL) kmax = fmaxf(1.0f, fabsf(kp.kpar[1]));
   if (kp.kernel_type == CLUE_KERNEL_GAUSSIAN) kmax = fmaxf(1.0f, fabsf(kp.kpar[2]));
-  cudaMemsetAsync(ws.rho_fix, 0, (size_t)kp.n * sizeof(int64_t), s);
   if (kp.kernel_type == CLUE_KERNEL_EXPONENTIAL && kp.kpar[1] == 1.0f)
     launch_density_sym_form<N, MT, kDensExpUnit>(kp, ws, s, -kp.kpar[0] * log2e, kmax);
   else if (kp.kernel_type == CLUE_KERNEL_GAUSSIAN && kp.kpar[0] == 0.0f && kp.kpar[2] == 1.0f)
@@ -2070,8 +2499,89 @@ void launch_density_sym_metric(int metric, const KParams& kp, Workspace& ws, cud
 template <int N, int MT>
 void launch_near_ties(const KParams& kp, Workspace& ws, cudaStream_t s) {
   k_near_ties<N, MT><<<chunk_grid(kp), kTileThreads, 0, s>>>(
-      kp, events_of(ws), ws.offsets, ws.mq, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_r, ws.rec_m_cur,
-      ws.mq, ws.blk, ws.sblk, ws.minv, ws.nh_s, ws.status);
+      kp, events_of(ws), ws.offsets, ws.chunk_tile, ws.chunk_count, ws.chunk_total, ws.rec_r, ws.rec_m_cur,
+      ws.mq, ws.blk, ws.sblk, ws.nh_s, ws.status);
+}
+
+// Whether k_build takes the call: keys of 32 bits, and sizes where a few clusters beat the whole
+// chip's separate launches.  Whole calls, k_build against separate launches: one flat 2-D event of 16k
+// points 133 against 207 us, 40k 186 / 233, 65k 216 / 232, 100k 285 / 262; 24 events of 3300 4-D
+// points 167 / 246, 64 events 269 / 318, 100 2-D events of 3300 points 293 / 333, 300 events 798 / 756.
+constexpr int kBuildPoints = 65536;        // of a single event
+constexpr int kBuildBatchPoints = 1 << 19;  // of a batch, each event at most kBuildEventPoints
+constexpr int kBuildEventPoints = 32768;
+constexpr int kBuildTileBits = 16;
+inline bool build_takes(const KParams& kp, int max_points, int tile_bits, int mbits) {
+  if (tile_bits > kBuildTileBits || tile_bits + mbits > 32) return false;
+  if (kp.n_events == 1) return kp.n <= kBuildPoints;
+  // a batch's chunks and blocks have slots per event (k_build): they must fit the buffers
+  return kp.n <= kBuildBatchPoints && max_points <= kBuildEventPoints && kp.n / 32 + kp.ntiles + 1 <= kp.n;
+}
+// CTAs per cluster: of 1024 threads for a single event, about a point per thread and more from 8192
+// points on; of 512 threads for a batch, as many as leave the clusters on the chip together (24 events:
+// 8 CTAs 167 us, 4 176; 100 events: 4 CTAs 293 us, 8 319, 2 317).
+inline int build_ranks(int n_events, int n) {
+  if (n_events == 1) return n <= 1024 ? 1 : (n <= 2048 ? 2 : (n <= 4096 ? 4 : 8));
+  return n_events <= 64 ? 8 : (n_events <= 128 ? 4 : (n_events <= 256 ? 2 : 1));
+}
+
+template <int N, int W>
+void launch_build_cluster(const KParams& kp, const InPtrs& in, EvGrid* eg, const BuildBufs& o, bool two, int mbits,
+                          int tile_passes, int passes, int ranks, cudaStream_t s) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(kp.n_events * ranks));
+  cfg.blockDim = dim3(32 * W);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_build<N, W>, kp, in, eg, o, two, mbits, tile_passes, passes, ranks);
+}
+
+// Stage 1 through k_build; returns the launches.
+template <int N>
+int launch_build(const KParams& kp, const InPtrs& in, Workspace& ws, bool two, int mbits, int tile_bits,
+                 cudaStream_t s) {
+  const int passes = (tile_bits + mbits + kRadixBits - 1) / kRadixBits;
+  const int tile_passes = std::max(1, (tile_bits + kRadixBits - 1) / kRadixBits);
+  const bool odd = passes & 1;
+  const int ranks = build_ranks(kp.n_events, kp.n);
+  ws.build_ranks = ranks;
+  BuildBufs o{};
+  o.k0 = ws.keys[0];
+  o.k1 = ws.keys[1];
+  o.k2 = ws.mkeys_alt;
+  o.va = ws.vals[0];
+  o.vb = ws.vals[1];
+  o.perm = ws.mq_alt;
+  o.vt = ws.nh_s;   // (nearest highers, label parents: not in use yet)
+  o.inv = ws.par;
+  o.rec_w = ws.rec_w;
+  o.off = ws.offsets;
+  o.chunk_off = ws.chunk_count;
+  o.tblk_off = two ? nullptr : ws.tblk_off;
+  o.chunk_tile = ws.chunk_tile;
+  o.chunk_total = ws.chunk_total;
+  o.tblk = two ? nullptr : ws.tblk;
+  o.rho_fix = two ? nullptr : ws.rho_fix;
+  o.seed_bits = ws.seed_bits;
+  o.ev_pt = ws.ev_pt;
+  o.ev_tile = ws.ev_tile;
+  o.ev_chunk = ws.ev_chunk;
+  o.st = ws.status;
+  ws.perm = two ? ws.mq_alt : (odd ? ws.vals[0] : ws.vals[1]);
+  ws.mq = two ? (odd ? ws.vals[1] : ws.vals[0]) : nullptr;
+  if (kp.n_events > 1) {
+    k_init<N><<<grid_for(std::max(kp.n_events, kp.n / 128), 256), 256, 0, s>>>(kp, events_of(ws), ws.ev_pt, ws.ev_tile,
+                                                                               ws.seed_bits, ws.chunk_total, ws.status);
+    launch_build_cluster<N, 16>(kp, in, ws.ev, o, two, mbits, tile_passes, passes, ranks, s);
+    return 2;
+  }
+  launch_build_cluster<N, 32>(kp, in, ws.ev, o, two, mbits, tile_passes, passes, ranks, s);
+  return 1;
 }
 
 #define CLUE_METRIC_SWITCH(mt, FN, ...)                                           \
@@ -2107,101 +2617,100 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
   ws.near_from_host = false;  // this run's counts land in the device status block
 
   stage_mark(ws, 0, s);
-  k_init<N><<<grid_for(std::max(kp.n_events, n / 128), 256), 256, 0, s>>>(kp, ev, ws.ev_pt, ws.ev_tile, ws.seed_bits,
-                                                                          ws.status);
-  int launches_pre = 0;
-  if (kp.n_events == 1)
-    k_bbox_single<N><<<std::max(1, std::min(grid_for(n, 1024), 148 * 4)), 256, 0, s>>>(in, n, ws.ev, ws.status);
-  else
-  {
-    // spans of 32..1024 points: about four spans per resident warp (64 per SM) when there
-    // are enough points, so the loads of many spans are in flight
-    const int span = std::max(32, std::min(1024, (n / (148 * 64 * 4)) & ~31));
-    const int blocks = std::max(1, std::min(grid_for(n, 256), ((n + span - 1) / span + 7) / 8));
-    if (ws.ev_chunk) {
-      k_event_chunks<<<grid_for(kp.n_events, 256), 256, 0, s>>>(kp.n_events, ws.ev_pt, ws.ev_chunk);
-      ++launches_pre;
-    }
-    k_bbox_events<N><<<blocks, 256, 0, s>>>(in, n, kp.n_events, ws.ev_pt, ws.ev_chunk, ws.ev, ws.status, span);
-  }
-  k_grid<N><<<grid_for(kp.n_events, 256), 256, 0, s>>>(kp.n_events, ws.ev);
-  int launches = 4 + launches_pre;  // init, (chunk table,) bbox, grid, bin
+  int launches = 0;
   // density order: the reference's candidate order for the flat kernel (bit-exact sums), spatial
   // order for the exponential and Gaussian kernels (whose device expf already differs from the
   // host's by an ulp) unless the caller asks for the reference order
   const bool spatial_density = (kp.flags & CLUE_FLAG_REFERENCE_ORDER) == 0 &&
                                (kp.kernel_type != CLUE_KERNEL_FLAT || (kp.flags & CLUE_FLAG_SPATIAL_DENSITY) != 0);
-  // (a workspace without the symmetric sweep's buffers, such as the fixed scratch of the
-  // no-allocation entry point, keeps the one-sided sweep)
   const bool symmetric =
       spatial_density && symmetric_density_ok(kp, a.metric, N) && ws.tblk && ws.tblk_off && ws.rho_fix &&
       ws.tune_symmetric != 0;
   const int bits = bits_for((uint32_t)(kp.ntiles - 1));
   const int mbits = MortonSortBits<N>::kBits;
-  // The symmetric sweep needs no tile order by point index: one sort by (tile, Morton) composite
-  // keys gives its record order, and positions inside a tile are only compared through the
-  // points' indices.  The other sweeps take the tile order by index and a Morton order beside it.
-  const bool composite = symmetric && bits + mbits <= 32;
-  if (composite) {
-    k_bin_composite<N><<<grid_for(n, 1024), 256, 0, s>>>(kp, in, ev, mbits, ws.keys[0]);
-    const int cur = radix_sort_pairs(ws.keys, ws.vals, true, n, bits + mbits, ws.hist, ws.scan_scratch, s);
-    ws.perm = ws.vals[cur];
-    ws.sorted_keys = ws.keys[cur];
-    offsets_from_sorted(ws.sorted_keys, n, kp.ntiles, ws.offsets, s, mbits);
-    ws.mq = ws.vals[cur ^ 1];
-    ws.minv = ws.mq_alt;
-    k_gather<N><<<grid_for(n, 256), 256, 0, s>>>(in, n, ws.perm, ws.rec_w, ws.status, ws.mq, ws.minv);
-    ws.rec_m_cur = ws.rec_w;
-    launches += radix_sort_launches(bits + mbits) + 2;
-  } else {
-    k_bin<N><<<grid_for(n, 256), 256, 0, s>>>(kp, in, ev, ws.keys[0]);
-    const int cur = radix_sort_pairs(ws.keys, ws.vals, true, n, bits, ws.hist, ws.scan_scratch, s);
-    ws.perm = ws.vals[cur];
-    ws.sorted_keys = ws.keys[cur];
-    offsets_from_sorted(ws.sorted_keys, n, kp.ntiles, ws.offsets, s);
-    k_gather<N><<<grid_for(n, 256), 256, 0, s>>>(in, n, ws.perm, ws.rec_w, ws.status, nullptr, nullptr);
-    // fine Morton order inside every tile: a stable sort by Morton key, then a stable sort by
-    // tile; mq[p] = tile-sorted position of the p-th record in (tile, Morton) order
-    uint32_t* mkeys[2] = {ws.keys[cur ^ 1], ws.mkeys_alt};
-    int32_t* mvals[2] = {ws.vals[cur ^ 1], ws.mq_alt};
-    k_morton_keys<N><<<grid_for(n, 256), 256, 0, s>>>(kp, ev, ws.rec_w, ws.sorted_keys, mkeys[0]);
-    int mc = radix_sort_pairs(mkeys, mvals, true, n, MortonSortBits<N>::kBits, ws.hist, ws.scan_scratch, s);
-    if (mc != 0) {
-      std::swap(mkeys[0], mkeys[1]);
-      std::swap(mvals[0], mvals[1]);
-    }
-    k_tile_of<<<grid_for(n, 256), 256, 0, s>>>(ws.sorted_keys, mvals[0], n, mkeys[0]);
-    mc = radix_sort_pairs(mkeys, mvals, false, n, bits, ws.hist, ws.scan_scratch, s);
-    ws.mq = mvals[mc];
-    ws.minv = mvals[mc ^ 1];
-    k_invert<<<grid_for(n, 256), 256, 0, s>>>(ws.mq, n, ws.minv);
-    ws.rec_m_cur = ws.rec_m;
-    launches += radix_sort_launches(bits) + 2 + 1 + radix_sort_launches(MortonSortBits<N>::kBits) + 1 +
-                radix_sort_launches(bits) + 1;
-  }
-  k_tile_counts<<<grid_for(kp.ntiles, 256), 256, 0, s>>>(kp.ntiles, ws.offsets, ws.chunk_count,
-                                                         symmetric ? ws.tblk_off : nullptr);
-  exclusive_scan(ws.chunk_count, ws.chunk_count, (size_t)kp.ntiles, ws.scan_scratch, ws.chunk_total, s);
-  if (symmetric) exclusive_scan(ws.tblk_off, ws.tblk_off, (size_t)kp.ntiles, ws.scan_scratch, nullptr, s);
-  k_chunk_map<<<grid_for(kp.ntiles, 256), 256, 0, s>>>(kp.ntiles, ws.offsets, ws.chunk_count, ws.chunk_tile);
-  launches += 1 + scan_launches(kp.ntiles) * (symmetric ? 2 : 1) + 1;
-
-  const int nblk_threads = ((n + 31) >> 5) * 32;
-  const int nsb_threads = ((((n + 31) >> 5) + 31) >> 5) * 32;
+  const int nsb = (n + 1023) >> 10;
   const int max_slots = kChunkWarps * (n / kChunk + kp.ntiles + 1);
-  if (symmetric) {
-    if (!composite) {
-      k_gather_morton<N><<<grid_for(n, 256), 256, 0, s>>>(ws.rec_w, n, ws.mq, ws.rec_m);
+  const int pts_max = kp.n_events == 1 ? n : a.max_points;
+  const int ev_bits = bits_for((uint32_t)((kp.n_events == 1 ? kp.ntiles : a.max_tiles) - 1));
+  bool composite = false;
+  if (build_takes(kp, pts_max, ev_bits, mbits)) {
+    composite = symmetric;
+    launches += launch_build<N>(kp, in, ws, !symmetric, mbits, ev_bits, s);
+  } else {
+    ws.build_ranks = 0;
+    launches += 4;  // init, bbox, grid, bin
+    k_init<N><<<grid_for(std::max(kp.n_events, n / 128), 256), 256, 0, s>>>(kp, ev, ws.ev_pt, ws.ev_tile, ws.seed_bits,
+                                                                            nullptr, ws.status);
+    if (symmetric) cudaMemsetAsync(ws.rho_fix, 0, (size_t)n * sizeof(int64_t), s);
+    if (kp.n_events == 1) {
+      k_bbox_single<N><<<std::max(1, std::min(grid_for(n, 1024), 148 * 4)), 256, 0, s>>>(in, n, ws.ev, ws.status);
+    } else {
+      // spans of 32..1024 points: about four spans per resident warp (64 per SM) when there
+      // are enough points, so the loads of many spans are in flight
+      const int span = std::max(32, std::min(1024, (n / (148 * 64 * 4)) & ~31));
+      const int blocks = std::max(1, std::min(grid_for(n, 256), ((n + span - 1) / span + 7) / 8));
+      if (ws.ev_chunk) {
+        k_event_chunks<<<grid_for(kp.n_events, 256), 256, 0, s>>>(kp.n_events, ws.ev_pt, ws.ev_chunk);
+        ++launches;
+      }
+      k_bbox_events<N><<<blocks, 256, 0, s>>>(in, n, kp.n_events, ws.ev_pt, ws.ev_chunk, ws.ev, ws.status, span);
+    }
+    k_grid<N><<<grid_for(kp.n_events, 256), 256, 0, s>>>(kp.n_events, ws.ev);
+    // The symmetric sweep needs no tile order by point index: one sort by (tile, Morton) composite
+    // keys gives its record order, and positions inside a tile are only compared through the
+    // points' indices.  The other sweeps take the tile order by index and a Morton order beside it.
+    composite = symmetric && bits + mbits <= 32;
+    if (composite) {
+      k_bin_composite<N><<<grid_for(n, 1024), 256, 0, s>>>(kp, in, ev, mbits, ws.keys[0]);
+      const int cur = radix_sort_pairs(ws.keys, ws.vals, true, n, bits + mbits, ws.hist, ws.scan_scratch, s);
+      ws.perm = ws.vals[cur];
+      offsets_from_sorted(ws.keys[cur], n, kp.ntiles, ws.offsets, s, mbits);
+      ws.mq = nullptr;
+      k_gather<N><<<grid_for(n, 256), 256, 0, s>>>(in, n, ws.perm, ws.rec_w, ws.status);
+      launches += radix_sort_launches(bits + mbits) + 2;
+    } else {
+      k_bin<N><<<grid_for(n, 256), 256, 0, s>>>(kp, in, ev, ws.keys[0]);
+      const int cur = radix_sort_pairs(ws.keys, ws.vals, true, n, bits, ws.hist, ws.scan_scratch, s);
+      ws.perm = ws.vals[cur];
+      const uint32_t* sorted_keys = ws.keys[cur];
+      offsets_from_sorted(sorted_keys, n, kp.ntiles, ws.offsets, s);
+      k_gather<N><<<grid_for(n, 256), 256, 0, s>>>(in, n, ws.perm, ws.rec_w, ws.status);
+      // fine Morton order inside every tile: a stable sort by Morton key, then a stable sort by
+      // tile; mq[p] = tile-sorted position of the p-th record in (tile, Morton) order
+      uint32_t* mkeys[2] = {ws.keys[cur ^ 1], ws.mkeys_alt};
+      int32_t* mvals[2] = {ws.vals[cur ^ 1], ws.mq_alt};
+      k_morton_keys<N><<<grid_for(n, 256), 256, 0, s>>>(kp, ev, ws.rec_w, sorted_keys, mkeys[0]);
+      int mc = radix_sort_pairs(mkeys, mvals, true, n, MortonSortBits<N>::kBits, ws.hist, ws.scan_scratch, s);
+      if (mc != 0) {
+        std::swap(mkeys[0], mkeys[1]);
+        std::swap(mvals[0], mvals[1]);
+      }
+      k_tile_of<<<grid_for(n, 256), 256, 0, s>>>(sorted_keys, mvals[0], n, mkeys[0]);
+      mc = radix_sort_pairs(mkeys, mvals, false, n, bits, ws.hist, ws.scan_scratch, s);
+      ws.mq = mvals[mc];
+      launches += 2 * radix_sort_launches(bits) + 2 + 1 + radix_sort_launches(MortonSortBits<N>::kBits) + 1;
+    }
+    k_tile_counts<<<grid_for(kp.ntiles, 256), 256, 0, s>>>(kp.ntiles, ws.offsets, ws.chunk_count,
+                                                           symmetric ? ws.tblk_off : nullptr);
+    exclusive_scan(ws.chunk_count, ws.chunk_count, (size_t)kp.ntiles, ws.scan_scratch, ws.chunk_total, s);
+    if (symmetric) exclusive_scan(ws.tblk_off, ws.tblk_off, (size_t)kp.ntiles, ws.scan_scratch, nullptr, s);
+    k_chunk_map<<<grid_for(kp.ntiles, 256), 256, 0, s>>>(kp.ntiles, ws.offsets, ws.chunk_count, ws.chunk_tile);
+    launches += 1 + scan_launches(kp.ntiles) * (symmetric ? 2 : 1) + 1;
+    if (symmetric) {
+      if (!composite) {
+        k_gather_morton<N><<<grid_for(n, 256), 256, 0, s>>>(ws.rec_w, n, ws.mq, ws.rec_m);
+        ++launches;
+      }
+      k_tblock_bbox<N><<<grid_for(max_slots, 256), 256, 0, s>>>(max_slots, ws.chunk_total, ws.offsets, ws.chunk_tile,
+                                                                 ws.chunk_count, ws.tblk_off,
+                                                                 composite ? ws.rec_w : ws.rec_m, ws.tblk);
       ++launches;
     }
-    k_tblock_bbox<N><<<grid_for(max_slots, 256), 256, 0, s>>>(max_slots, ws.chunk_total, ws.offsets, ws.chunk_tile,
-                                                               ws.chunk_count, ws.tblk_off, ws.rec_m_cur, ws.tblk);
+  }
+  ws.rec_m_cur = composite ? ws.rec_w : ws.rec_m;
+  if (spatial_density && !symmetric) {
+    k_boxes<N, true><<<nsb, 1024, 0, s>>>(kp, ev, ws.mq, ws.rec_w, ws.rec_m, nullptr, 0.0f, ws.blk, ws.sblk);
     ++launches;
-  } else if (spatial_density) {
-    k_gather_morton<N><<<grid_for(n, 256), 256, 0, s>>>(ws.rec_w, n, ws.mq, ws.rec_m);
-    k_block_bbox<N><<<grid_for(nblk_threads, 256), 256, 0, s>>>(ws.rec_m, n, ws.blk);
-    k_superblock_bbox<N><<<grid_for(nsb_threads, 256), 256, 0, s>>>(ws.blk, n, ws.sblk);
-    launches += 3;
   }
 
   stage_mark(ws, 1, s);
@@ -2215,21 +2724,15 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
   launches += symmetric && !composite ? 2 : 1;  // (a composite run combines with the block boxes)
   stage_mark(ws, 2, s);
   // Morton-ordered copy of the records with their densities (the tile-ordered records themselves
-  // after a composite sort) and its block / super-block boxes with the largest rho, for the
-  // nearest-higher search
+  // after a composite sort, where the density's fixed-point sums are added in here) and its block
+  // and super-block boxes with the largest rho, for the nearest-higher search
   if (composite) {
-    // the tile-ordered records are the Morton-ordered ones; the density's fixed-point sums are
-    // added in while the block boxes are built
+    k_boxes<N, false><<<nsb, 1024, 0, s>>>(kp, ev, nullptr, ws.rec_r, nullptr, ws.rho_fix, ws.sym_kmax, ws.blk, ws.sblk);
     ws.rec_m_cur = ws.rec_r;
-    k_combine_block_bbox<N><<<grid_for(nblk_threads, 256), 256, 0, s>>>(kp, ev, n, ws.rho_fix, ws.rec_r,
-                                                                         ws.sym_kmax, ws.blk);
   } else {
-    k_gather_morton<N><<<grid_for(n, 256), 256, 0, s>>>(ws.rec_r, n, ws.mq, ws.rec_m);
+    k_boxes<N, true><<<nsb, 1024, 0, s>>>(kp, ev, ws.mq, ws.rec_r, ws.rec_m, nullptr, 0.0f, ws.blk, ws.sblk);
     ws.rec_m_cur = ws.rec_m;
-    ++launches;
-    k_block_bbox<N><<<grid_for(nblk_threads, 256), 256, 0, s>>>(ws.rec_m_cur, n, ws.blk);
   }
-  k_superblock_bbox<N><<<grid_for(nsb_threads, 256), 256, 0, s>>>(ws.blk, n, ws.sblk);
   CLUE_METRIC_SWITCH(a.metric, launch_nh, kp, ws, a.out, s);
   if (kp.flags & CLUE_FLAG_NEAR_TIES) {
     CLUE_METRIC_SWITCH(a.metric, launch_near_ties, kp, ws, s);
@@ -2237,11 +2740,17 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
   }
   stage_mark(ws, 3, s);
   const size_t words = ((size_t)n + 31) / 32;
-  exclusive_scan_bits(ws.seed_bits, ws.seed_rank, words, ws.scan_scratch, ws.seed_total, s);
-  k_seed_labels<<<std::min(grid_for(std::max(kp.n_events, n / 8), 256), 148 * 8), 256, 0, s>>>(
-      kp, ev, ws.seed_bits, ws.seed_rank, ws.seed_total, ws.seed_list, ws.perm, ws.par, a.ev_n_seeds, a.ev_n_clusters,
-      ws.status);
-  launches += scan_launches(words) + 1;
+  if (words <= kScanOneBlock) {
+    k_seed_labels_one<<<1, 1024, 0, s>>>(kp, ev, ws.seed_bits, ws.seed_rank, ws.seed_total, (int)words, ws.seed_list,
+                                         ws.perm, ws.par, a.ev_n_seeds, a.ev_n_clusters, ws.status);
+    launches += 1;
+  } else {
+    exclusive_scan_bits(ws.seed_bits, ws.seed_rank, words, ws.scan_scratch, ws.seed_total, s);
+    k_seed_labels<<<std::min(grid_for(std::max(kp.n_events, n / 8), 256), 148 * 8), 256, 0, s>>>(
+        kp, ev, ws.seed_bits, ws.seed_rank, ws.seed_total, ws.seed_list, ws.perm, ws.par, a.ev_n_seeds,
+        a.ev_n_clusters, ws.status);
+    launches += scan_launches(words) + 1;
+  }
   if (ws.tune_labels_bfs) {
     // follower CSR in buffers that are dead by now: the sort keys and the weight records
     uint32_t* counts = ws.keys[0];
@@ -2267,8 +2776,8 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
     k_labels_again<<<grid_for(n, 256), 256, 0, s>>>(ws.par, ws.perm, a.out.cluster_index, n, ws.status);
   }
   stage_mark(ws, 4, s);
-  // Morton boxes (blocks, super-blocks), nearest higher, labels
-  ws.launches += launches + 3 + (a.blocking ? 1 : 1 + kJumpLaunches);
+  // Morton boxes, nearest higher, labels
+  ws.launches += launches + 2 + (a.blocking ? 1 : 1 + kJumpLaunches);
   CLUE_CUDA_TRY(cudaGetLastError());
   return CLUE_OK;
 }

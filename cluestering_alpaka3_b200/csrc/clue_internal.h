@@ -87,6 +87,7 @@ struct RunArgs {
   // The caller reads the status back and continues label chains the first round left unresolved
   // (finish_labels); otherwise all rounds are enqueued.
   bool blocking;
+  int32_t max_points, max_tiles;  // of one event of a batched call
 };
 
 template <int N>
@@ -127,11 +128,10 @@ struct Workspace {
   float4* blk = nullptr;          // bounding boxes of 32-record blocks of the sorted records
   int32_t* mq_alt = nullptr;      // second value buffer of the Morton sort
   uint32_t* mkeys_alt = nullptr;  // second key buffer of the Morton sort
-  int32_t* minv = nullptr;        // tile-sorted position -> Morton position (alias after the sort)
   float4* rec_m = nullptr;        // records in Morton order inside every tile
   const float4* rec_m_cur = nullptr;  // Morton-ordered records the sweeps of this run read
   float4* sblk = nullptr;         // bounding boxes of 1024-record super-blocks
-  int32_t* mq = nullptr;          // Morton position -> tile-sorted position (alias after the sort)
+  int32_t* mq = nullptr;          // Morton position -> tile-sorted position (alias; null: the identity)
   uint32_t* chunk_count = nullptr;  // [ntiles] chunks per tile, then exclusive-scanned
   int32_t* chunk_tile = nullptr;  // [max chunks] tile of every chunk
   uint32_t* chunk_total = nullptr;
@@ -175,6 +175,7 @@ struct Workspace {
   int32_t* perm = nullptr;  // alias of the sorted values buffer after the tile sort
   uint32_t* sorted_keys = nullptr;
 
+  int build_ranks = 0;  // CTAs per cluster of the last run's k_build launch, 0 without one
   KParams last_kp{};  // parameters of the last enqueued run (for clue_context_read_info)
   // near-threshold counts summed on the host over the chunks of an overlapped host-memory
   // batch (near_from_host); every other run leaves them in the device status block

@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -183,8 +184,15 @@ size_t workspace_bytes_for(int ndim, size_t n, size_t ntiles, size_t n_events) {
   return arena_total(arena_items(nw, &evtab, n, ntiles, n_events, (size_t)((ndim + 1 + 3) / 4)));
 }
 
+// Before a buffer is replaced.  (Only when something may be in flight: waiting for the device breaks
+// the captures of other threads' streams.)
+static void wait_idle(Workspace& ws) {
+  if (ws.busy) cudaDeviceSynchronize();
+}
+
 clue_status workspace_reserve(Workspace& ws, int ndim, size_t n, size_t ntiles, size_t n_events) {
   const size_t words = (size_t)((ndim + 1 + 3) / 4);
+  ws.reused = false;
   if (n <= ws.cap_n && ntiles <= ws.cap_tiles && words <= ws.cap_words && n_events <= ws.cap_events && ws.arena)
     return CLUE_OK;
   n = std::max(n, ws.cap_n);
@@ -199,12 +207,12 @@ clue_status workspace_reserve(Workspace& ws, int ndim, size_t n, size_t ntiles, 
   cudaGetDevice(&prev);
   cudaSetDevice(ws.device);
   if (ws.arena) {
-    cudaDeviceSynchronize();
+    wait_idle(ws);
     cudaFree(ws.arena);
     ws.arena = nullptr;
   }
   void* arena = nullptr;
-  cudaError_t e = cudaMalloc(&arena, total);
+  cudaError_t e = device_malloc(&arena, total);
   if (e != cudaSuccess) {
     cudaGetLastError();
     cudaSetDevice(prev);
@@ -256,12 +264,12 @@ clue_status workspace_reserve(Workspace& ws, int ndim, size_t n, size_t ntiles, 
 static clue_status reserve_stage(Workspace& ws, size_t bytes) {
   if (bytes <= ws.dstage_bytes) return CLUE_OK;
   if (ws.dstage) {
-    cudaDeviceSynchronize();
+    wait_idle(ws);
     cudaFree(ws.dstage);
     ws.dstage = nullptr;
     ws.dstage_bytes = 0;
   }
-  CLUE_CUDA_TRY(cudaMalloc(&ws.dstage, bytes));
+  CLUE_CUDA_TRY(device_malloc(&ws.dstage, bytes));
   ws.dstage_bytes = bytes;
   return CLUE_OK;
 }
@@ -369,12 +377,12 @@ clue_status post_reserve(Workspace& ws, size_t device_bytes, size_t host_bytes) 
   cudaError_t e = cudaSuccess;
   if (device_bytes > ws.post_bytes) {
     if (ws.post) {
-      cudaDeviceSynchronize();
+      wait_idle(ws);
       cudaFree(ws.post);
     }
     ws.post = nullptr;
     ws.post_bytes = 0;
-    e = cudaMalloc(&ws.post, device_bytes);
+    e = device_malloc(&ws.post, device_bytes);
     if (e == cudaSuccess) ws.post_bytes = device_bytes;
   }
   if (e == cudaSuccess && host_bytes > ws.post_host_bytes) {
@@ -398,6 +406,7 @@ clue_status clusters_csr(Workspace& ws, int n, const int32_t* cluster_index, int
   // keys = label + 1 in [0, n]; offsets_from_sorted needs n + 2 entries
   clue_status st = workspace_reserve(ws, 1, (size_t)n, (size_t)n + 2, 1);
   if (st != CLUE_OK) return st;
+  ws.busy = true;  // (cleared by the callers, which wait)
   CLUE_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(CsrInfo), s));
   const int threads = 256;
   const int blocks = std::min((n + threads - 1) / threads, 148 * 16);
@@ -445,6 +454,114 @@ struct clue_context_s {
 
 namespace clue_b200 {
 Workspace& context_workspace(clue_context ctx) { return ctx->ws; }
+
+static void context_free(clue_context ctx) {
+  int prev = 0;
+  cudaGetDevice(&prev);
+  cudaSetDevice(ctx->ws.device);
+  workspace_release(ctx->ws);
+  if (ctx->alt) {
+    workspace_release(*ctx->alt);
+    delete ctx->alt;
+  }
+  if (ctx->alt_stream) cudaStreamDestroy(ctx->alt_stream);
+  if (ctx->chunk_stream) cudaStreamDestroy(ctx->chunk_stream);
+  for (auto& slot : ctx->chunk_exec) slot.destroy();
+  ctx->plain_exec.destroy();
+  for (auto& e : ctx->plain_ev)
+    if (e) cudaEventDestroy(e);
+  cudaSetDevice(prev);
+  delete ctx;
+}
+
+// Destroyed contexts kept for the next clue_context_create on their device: a program that makes a
+// Clusterer (or a Python clusterer) per table paid for the workspace, pinned buffers, stream and
+// executable graph of a new context on every call (4.0 ms of a 2000-point Python call, 0.28 ms with a
+// kept one).  At most kIdleContexts per device, each holding at most kIdleBytes of device memory; all
+// are freed when an allocation of the library fails (device_malloc).
+constexpr size_t kIdleContexts = 2;
+constexpr size_t kIdleBytes = 64u << 20;
+struct IdleContexts {
+  std::mutex mutex;
+  std::vector<clue_context_s*> list;  // oldest first
+};
+static IdleContexts& idle_contexts() {
+  static IdleContexts* p = new IdleContexts;  // (not destroyed: the driver may be gone at exit)
+  return *p;
+}
+
+// Keeps ctx if it is small; false: the caller frees it.
+static bool idle_put(clue_context ctx) {
+  Workspace& ws = ctx->ws;
+  // (nothing of this context may be in flight when its buffers get their next owner)
+  if (!ws.arena || ws.busy || ctx->alt || ws.arena_bytes + ws.dstage_bytes + ws.post_bytes > kIdleBytes ||
+      ws.pipe_pinned)
+    return false;
+  for (auto& t : ws.tev)
+    if (t) cudaEventDestroy(t);
+  // as a new context, with the buffers, streams, events and executable graphs
+  Workspace fresh;
+  for (auto& t : ws.tev) t = nullptr;
+  ws.tune_symmetric = fresh.tune_symmetric;
+  ws.tune_nh_split = fresh.tune_nh_split;
+  ws.tune_overlap_chunk_points = fresh.tune_overlap_chunk_points;
+  ws.tune_density_gate = fresh.tune_density_gate;
+  ws.tune_density_exp2 = fresh.tune_density_exp2;
+  ws.tune_labels_bfs = fresh.tune_labels_bfs;
+  ws.last_kp = KParams{};
+  ws.near_from_host = false;
+  ws.timing = false;
+  ws.launches = 0;
+  ws.reused = true;
+  clue_context drop = nullptr;
+  {
+    IdleContexts& idle = idle_contexts();
+    std::lock_guard<std::mutex> lock(idle.mutex);
+    size_t same = 0;
+    for (auto* c : idle.list) same += c->ws.device == ws.device;
+    if (same >= kIdleContexts)
+      for (size_t k = 0; k < idle.list.size() && !drop; ++k)
+        if (idle.list[k]->ws.device == ws.device) {
+          drop = idle.list[k];
+          idle.list.erase(idle.list.begin() + (ptrdiff_t)k);
+        }
+    idle.list.push_back(ctx);
+  }
+  if (drop) context_free(drop);
+  return true;
+}
+
+// The most recent idle context of the device, or null.
+static clue_context idle_take(int device) {
+  IdleContexts& idle = idle_contexts();
+  std::lock_guard<std::mutex> lock(idle.mutex);
+  for (size_t k = idle.list.size(); k-- > 0;) {
+    clue_context c = idle.list[k];
+    if (c->ws.device != device) continue;
+    idle.list.erase(idle.list.begin() + (ptrdiff_t)k);
+    // a device reset by the program took its buffers along: forget it
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, c->ws.arena) == cudaSuccess && at.type == cudaMemoryTypeDevice) return c;
+    cudaGetLastError();
+    delete c;
+  }
+  return nullptr;
+}
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  std::vector<clue_context_s*> all;
+  {
+    IdleContexts& idle = idle_contexts();
+    std::lock_guard<std::mutex> lock(idle.mutex);
+    all.swap(idle.list);
+  }
+  if (all.empty()) return e;
+  cudaGetLastError();
+  for (auto* c : all) context_free(c);
+  return cudaMalloc(p, bytes);
+}
 }  // namespace clue_b200
 
 // Captures the pipeline enqueued by run_pipeline_dispatch on `g` into a graph and launches it
@@ -639,7 +756,7 @@ clue_status clue_device_alloc(int32_t device, size_t bytes, void** ptr) {
   int prev = 0;
   CLUE_CUDA_TRY(cudaGetDevice(&prev));
   CLUE_CUDA_TRY(cudaSetDevice(device));
-  cudaError_t e = cudaMalloc(ptr, bytes ? bytes : 1);
+  cudaError_t e = device_malloc(ptr, bytes ? bytes : 1);
   cudaSetDevice(prev);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -709,7 +826,8 @@ clue_status clue_context_create(int32_t device, clue_context* ctx) {
     set_error("no CUDA device with id " + std::to_string(device));
     return CLUE_ERR_CUDA;
   }
-  auto* c = new (std::nothrow) clue_context_s;
+  auto* c = idle_take(device);
+  if (!c) c = new (std::nothrow) clue_context_s;
   if (!c) return CLUE_ERR_OUT_OF_MEMORY;
   c->ws.device = device;
   *ctx = c;
@@ -718,22 +836,7 @@ clue_status clue_context_create(int32_t device, clue_context* ctx) {
 
 clue_status clue_context_destroy(clue_context ctx) {
   if (!ctx) return CLUE_OK;
-  int prev = 0;
-  cudaGetDevice(&prev);
-  cudaSetDevice(ctx->ws.device);
-  workspace_release(ctx->ws);
-  if (ctx->alt) {
-    workspace_release(*ctx->alt);
-    delete ctx->alt;
-  }
-  if (ctx->alt_stream) cudaStreamDestroy(ctx->alt_stream);
-  if (ctx->chunk_stream) cudaStreamDestroy(ctx->chunk_stream);
-  for (auto& slot : ctx->chunk_exec) slot.destroy();
-  ctx->plain_exec.destroy();
-  for (auto& e : ctx->plain_ev)
-    if (e) cudaEventDestroy(e);
-  cudaSetDevice(prev);
-  delete ctx;
+  if (!idle_put(ctx)) context_free(ctx);
   return CLUE_OK;
 }
 
@@ -879,6 +982,7 @@ clue_status clue_make_clusters(clue_context ctx, const clue_params* params, cons
   cudaStream_t s = (cudaStream_t)stream;
   const size_t nn = (size_t)n;
   clue_outputs dev_out = *out;
+  const bool was_busy = ws.busy;
   if (memory == CLUE_MEM_HOST) {
     // device staging: coords, weight, then the five outputs
     st = reserve_stage(ws, (nn * (size_t)(ndim + 1) + 5 * nn) * 4);
@@ -901,6 +1005,7 @@ clue_status clue_make_clusters(clue_context ctx, const clue_params* params, cons
     a.out = dev_out;
   }
   a.blocking = true;
+  ws.busy = true;
   st = run_pipeline_graph(ctx, a, s);
   bool unresolved = false;
   if (st == CLUE_OK) st = read_info(ws, a.kp, s, info, unresolved);
@@ -923,6 +1028,7 @@ clue_status clue_make_clusters(clue_context ctx, const clue_params* params, cons
       st = CLUE_ERR_CUDA;
     }
   }
+  if (st == CLUE_OK) ws.busy = was_busy;  // all of it was waited for
   cudaSetDevice(prev);
   return st;
 }
@@ -933,11 +1039,12 @@ clue_status clue_make_clusters_async(clue_context ctx, const clue_params* params
   RunArgs a;
   clue_status st = prepare(ctx, params, kernel, metric, ndim, n, coords, weight, out, a);
   if (st != CLUE_OK) return st;
+  ctx->ws.busy = true;
   return run_pipeline_dispatch(ctx->ws, a, (cudaStream_t)stream);
 }
 
 clue_status clue_context_read_info(clue_context ctx, void* stream, clue_run_info* info) {
-  if (!ctx || !ctx->ws.arena) {
+  if (!ctx || !ctx->ws.arena || ctx->ws.reused) {
     set_error("context has no completed run");
     return CLUE_ERR_INVALID_ARG;
   }
@@ -951,7 +1058,7 @@ clue_status clue_context_read_info(clue_context ctx, void* stream, clue_run_info
 }
 
 clue_status clue_context_read_near_counts(clue_context ctx, void* stream, clue_near_counts* counts) {
-  if (!ctx || !ctx->ws.arena || !counts) {
+  if (!ctx || !ctx->ws.arena || ctx->ws.reused || !counts) {
     set_error("context has no completed run");
     return CLUE_ERR_INVALID_ARG;
   }
@@ -1030,6 +1137,7 @@ clue_status clue_get_clusters(clue_context ctx, int32_t n, const int32_t* cluste
   cudaSetDevice(ws.device);
   CsrInfo* info = static_cast<CsrInfo*>(ws.post);
   const CsrInfo* h = static_cast<const CsrInfo*>(ws.post_host);
+  const bool was_busy = ws.busy;
   st = clusters_csr(ws, n, cluster_index, offsets, points, info, s);
   cudaError_t e = cudaSuccess;
   if (st == CLUE_OK) e = cudaMemcpyAsync(ws.post_host, info, sizeof(CsrInfo), cudaMemcpyDeviceToHost, s);
@@ -1037,6 +1145,7 @@ clue_status clue_get_clusters(clue_context ctx, int32_t n, const int32_t* cluste
   cudaSetDevice(prev);
   if (st != CLUE_OK) return st;
   CLUE_CUDA_TRY(e);
+  ws.busy = was_busy;
   if (h->bad) {
     set_error("clue_get_clusters: cluster index outside [-1, n)");
     return CLUE_ERR_OUT_OF_RANGE;
@@ -1192,6 +1301,7 @@ static clue_status batch_plain(clue_context ctx, const clue_params* params, cons
   cudaStream_t s = (cudaStream_t)stream;
   const size_t nn = (size_t)a.n;
   clue_outputs dev_out = *out;
+  const bool was_busy = ws.busy;
   int32_t* dev_ncl = ev_n_clusters;
   if (memory == CLUE_MEM_HOST) {
     st = reserve_stage(ws, (nn * (size_t)(ndim + 1) + 5 * nn + (size_t)n_events) * 4);
@@ -1219,6 +1329,7 @@ static clue_status batch_plain(clue_context ctx, const clue_params* params, cons
   a.out = dev_out;
   a.ev_n_clusters = dev_ncl;
   a.blocking = true;
+  ws.busy = true;
   st = upload_events(ws, n_events, s);
   if (st == CLUE_OK) st = run_pipeline_graph(ctx, a, s);
   bool unresolved = false;
@@ -1244,6 +1355,7 @@ static clue_status batch_plain(clue_context ctx, const clue_params* params, cons
     }
   }
   if (st == CLUE_OK && info) info->n_per_dim = 0;
+  if (st == CLUE_OK) ws.busy = was_busy;  // all of it was waited for
   cudaSetDevice(prev);
   return st;
 }
@@ -1332,6 +1444,7 @@ static clue_status batch_host_overlapped(clue_context ctx, const clue_params* pa
   }
   clue_status st = workspace_reserve(ws, ndim, max_n, max_tiles, max_ev);
   if (st != CLUE_OK) return st;
+  ws.busy = true;
   int prev = 0;
   CLUE_CUDA_TRY(cudaGetDevice(&prev));
   CLUE_CUDA_TRY(cudaSetDevice(ws.device));
@@ -1752,7 +1865,7 @@ clue_status clue_autotune_batch(clue_context ctx, const clue_params* params, con
   cudaStream_t s = (cudaStream_t)stream;
   int32_t* labels = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
-  cudaError_t ce = cudaMalloc(&labels, (size_t)n * sizeof(int32_t));
+  cudaError_t ce = device_malloc((void**)&labels, (size_t)n * sizeof(int32_t));
   if (ce == cudaSuccess) ce = cudaEventCreate(&e0);
   if (ce == cudaSuccess) ce = cudaEventCreate(&e1);
   clue_status st = ce == cudaSuccess ? CLUE_OK : CLUE_ERR_CUDA;
@@ -1856,6 +1969,7 @@ clue_status clue_batch_make_clusters_async(clue_context ctx, const clue_params* 
   a.weight = weight;
   a.ev_n_clusters = ev_n_clusters;
   cudaStream_t s = (cudaStream_t)stream;
+  ctx->ws.busy = true;
   st = upload_events(ctx->ws, n_events, s);
   if (st != CLUE_OK) return st;
   return run_pipeline_dispatch(ctx->ws, a, s);
@@ -1882,6 +1996,7 @@ clue_status clue_graph_capture_batch(clue_context ctx, const clue_params* params
   a.ev_n_clusters = ev_n_clusters;
   cudaStream_t s = (cudaStream_t)stream;
   Workspace& ws = ctx->ws;
+  ws.busy = true;  // (its launches are not seen here)
   const bool timing = ws.timing;
   ws.timing = false;
   auto* g = new (std::nothrow) clue_graph_s;
@@ -1952,6 +2067,7 @@ extern "C" clue_status clue_events_loop(clue_context ctx, const clue_params* par
   }
   Workspace& ws = ctx->ws;
   if ((st = workspace_reserve(ws, ndim, (size_t)nmax, (size_t)tmax, 1)) != CLUE_OK) return st;
+  ws.busy = true;
   cudaStream_t s = (cudaStream_t)stream;
   std::vector<cudaEvent_t> evs;
   if (event_ms) {

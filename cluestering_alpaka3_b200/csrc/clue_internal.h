@@ -96,9 +96,15 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s);
 // Dispatch on ndim (clue_dim.cu).
 clue_status run_pipeline_dispatch(Workspace& ws, const RunArgs& a, cudaStream_t s);
 
+// cudaMalloc on the current device; when it fails, the idle contexts' memory is given back and it is
+// tried once more.
+cudaError_t device_malloc(void** p, size_t bytes);
+
 // ---- workspace ----------------------------------------------------------------
 struct Workspace {
   int device = 0;
+  bool reused = false;  // buffers of an idle context, no run or reservation of this one yet
+  bool busy = false;    // work may be in flight: set by every call, cleared by one that waited for its end
   // current capacities
   size_t cap_n = 0, cap_tiles = 0, cap_words = 0;
   size_t cap_events = 0;

@@ -248,6 +248,7 @@ clue_status clue_cluster_centroids(clue_context ctx, int32_t ndim, int32_t n, co
   int prev = 0;
   cudaGetDevice(&prev);
   cudaSetDevice(ws.device);
+  const bool was_busy = ws.busy;
   st = clusters_csr(ws, n, cluster_index, offsets, points, info, s);
   cudaError_t e = cudaSuccess;
   if (st == CLUE_OK) {
@@ -266,6 +267,7 @@ clue_status clue_cluster_centroids(clue_context ctx, int32_t ndim, int32_t n, co
     set_error(std::string("clue_cluster_centroids: ") + cudaGetErrorString(e));
     return CLUE_ERR_CUDA;
   }
+  ws.busy = was_busy;  // all of it was waited for
   const CsrInfo* h = static_cast<const CsrInfo*>(ws.post_host);
   if (h->bad) {
     set_error("clue_get_clusters: cluster index outside [-1, n)");
@@ -307,6 +309,7 @@ clue_status clue_silhouette(clue_context ctx, int32_t ndim, int32_t n, const flo
   int prev = 0;
   cudaGetDevice(&prev);
   cudaSetDevice(ws.device);
+  const bool was_busy = ws.busy;
   st = clusters_csr(ws, n, cluster_index, offsets, points, info, s);
   cudaError_t e = cudaSuccess;
   if (st == CLUE_OK) {
@@ -333,6 +336,7 @@ clue_status clue_silhouette(clue_context ctx, int32_t ndim, int32_t n, const flo
     set_error(std::string("clue_silhouette: ") + cudaGetErrorString(e));
     return CLUE_ERR_CUDA;
   }
+  ws.busy = was_busy;  // all of it was waited for
   if (static_cast<const CsrInfo*>(ws.post_host)->bad) {
     set_error("clue_get_clusters: cluster index outside [-1, n)");
     return CLUE_ERR_OUT_OF_RANGE;

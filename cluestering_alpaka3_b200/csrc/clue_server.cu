@@ -122,8 +122,8 @@ clue_status alloc_slot(clue_server_s* S, Slot& s) {
   const size_t out_words = 5 * (size_t)S->cap_points + S->cap_events;
   CLUE_CUDA_TRY(cudaMallocHost((void**)&s.h_in, in_words * 4));
   CLUE_CUDA_TRY(cudaMallocHost((void**)&s.h_out, out_words * 4));
-  CLUE_CUDA_TRY(cudaMalloc((void**)&s.d_in, in_words * 4));
-  CLUE_CUDA_TRY(cudaMalloc((void**)&s.d_out, out_words * 4));
+  CLUE_CUDA_TRY(device_malloc((void**)&s.d_in, in_words * 4));
+  CLUE_CUDA_TRY(device_malloc((void**)&s.d_out, out_words * 4));
   s.off.reserve(S->cap_events + 1);
   s.reqs.reserve(S->cap_events);
   return CLUE_OK;

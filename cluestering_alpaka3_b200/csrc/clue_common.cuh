@@ -51,6 +51,7 @@ struct KParams {
   int32_t lb_ok;  // metric parameters allow box lower bounds (no negative weights)
   int32_t flags;  // clue_params.flags
   float ginv;     // 1 / (2 std^2) of the Gaussian kernel (spatial-order density)
+  float one;      // 1, unknown to the compiler (partial_packed); set by run_pipeline
 };
 
 // Bounding box of 32 consecutive tile-sorted records: lo[N], hi[N], max payload.
@@ -453,20 +454,24 @@ __device__ __forceinline__ float2 partial_pair(const float* x, const float* a, c
 }
 // The same for two points whose coordinates are already paired (c[d] holds both of dimension d, x[d]
 // the one point's coordinate twice), as they come from 64-bit loads: no moves to pair registers.
+// Sums are paired too, as t * one + acc with a one that the compiler does not know (a paired add
+// behind a paired multiply would be contracted, see above): one rounding, the bits of t + acc.
 template <int N, int MT>
 __device__ __forceinline__ float2 partial_packed(const unsigned long long* x, const unsigned long long* c,
-                                                 const float* mpar) {
+                                                 const float* mpar, unsigned long long one) {
   if constexpr (MT == CLUE_METRIC_EUCLIDEAN) {
-    float2 acc;
+    unsigned long long acc;
 #pragma unroll
     for (int d = N - 1; d >= 0; --d) {
       unsigned long long df, sq;
       asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(df) : "l"(x[d]), "l"(c[d]));
       asm("mul.rn.f32x2 %0, %1, %1;" : "=l"(sq) : "l"(df));
-      const float2 t = upk2(sq);
-      acc = d == N - 1 ? t : make_float2(fadd(t.x, acc.x), fadd(t.y, acc.y));
+      if (d == N - 1)
+        acc = sq;
+      else
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(sq), "l"(one));
     }
-    return acc;
+    return upk2(acc);
   } else {
     float xx[N], a[N], b[N];
 #pragma unroll
@@ -494,6 +499,33 @@ __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// Unit-amplitude kernel values 2^(kexp d) (EXPO) or 2^(kexp d^2) of two metric values s, 0 where s > thr:
+// the same instructions as sqrt_approx and ex2_approx, predicated on s <= thr, so that the MUFU pipe
+// does not run for a step that no lane of the warp holds within reach.
+template <bool EXPO, bool ROOT>
+__device__ __forceinline__ float2 kernel_within(float2 s, float thr, float2 kexp) {
+  float2 v;
+  if constexpr (EXPO && ROOT) {
+    asm("{\n\t.reg .pred p, q;\n\t.reg .f32 a, b;\n\t.reg .b64 t;\n\t"
+        "setp.le.f32 p, %2, %4;\n\tsetp.le.f32 q, %3, %4;\n\t"
+        "mov.f32 a, %2;\n\tmov.f32 b, %3;\n\t"
+        "@p sqrt.approx.ftz.f32 a, a;\n\t@q sqrt.approx.ftz.f32 b, b;\n\t"
+        "mov.b64 t, {a, b};\n\tmul.rn.f32x2 t, t, %5;\n\tmov.b64 {a, b}, t;\n\t"
+        "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
+        "@p ex2.approx.ftz.f32 %0, a;\n\t@q ex2.approx.ftz.f32 %1, b;\n\t}"
+        : "=&f"(v.x), "=&f"(v.y)
+        : "f"(s.x), "f"(s.y), "f"(thr), "l"(pk2(kexp)));
+  } else {
+    const float2 e = mul2(kexp, EXPO != ROOT ? s : mul2(s, s));
+    asm("{\n\t.reg .pred p, q;\n\t"
+        "setp.le.f32 p, %2, %4;\n\tsetp.le.f32 q, %3, %4;\n\t"
+        "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
+        "@p ex2.approx.ftz.f32 %0, %5;\n\t@q ex2.approx.ftz.f32 %1, %6;\n\t}"
+        : "=&f"(v.x), "=&f"(v.y)
+        : "f"(s.x), "f"(s.y), "f"(thr), "f"(e.x), "f"(e.y));
+  }
+  return v;
 }
 // 2^e of two values on the FMA pipe instead of the MUFU (XU) pipe, for e <= 0: e is split as
 // n + f with n the nearest integer (adding and subtracting 1.5 * 2^23 rounds to an integer) and

@@ -1390,6 +1390,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4)) k_density(
   unsigned long long x2[N];
 #pragma unroll
   for (int d = 0; d < N; ++d) x2[d] = pk2(make_float2(x[d], x[d]));
+  const unsigned long long one = pk2(make_float2(kp.one, kp.one));
   float rho = 0.0f;
   box_tiles<N>(h.g, off, hb, wl, wh, -1, lane, [&](const int* v, int, int pb, int pe) {
     bool inbox = valid;
@@ -1413,8 +1414,8 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4)) k_density(
           unsigned long long ca[N], cb[N];
 #pragma unroll
           for (int d = 0; d < N; ++d) ca[d] = c2[d].x, cb[d] = c2[d].y;
-          s2[0] = partial_packed<N, MT>(x2, ca, kp.mpar);
-          s2[1] = partial_packed<N, MT>(x2, cb, kp.mpar);
+          s2[0] = partial_packed<N, MT>(x2, ca, kp.mpar, one);
+          s2[1] = partial_packed<N, MT>(x2, cb, kp.mpar, one);
         }
         const float4 tv = reinterpret_cast<const float4&>(s_buf[warp][N][q0 + q]);
         float s[4] = {s2[0].x, s2[0].y, s2[1].x, s2[1].y}, tt[4] = {tv.x, tv.y, tv.z, tv.w};
@@ -1527,6 +1528,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
   unsigned long long x2[N];
 #pragma unroll
   for (int d = 0; d < N; ++d) x2[d] = pk2(make_float2(x[d], x[d]));
+  const unsigned long long one = pk2(make_float2(kp.one, kp.one));
   const float slack = M::kRoot ? 1.0f + 1.0f / 524288.0f : 1.0f;  // s range of one rounded distance
   float s_best = INFINITY;  // metric value of the nearest higher so far
   // Candidates beyond bnd cannot be nearer than the best so far (nor within dm): its distance
@@ -1609,7 +1611,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
           unsigned long long cp[N];
 #pragma unroll
           for (int d = 0; d < N; ++d) cp[d] = e ? c2[d].y : c2[d].x;
-          const float2 s2 = partial_packed<N, MT>(x2, cp, kp.mpar);
+          const float2 s2 = partial_packed<N, MT>(x2, cp, kp.mpar, one);
 #pragma unroll
           for (int f = 0; f < 2; ++f) {
             const int j = 4 * q + e + f;
@@ -1847,6 +1849,30 @@ __device__ __forceinline__ int fix_exponent(const EvGrid* g, float kmax) {
   return max(-126, min(126, 61 - e));
 }
 
+// A candidate block in shared memory for the pair steps, in pairs of neighbours: component j (N: the
+// weight) of candidates 2 m and 2 m + 1 side by side, two components to a 16-byte word, 16 words (one
+// per pair) in a row, so that two steps read both candidates of a pair as operands of paired
+// arithmetic, without a move.  Two neighbouring lanes read the same words.
+// The sweep is bound by the MUFU pipe (two operations a pair for the exponential kernel, 73% busy) and
+// instruction issue (71%).  With every component by butterfly shuffle (eight shuffles for two steps,
+// the shared-memory pipe 75% busy as well, and moves to pair the operands) it took 7000 instructions
+// a warp, now 4700: 3.43 -> 3.22 ms on the 4096-event batch, 1.16 -> 1.01 ms on 4M 3-D points, 0.30 ->
+// 0.27 ms on 1M 2-D points (Gaussian).  A second copy for odd lanes, which spares the two selects a
+// step pair, costs more in shared-memory reads: 3.53 and 1.12 ms.
+template <int N>
+struct PairSmem {
+  static constexpr int kRows = (N + 2) / 2;
+  static constexpr int kFloats = kRows * 64;
+};
+// All components of a pair at shared-memory address `a` (row 0's word).
+template <int N>
+__device__ __forceinline__ void load_pairs(uint32_t a, unsigned long long* c) {
+#pragma unroll
+  for (int f = 0; f < (N + 1) / 2; ++f)
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(c[2 * f]), "=l"(c[2 * f + 1]) : "r"(a + 256u * f));
+  if constexpr ((N + 1) & 1) asm volatile("ld.shared.u64 %0, [%1];" : "=l"(c[N]) : "r"(a + 256u * (N / 2)));
+}
+
 // VAR selects measured alternatives of the pair step (clue_tuning.density_gate / density_exp2):
 // bit 0: a warp vote per pair of steps skips the kernel evaluation and the mirrored shuffles when
 // no lane of the warp has a candidate within dc (the same bits: the skipped terms are zeros);
@@ -1862,9 +1888,13 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
   using M = Metric<N, MT>;
   constexpr int BW = Blk<N>::kWords;
   __shared__ float4 s_rec[kTileThreads / 32][32 * Rec<N>::kWords];
+  __shared__ alignas(256) float4 s_pair[kTileThreads / 32][PairSmem<N>::kFloats / 4];
   const int c = blockIdx.x;
   if (c >= (int)*chunk_total) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  float* sp = reinterpret_cast<float*>(s_pair[warp]);
+  const uint32_t sp_own = (uint32_t)__cvta_generic_to_shared(sp) + 16u * (lane >> 1);
+  const bool odd = lane & 1;
   const int t = chunk_tile[c];
   if (t < 0) return;  // a slot that its event does not need (k_build)
   const int a_loc = (c - (int)chunk_off[t]) * kChunkWarps + warp;  // block of the tile
@@ -1885,7 +1915,16 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
     wl[d] = warp_min_i(hv ? lo[d] : INT_MAX);
     wh[d] = warp_max_i(hv ? hi[d] : INT_MIN);
   }
-  const float tdc = kp.t_dc;
+  const float tdc = kp.t_dc, thr = hv ? tdc : -INFINITY;
+  float hlo[N], hhi[N];  // box of block A
+  unsigned long long x2[N];
+#pragma unroll
+  for (int d = 0; d < N; ++d) {
+    hlo[d] = warp_min_f(hv ? x[d] : INFINITY);
+    hhi[d] = warp_max_f(hv ? x[d] : -INFINITY);
+    x2[d] = pk2(make_float2(x[d], x[d]));
+  }
+  const unsigned long long one = pk2(make_float2(kp.one, kp.one));
   const float scale = ldexpf(1.0f, fix_exponent(g, kmax));
   auto kval = [&](float s, bool self) -> float {
     if (FORM == kDensExpUnit) return ex2_approx(kexp * (M::kRoot ? sqrt_approx(s) : s));
@@ -1953,55 +1992,77 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
     if (u >= t && !dcheck_bad(st, u, kp.ntiles, kChkDensityTile)) {
       const int pb = off[u], pe = off[u + 1];
       const int nb = (pe - pb + 31) >> 5;
-      for (int b = (u == t ? a_loc + 1 : 0); b < nb; ++b) {
-        float bb[4 * BW];
-        load_box<N>(tblk, (int)bo[u] + b, bb);
-        const bool need = hv && lower_point<N, M>(x, bb, bb + N, kp.mpar) <= tdc;
-        if (!__any_sync(0xffffffffu, need)) continue;
-        const int first = pb + (b << 5);
-        const int cntB = min(32, pe - first);
-        const bool cv = lane < cntB;
-        // lane m owns candidate m of the block; at step k lane l meets candidate l ^ k and the
-        // candidate's owner collects the term from lane m ^ k = l (butterfly shuffles with
-        // immediate lane masks), so no value is carried from one step to the next
-        float ox[N], ow;
-        load_rec<N>(rec_m, first + (cv ? lane : 0), ox, ow);
-        if (!cv) {
-#pragma unroll
-          for (int d = 0; d < N; ++d) ox[d] = INFINITY;  // never within dc
-          ow = 0.0f;
+      const int b0 = u == t ? a_loc + 1 : 0, box0 = (int)bo[u];
+      // the block boxes are tested 32 at a time against the box of block A, and those in reach by
+      // every lane for its own point
+      for (int c0 = b0; c0 < nb; c0 += 32) {
+        bool near = false;
+        if (c0 + lane < nb) {
+          float bb[4 * BW];
+          load_box<N>(tblk, box0 + c0 + lane, bb);
+          near = lower_box<N, M>(hlo, hhi, bb, bb + N, kp.mpar) <= tdc;
         }
-        // two steps at a time, with paired arithmetic; the own terms of this block are summed
-        // (fused multiply-add) in two running sums, even and odd steps, added at the block's end
-        float2 acc2 = make_float2(0.0f, 0.0f), cacc2 = make_float2(0.0f, 0.0f);
-        const float2 wi2 = make_float2(wi, wi);
+        for (unsigned mask = __ballot_sync(0xffffffffu, near); mask; mask &= mask - 1) {
+          const int b = c0 + __ffs(mask) - 1;
+          float bb[4 * BW];
+          load_box<N>(tblk, box0 + b, bb);
+          const bool need = hv && lower_point<N, M>(x, bb, bb + N, kp.mpar) <= tdc;
+          if (!__any_sync(0xffffffffu, need)) continue;
+          const int first = pb + (b << 5);
+          const int cntB = min(32, pe - first);
+          const bool cv = lane < cntB;
+          // lane m owns candidate m of the block; at step k lane l meets candidate l ^ k and the
+          // candidate's owner collects the term from lane m ^ k = l (butterfly shuffles with
+          // immediate lane masks), so no value is carried from one step to the next
+          {
+            float ox[N + 1];
+            load_rec<N>(rec_m, first + (cv ? lane : 0), ox, ox[N]);
+            if (!cv) {
 #pragma unroll
-        for (int k = 0; k < 32; k += 2) {
-          float ca[N], cb[N];
+              for (int d = 0; d < N; ++d) ox[d] = INFINITY;  // never within dc
+              ox[N] = 0.0f;
+            }
+            __syncwarp();  // the previous block's readers are done
 #pragma unroll
-          for (int d = 0; d < N; ++d) {
-            ca[d] = __shfl_xor_sync(0xffffffffu, ox[d], k);
-            cb[d] = __shfl_xor_sync(0xffffffffu, ox[d], k + 1);
+            for (int j = 0; j <= N; ++j) {
+              sp[(j / 2) * 64 + (lane >> 1) * 4 + (j & 1) * 2 + (lane & 1)] = ox[j];
+            }
+            __syncwarp();
           }
-          const float2 cw = make_float2(__shfl_xor_sync(0xffffffffu, ow, k), __shfl_xor_sync(0xffffffffu, ow, k + 1));
-          const float2 sd = partial_pair<N, MT>(x, ca, cb, kp.mpar);
-          const bool ix = hv && sd.x <= tdc, iy = hv && sd.y <= tdc;
-          if ((VAR & 1) == 0 || __any_sync(0xffffffffu, ix || iy)) {
-            float2 kv = kval2(sd);
-            kv.x = ix ? kv.x : 0.0f;
-            kv.y = iy ? kv.y : 0.0f;
-            acc2 = fma2(kv, cw, acc2);
-            const float2 tc = mul2(kv, wi2);
-            cacc2 = add2(cacc2, make_float2(__shfl_xor_sync(0xffffffffu, tc.x, k),
-                                            __shfl_xor_sync(0xffffffffu, tc.y, k + 1)));
+          // two steps at a time, with paired arithmetic; the own terms of this block are summed
+          // (fused multiply-add) in two running sums, even and odd steps (in the other order in odd
+          // lanes, which meet a pair's second candidate first), added at the block's end
+          float2 acc2 = make_float2(0.0f, 0.0f), cacc2 = make_float2(0.0f, 0.0f);
+          const float2 wi2 = make_float2(wi, wi);
+#pragma unroll
+          for (int k = 0; k < 32; k += 2) {
+            unsigned long long c2[N + 1];
+            load_pairs<N>(sp_own ^ (uint32_t)(8 * k), c2);
+            const float2 cw = upk2(c2[N]);
+            const float2 sd = partial_packed<N, MT>(x2, c2, kp.mpar, one);
+            const bool ix = sd.x <= thr, iy = sd.y <= thr;
+            if ((VAR & 1) == 0 || __any_sync(0xffffffffu, ix || iy)) {
+              float2 kv;
+              if constexpr (FORM == kDensGeneric || (VAR & 2) != 0) {
+                kv = kval2(sd);
+                kv.x = ix ? kv.x : 0.0f;
+                kv.y = iy ? kv.y : 0.0f;
+              } else {
+                kv = kernel_within<FORM == kDensExpUnit, M::kRoot>(sd, thr, kexp2);
+              }
+              acc2 = fma2(kv, cw, acc2);
+              const float2 tc = mul2(kv, wi2);
+              const float t0 = odd ? tc.y : tc.x, t1 = odd ? tc.x : tc.y;  // of steps k and k + 1
+              cacc2 = add2(cacc2, make_float2(__shfl_xor_sync(0xffffffffu, t0, k), __shfl_xor_sync(0xffffffffu, t1, k + 1)));
+            }
           }
-        }
-        acc = fadd(acc, fadd(acc2.x, acc2.y));
-        const float cacc = fadd(cacc2.x, cacc2.y);
-        if (cv && cacc != 0.0f) {
-          const int mi = order_at(mq, first + lane);
-          if (!dcheck_bad(st, mi, kp.n, kChkDensityMirror))
-            atomicAdd(reinterpret_cast<unsigned long long*>(rho_fix + mi), (unsigned long long)__float2ll_rn(cacc * scale));
+          acc = fadd(acc, fadd(acc2.x, acc2.y));
+          const float cacc = fadd(cacc2.x, cacc2.y);
+          if (cv && cacc != 0.0f) {
+            const int mi = order_at(mq, first + lane);
+            if (!dcheck_bad(st, mi, kp.n, kChkDensityMirror))
+              atomicAdd(reinterpret_cast<unsigned long long*>(rho_fix + mi), (unsigned long long)__float2ll_rn(cacc * scale));
+          }
         }
       }
     }
@@ -2608,7 +2669,8 @@ constexpr int kJumpIters = 4096;
 
 template <int N>
 clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
-  const KParams& kp = a.kp;
+  KParams kp = a.kp;
+  kp.one = 1.0f;
   const int n = kp.n;
   InPtrs in{};
   for (int d = 0; d < N; ++d) in.c[d] = a.coords[d];

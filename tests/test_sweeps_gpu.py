@@ -72,3 +72,22 @@ def test_label_chains(gpu_context, n, fall, blocking):
     assert isinstance(info, capi.RunInfo) and info.n_clusters == ref.stats["n_clusters"]
     for k, t in out.items():
         np.testing.assert_array_equal(t.cpu().numpy(), getattr(ref, k), err_msg=k)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 64, 127, 1025])
+@pytest.mark.parametrize("ndim", [1, 2, 3, 4, 9])
+@pytest.mark.parametrize("kernel,metric", [(("exp", (1.0, 1.0)), "euclidean"), (("gaus", (0.0, 0.5, 1.0)), "euclidean"),
+                                           (("exp", (1.0, 1.0)), "manhattan"), (("gaus", (0.0, 0.5, 1.0)), "chebyshev"),
+                                           (("gaus", (1.0, 2.0, 1.5)), "euclidean")])
+def test_symmetric_density_edges(gpu_context, n, ndim, kernel, metric):
+    """Whole and partial blocks against each other, every kernel form and metric of the symmetric sweep,
+    by the tolerance rule (densities within 1e-5 of FP64, everything after them exact)."""
+    from oracle import oracle as O
+    from parity_util import check_tolerant, gpu_args, oracle_cfg
+    rng = np.random.default_rng(100 * n + ndim)
+    c, w = random_blobs(rng, n, ndim, nblobs=min(3, n), extent=25.0, sigma=1.0)
+    for dc in (0.7, 3.0, 100.0):
+        kw = dict(dc=dc, rhoc=1.0, dm=1.3 * dc, kernel=kernel, metric=(metric, ()), ppbin=100)
+        got = gpu_context.make_clusters_host(c, w, *gpu_args(**kw))
+        cfg = oracle_cfg(**kw)
+        check_tolerant(c, w, cfg, got, ref=O.run(c, w, cfg), rtol=1e-5)

@@ -427,9 +427,9 @@ using namespace clue_b200;
 // An executable graph kept for the next call's pipeline, and the cluster size of its k_build launch:
 // an update in place keeps a kernel node's cluster size, so each size has an executable of its own.
 struct GraphSlot {
-  static constexpr int kSizes = 5;  // none, 1, 2, 4, 8 CTAs
+  static constexpr int kSizes = 6;  // none, 1, 2, 4, 8, 16 CTAs
   cudaGraphExec_t exec[kSizes] = {};
-  cudaGraphExec_t& at(int ranks) { return exec[ranks >= 8 ? 4 : (ranks >= 4 ? 3 : ranks)]; }
+  cudaGraphExec_t& at(int ranks) { return exec[ranks >= 16 ? 5 : (ranks >= 8 ? 4 : (ranks >= 4 ? 3 : ranks))]; }
   void destroy() {
     for (auto& e : exec)
       if (e) cudaGraphExecDestroy(e);

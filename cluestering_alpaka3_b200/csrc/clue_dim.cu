@@ -884,13 +884,13 @@ __global__ void __launch_bounds__(256) k_gather_morton(const float4* __restrict_
   }
 }
 
-// ---- stage 1 in one launch: events of up to kBuildPoints points -----------------
+// ---- stage 1 in one launch: single events of up to kBuildPoints points, small batches ----------
 // A cluster of CTAs takes one event through the whole stage: bounding box, grid, tile and Morton keys,
 // the stable radix sorts, records, tile offsets, chunks and the symmetric density's block boxes.
 // Its CTAs exchange digit counts through distributed shared memory and the keys through L2, with a
 // cluster barrier between steps.  Bound by the latency of its steps (a radix pass of 16k points takes
 // about 5 us, one of 1000 points 2 us), where a launch takes 2 to 3 us: stage 1 of a flat event was
-// 24 launches, 125 us of direct launches for 16k points against 42 us, 180 against 92 us for 50k.
+// 24 launches, 125 us of direct launches for 16k points against 40 us, 163 against 73 us for 65k.
 
 // Shared memory of one CTA of a build cluster.
 template <int N, int W>
@@ -2566,9 +2566,10 @@ void launch_near_ties(const KParams& kp, Workspace& ws, cudaStream_t s) {
 
 // Whether k_build takes the call: keys of 32 bits, and sizes where a few clusters beat the whole
 // chip's separate launches.  Whole calls, k_build against separate launches: one flat 2-D event of 16k
-// points 133 against 207 us, 40k 186 / 233, 65k 216 / 232, 100k 285 / 262; 24 events of 3300 4-D
-// points 167 / 246, 64 events 269 / 318, 100 2-D events of 3300 points 293 / 333, 300 events 798 / 756.
-constexpr int kBuildPoints = 65536;        // of a single event
+// points 134 against 180 us, 40k 173 / 233, 65k 183 / 233, 131k 261 / 283 (a 3-D one with the symmetric
+// density 293 / 304); 24 events of 3300 4-D points 167 / 246, 64 events 269 / 318, 100 2-D events of
+// 3300 points 293 / 333, 300 events 798 / 756.
+constexpr int kBuildPoints = 131072;       // of a single event
 constexpr int kBuildBatchPoints = 1 << 19;  // of a batch, each event at most kBuildEventPoints
 constexpr int kBuildEventPoints = 32768;
 constexpr int kBuildTileBits = 16;
@@ -2578,11 +2579,12 @@ inline bool build_takes(const KParams& kp, int max_points, int tile_bits, int mb
   // a batch's chunks and blocks have slots per event (k_build): they must fit the buffers
   return kp.n <= kBuildBatchPoints && max_points <= kBuildEventPoints && kp.n / 32 + kp.ntiles + 1 <= kp.n;
 }
-// CTAs per cluster: of 1024 threads for a single event, about a point per thread and more from 8192
-// points on; of 512 threads for a batch, as many as leave the clusters on the chip together (24 events:
-// 8 CTAs 167 us, 4 176; 100 events: 4 CTAs 293 us, 8 319, 2 317).
+// CTAs per cluster: of 1024 threads for a single event, about a point per thread up to 16 CTAs (6k
+// points: 8 CTAs 122 us, 16 123; 16k: 8 CTAs 136 us, 16 134; 65k: 209, 183); of 512 threads for a batch,
+// as many as leave the clusters on the chip together (24 events: 8 CTAs 167 us, 4 176; 100 events: 4
+// CTAs 293 us, 8 319, 2 317).  16 is beyond the portable cluster size, which the launch asks for.
 inline int build_ranks(int n_events, int n) {
-  if (n_events == 1) return n <= 1024 ? 1 : (n <= 2048 ? 2 : (n <= 4096 ? 4 : 8));
+  if (n_events == 1) return n <= 1024 ? 1 : (n <= 2048 ? 2 : (n <= 4096 ? 4 : (n <= 8192 ? 8 : 16)));
   return n_events <= 64 ? 8 : (n_events <= 128 ? 4 : (n_events <= 256 ? 2 : 1));
 }
 
@@ -2599,6 +2601,7 @@ void launch_build_cluster(const KParams& kp, const InPtrs& in, EvGrid* eg, const
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (ranks > 8) cudaFuncSetAttribute(k_build<N, W>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaLaunchKernelEx(&cfg, k_build<N, W>, kp, in, eg, o, two, mbits, tile_passes, passes, ranks);
 }
 

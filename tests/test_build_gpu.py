@@ -1,4 +1,4 @@
-"""The one-launch first stage (events of up to 65536 points): sizes around its clusters, tile counts around
+"""The one-launch first stage (single events of up to 131072 points, small batches): sizes around its clusters, tile counts around
 its radix digits, and the same bits as the separate launches that larger calls take."""
 import numpy as np
 import pytest
@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,ppbin", [(1, 128), (2, 1), (32, 128), (33, 4), (1023, 128), (1025, 128), (2049, 7),
-                                     (4097, 128), (8193, 20), (30000, 60), (65535, 128), (65536, 128), (65537, 128)])
+                                     (4097, 128), (8192, 128), (8193, 20), (30000, 60), (65537, 128), (131072, 128),
+                                     (131073, 128)])
 @pytest.mark.parametrize("ndim", [1, 2, 3])
 def test_sizes_against_oracle(gpu_context, n, ppbin, ndim):
     rng = np.random.default_rng(n + ndim)
@@ -65,7 +66,7 @@ def test_same_bits_as_separate_launches(gpu_context, kernel, metric, wrapped):
 def test_graphs_of_alternating_cluster_sizes(gpu_context):
     """Blocking calls keep one executable graph per cluster size."""
     rng = np.random.default_rng(3)
-    evs = [random_blobs(rng, n, 2, nblobs=5, extent=40.0) for n in (9000, 700, 3000, 70000, 1500, 9001, 700)]
+    evs = [random_blobs(rng, n, 2, nblobs=5, extent=40.0) for n in (9000, 700, 3000, 140000, 5000, 1500, 9001, 700)]
     for _ in range(2):
         for c, w in evs:
             assert_exact(*run_both(gpu_context, c, w, dc=1.0, rhoc=2.0, dm=1.5))

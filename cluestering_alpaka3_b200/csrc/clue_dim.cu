@@ -1348,12 +1348,12 @@ __device__ __forceinline__ bool chunk_home(const KParams& kp, Events ev, const i
 // candidate with d <= dc; candidates beyond dc contribute +-0 and are skipped.
 //
 // The homes of a warp are 32 neighbours of a tile's Morton order, so most candidates of its
-// search-box tiles are out of every lane's reach: the lanes read 32 candidates at a time (in index
+// search-box tiles are out of every lane's reach: the lanes read 64 candidates at a time (in index
 // order), keep those within dc of the box of the warp's homes, and append them to the warp's buffer
 // in shared memory, coordinates and terms by dimension.  What is kept is summed 32 at a time, four
 // candidates per load with paired differences and squares: 7 instructions a candidate, where staging
 // whole tiles by bulk copy and testing every candidate took about 12.  Bound by instruction issue on
-// large inputs and by the sums' own chain of additions where a scheduler has one warp: 0.66 -> 0.32 ms
+// large inputs and by the sums' own chain of additions where a scheduler has one warp: 0.66 -> 0.31 ms
 // on 1M 2-D points, 67 -> 36 us on 16k (homes in Morton order as they are; grouping them by the
 // tiles their search boxes reach, in a pass of 25 us, is not needed any more).
 template <int N, int MT>
@@ -1362,8 +1362,8 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4)) k_density(
     const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ chunk_total,
     const float4* __restrict__ rec_w, const int32_t* __restrict__ mq, float4* __restrict__ rec_r) {
   using M = Metric<N, MT>;
-  // coordinates and flat-kernel terms (or weights) of up to 64 kept candidates: two halves of 32
-  __shared__ ulonglong2 s_buf[kChunkWarps][N + 1][16];
+  // coordinates and flat-kernel terms (or weights) of the kept candidates, a ring of 128
+  __shared__ ulonglong2 s_buf[kChunkWarps][N + 1][32];
   ChunkHome h;
   if (!chunk_home(kp, ev, off, chunk_tile, chunk_off, chunk_total, h)) return;
   const bool valid = h.valid;
@@ -1404,7 +1404,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4)) k_density(
     auto sum = [&](int f0, int f1) {
       // groups of four that hold some home's own point, whose term is its weight
       const unsigned own = __reduce_or_sync(0xffffffffu, self >= f0 && self < f1 ? 1u << ((self - f0) >> 2) : 0u);
-      const int q0 = (f0 >> 2) & 15;
+      const int q0 = (f0 >> 2) & 31;
       auto four = [&](int q, bool tail) {
         float2 s2[2];
         ulonglong2 c2[N];
@@ -1450,26 +1450,36 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4)) k_density(
         for (int q = 0; f0 + 4 * q < f1; ++q) four(q, f0 + 4 * q + 4 > f1);
       }
     };
-    float c[N], w;
-    load_rec<N>(rec_w, min(pb + lane, pe - 1), c, w);
-    for (int base = pb; base < pe; base += 32) {
-      const bool last = base + 32 >= pe;
-      const bool keep = base + lane < pe && (!kp.lb_ok || lower_point<N, M>(c, hlo, hhi, kp.mpar) <= tdc);
-      const unsigned m = __ballot_sync(0xffffffffu, keep);
-      const int was = fill;
-      if (keep) {
-        const int slot = (was + __popc(m & lt)) & 63;
+    int done = 0;  // candidates summed so far, a multiple of 32
+    float c[2][N], w[2];
 #pragma unroll
-        for (int d = 0; d < N; ++d) reinterpret_cast<float*>(s_buf[warp][d])[slot] = c[d];
-        reinterpret_cast<float*>(s_buf[warp][N])[slot] = flat ? fmul(kflat, w) : w;
-      }
-      fill += __popc(m);
+    for (int k = 0; k < 2; ++k) load_rec<N>(rec_w, min(pb + 32 * k + lane, pe - 1), c[k], w[k]);
+    for (int base = pb; base < pe; base += 64) {
+      const bool last = base + 64 >= pe;
+      bool keep[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        keep[k] = base + 32 * k + lane < pe && (!kp.lb_ok || lower_point<N, M>(c[k], hlo, hhi, kp.mpar) <= tdc);
+      const unsigned m0 = __ballot_sync(0xffffffffu, keep[0]), m1 = __ballot_sync(0xffffffffu, keep[1]);
+      const int mid = fill + __popc(m0);
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (keep[k]) {
+          const int slot = ((k ? mid : fill) + __popc((k ? m1 : m0) & lt)) & 127;
+#pragma unroll
+          for (int d = 0; d < N; ++d) reinterpret_cast<float*>(s_buf[warp][d])[slot] = c[k][d];
+          reinterpret_cast<float*>(s_buf[warp][N])[slot] = flat ? fmul(kflat, w[k]) : w[k];
+        }
       const int o = pos - base;  // (a home always lies within its warp's box)
-      if (o >= 0 && o < 32) self = was + __popc(m & ((1u << o) - 1u));
-      if (!last) load_rec<N>(rec_w, min(base + 32 + lane, pe - 1), c, w);  // while the kept ones are summed
+      if (o >= 0 && o < 64) self = (o < 32 ? fill : mid) + __popc((o < 32 ? m0 : m1) & ((1u << (o & 31)) - 1u));
+      fill = mid + __popc(m1);
+      if (!last) {  // the next ones, while the kept ones are summed
+#pragma unroll
+        for (int k = 0; k < 2; ++k) load_rec<N>(rec_w, min(base + 64 + 32 * k + lane, pe - 1), c[k], w[k]);
+      }
       __syncwarp();
-      if ((was ^ fill) & ~31) sum(was & ~31, (was & ~31) + 32);
-      if (last && (fill & 31)) sum(fill & ~31, fill);
+      for (; done + 32 <= fill; done += 32) sum(done, done + 32);
+      if (last && done < fill) sum(done, fill);
       __syncwarp();
     }
   });
@@ -2310,14 +2320,13 @@ __global__ void __launch_bounds__(1024) k_seed_labels_one(const KParams kp, Even
 // At most `iters` jumps per point per launch; a launch that leaves a point unresolved records
 // it in st->unresolved[round] and the next launch continues.  With LABELS every point that
 // reaches its root gets its label.
-template <bool LABELS>
+template <bool LABELS, int K>
 __device__ __forceinline__ void jump(int32_t* par, const int32_t* __restrict__ perm, int32_t* __restrict__ label,
                                      int n, int iters, DevStatus* st, int round) {
   bool unres = false;
   const int stride = gridDim.x * blockDim.x;
-  // four chains per thread walked in lockstep: each step's four parent loads are independent,
-  // so they are in flight together (the walk is bound by load latency, not bandwidth)
-  constexpr int K = 4;
+  // K chains per thread walked in lockstep: each step's parent loads are independent, so they are in
+  // flight together (the walk is bound by load latency, not bandwidth)
   for (int64_t pos0 = blockIdx.x * blockDim.x + threadIdx.x; pos0 < n; pos0 += (int64_t)K * stride) {
     int p[K], i[K];
     bool act[K];
@@ -2363,17 +2372,21 @@ __device__ __forceinline__ void jump(int32_t* par, const int32_t* __restrict__ p
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(&st->label_rounds, (uint32_t)round + 1);
 }
 
-// First round: the climb that ends most chains writes the labels as well.
+// First round: the climb that ends most chains writes the labels as well.  Four chains per thread from
+// 2M points on, one below, where there are threads enough (label stage: 4M points 0.075 ms against
+// 0.091 with one; 1M points 0.056 ms with four, 0.048 with one).
+constexpr int kLabelChainPoints = 1 << 21;
+template <int K>
 __global__ void __launch_bounds__(256) k_labels(int32_t* par, const int32_t* __restrict__ perm,
                                                 int32_t* __restrict__ label, int n, int iters, int rounds,
                                                 DevStatus* st) {
   if (blockIdx.x == 0 && threadIdx.x == 0) st->label_enqueued = (uint32_t)rounds;
-  jump<true>(par, perm, label, n, iters, st, 0);
+  jump<true, K>(par, perm, label, n, iters, st, 0);
 }
 
 __global__ void __launch_bounds__(256) k_jump(int32_t* par, int n, int iters, DevStatus* st, int round) {
   if (st->unresolved[round - 1] == 0) return;
-  jump<false>(par, nullptr, nullptr, n, iters, st, round);
+  jump<false, 4>(par, nullptr, nullptr, n, iters, st, round);
 }
 
 // All labels again, from parents that name roots, when the first round left a chain unresolved.
@@ -2833,8 +2846,8 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
                                      l);
     launches += scan_launches(n) + kBfsLevels + 3;  // count, scan, fill, seeds, levels
   }
-  k_labels<<<grid_for(n, 256), 256, 0, s>>>(ws.par, ws.perm, a.out.cluster_index, n, kJumpIters,
-                                           a.blocking ? 1 : kJumpLaunches, ws.status);
+  (n < kLabelChainPoints ? k_labels<1> : k_labels<4>)<<<grid_for(n, 256), 256, 0, s>>>(
+      ws.par, ws.perm, a.out.cluster_index, n, kJumpIters, a.blocking ? 1 : kJumpLaunches, ws.status);
   if (!a.blocking) {
     for (int r = 1; r < kJumpLaunches; ++r)
       k_jump<<<grid_for(n, 256), 256, 0, s>>>(ws.par, n, kJumpIters, ws.status, r);

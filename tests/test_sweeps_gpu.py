@@ -36,7 +36,7 @@ def test_nearest_higher_lattice(gpu_context, n, ppbin, wrapped):
                                tiebreak=tiebreak))
 
 
-@pytest.mark.parametrize("n", [1, 4, 31, 32, 33, 63, 64, 65, 127, 130, 1021])
+@pytest.mark.parametrize("n", [1, 4, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 130, 1021])
 @pytest.mark.parametrize("ndim,metric,wrapped", [
     (1, ("euclidean", ()), ()), (2, ("euclidean", ()), ()), (2, ("periodic_euclidean", (0.0, 40.0)), (0, 1)),
     (3, ("weighted_euclidean", (0.5, 2.0, 1.0)), ()), (4, ("chebyshev", ()), ()), (9, ("manhattan", ()), ()),

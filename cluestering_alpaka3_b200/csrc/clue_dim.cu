@@ -135,23 +135,6 @@ __device__ __forceinline__ void store_rec(float4* __restrict__ rec, int pos, con
     rec[(size_t)pos * W + k] = make_float4(buf[4 * k], buf[4 * k + 1], buf[4 * k + 2], buf[4 * k + 3]);
 }
 
-template <int N>
-__device__ __forceinline__ void unpack_rec(const float4* r, float* c, float& payload) {
-  constexpr int W = Rec<N>::kWords;
-  float buf[4 * W];
-#pragma unroll
-  for (int k = 0; k < W; ++k) {
-    const float4 v = r[k];
-    buf[4 * k + 0] = v.x;
-    buf[4 * k + 1] = v.y;
-    buf[4 * k + 2] = v.z;
-    buf[4 * k + 3] = v.w;
-  }
-#pragma unroll
-  for (int d = 0; d < N; ++d) c[d] = buf[d];
-  payload = buf[Rec<N>::kPayload];
-}
-
 // Search box of one point in "virtual" bins: the reference's [getBin(x - r), getBin(x + r)]
 // (TilesView.hpp:72-82, wrapped boxes extended by nperdim), shifted down by nperdim when a
 // wrapped box starts above the home bin, so that every lane of a warp expresses its box

@@ -179,7 +179,6 @@ struct Workspace {
   size_t pipe_pinned_bytes = 0;
 
   int32_t* perm = nullptr;  // alias of the sorted values buffer after the tile sort
-  uint32_t* sorted_keys = nullptr;
 
   int build_ranks = 0;  // CTAs per cluster of the last run's k_build launch, 0 without one
   KParams last_kp{};  // parameters of the last enqueued run (for clue_context_read_info)

@@ -2104,7 +2104,8 @@ __global__ void __launch_bounds__(1024) k_boxes(const KParams kp, Events ev, con
   if (b < nblk) {
     const int q = (b << 5) + lane;
     const bool valid = q < n;
-    const int qq = valid ? q : b << 5;  // lanes past the end repeat the first record
+    // lanes past the end repeat the last record: warp_event takes the last lane's for the largest
+    const int qq = min(q, n - 1);
     float x[N], pl;
     if (GATHER) {
       load_rec<N>(rec, mq[qq], x, pl);

@@ -2374,9 +2374,12 @@ __global__ void __launch_bounds__(256) k_jump(int32_t* par, int n, int iters, De
 }
 
 // All labels again, from parents that name roots, when the first round left a chain unresolved.
+// `rounds` have been enqueued by now (a blocking call's host adds to the one of k_labels), so a status
+// read after this call finds the last one's outcome.
 __global__ void __launch_bounds__(256) k_labels_again(const int32_t* __restrict__ par,
                                                       const int32_t* __restrict__ perm, int32_t* __restrict__ label,
-                                                      int n, DevStatus* st) {
+                                                      int n, int rounds, DevStatus* st) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) st->label_enqueued = (uint32_t)rounds;
   if (st->unresolved[0] == 0) return;
   const int stride = gridDim.x * blockDim.x;
   for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < n; pos += stride) {
@@ -2835,7 +2838,7 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
   if (!a.blocking) {
     for (int r = 1; r < kJumpLaunches; ++r)
       k_jump<<<grid_for(n, 256), 256, 0, s>>>(ws.par, n, kJumpIters, ws.status, r);
-    k_labels_again<<<grid_for(n, 256), 256, 0, s>>>(ws.par, ws.perm, a.out.cluster_index, n, ws.status);
+    k_labels_again<<<grid_for(n, 256), 256, 0, s>>>(ws.par, ws.perm, a.out.cluster_index, n, kJumpLaunches, ws.status);
   }
   stage_mark(ws, 4, s);
   // Morton boxes, nearest higher, labels
@@ -2849,15 +2852,14 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
 template <int N>
 clue_status finish_labels(Workspace& ws, const RunArgs& a, cudaStream_t s, int first_round) {
   const int n = a.kp.n;
-  for (int r = first_round; r < 64; ++r) {
+  int r = first_round;
+  for (uint32_t unres = 1; unres != 0 && r < 64; ++r) {
     k_jump<<<grid_for(n, 256), 256, 0, s>>>(ws.par, n, kJumpIters, ws.status, r);
     ++ws.launches;
-    uint32_t unres = 0;
     CLUE_CUDA_TRY(cudaMemcpyAsync(&unres, &ws.status->unresolved[r], 4, cudaMemcpyDeviceToHost, s));
     CLUE_CUDA_TRY(cudaStreamSynchronize(s));
-    if (unres == 0) break;
   }
-  k_labels_again<<<grid_for(n, 256), 256, 0, s>>>(ws.par, ws.perm, a.out.cluster_index, n, ws.status);
+  k_labels_again<<<grid_for(n, 256), 256, 0, s>>>(ws.par, ws.perm, a.out.cluster_index, n, r, ws.status);
   ++ws.launches;
   CLUE_CUDA_TRY(cudaGetLastError());
   return CLUE_OK;

@@ -138,25 +138,30 @@ __global__ void __launch_bounds__(kSilThreads) k_silhouette(const int32_t* __res
   if (p < m && b < FLT_MAX) atomicMin(other + p, __float_as_uint(b));  // means are not negative
 }
 
-// Scores in point order (NaN for points that are not scored), and which points are scored.
+// Scores in point order (NaN for points that are not scored), for the caller (optional) and for the
+// mean, and which points are scored; nothing after a label out of range (reported by the host).
 __global__ void __launch_bounds__(256) k_sil_score(int n, const int32_t* __restrict__ cluster_index,
                                                    const int32_t* __restrict__ offsets,
                                                    const int32_t* __restrict__ points, const CsrInfo* info,
                                                    const float* __restrict__ own_mean,
-                                                   const uint32_t* __restrict__ other, float* __restrict__ score,
-                                                   uint8_t* __restrict__ scored) {
+                                                   const uint32_t* __restrict__ other, float* __restrict__ per_point,
+                                                   float* __restrict__ score, uint8_t* __restrict__ scored) {
+  if (info->bad) return;
   const int m = info->n_clustered, stride = gridDim.x * blockDim.x;
   const int first = blockIdx.x * blockDim.x + threadIdx.x;
   for (int i = first; i < n; i += stride)
     if (cluster_index[i] < 0 || cluster_index[i] >= n) {
       score[i] = NAN;
+      if (per_point) per_point[i] = NAN;
       scored[i] = 0;
     }
   for (int p = first; p < m; p += stride) {
     const int i = points[p], c = cluster_index[i];
     const bool valid = offsets[c + 1] - offsets[c] >= 2;
     const float a = own_mean[p], b = __uint_as_float(other[p]);
-    score[i] = valid ? __fdiv_rn(__fsub_rn(b, a), a < b ? b : a) : NAN;  // std::max(a, b)
+    const float v = valid ? __fdiv_rn(__fsub_rn(b, a), a < b ? b : a) : NAN;  // std::max(a, b)
+    score[i] = v;
+    if (per_point) per_point[i] = v;
     scored[i] = valid ? 1 : 0;
   }
 }
@@ -164,14 +169,15 @@ __global__ void __launch_bounds__(256) k_sil_score(int n, const int32_t* __restr
 template <int N>
 void launch_silhouette(int n, const float* coords, const int32_t* cluster_index, const int32_t* offsets,
                        const int32_t* points, const CsrInfo* info, float* rec, float* own_mean, uint32_t* other,
-                       float* score, uint8_t* scored, cudaStream_t s) {
+                       float* per_point, float* score, uint8_t* scored, cudaStream_t s) {
   const int blocks = std::max(1, std::min((n + 255) / 256, 148 * 16));
   k_sil_gather<N><<<blocks, 256, 0, s>>>(n, coords, points, info, rec, other);
   // enough parts for four waves of 16 blocks an SM, and no part below 64 points
   const int64_t pb = (n + kSilThreads - 1) / kSilThreads;
   const int64_t parts = std::max<int64_t>(1, std::min<int64_t>({(int64_t)148 * 64 / pb, (int64_t)n / 64, 65535}));
   k_silhouette<N><<<dim3((unsigned)pb, (unsigned)parts), kSilThreads, 0, s>>>(offsets, info, rec, own_mean, other);
-  k_sil_score<<<blocks, 256, 0, s>>>(n, cluster_index, offsets, points, info, own_mean, other, score, scored);
+  k_sil_score<<<blocks, 256, 0, s>>>(n, cluster_index, offsets, points, info, own_mean, other, per_point, score,
+                                     scored);
 }
 
 constexpr int kCenThreads = 128;
@@ -295,6 +301,7 @@ clue_status clue_silhouette(clue_context ctx, int32_t ndim, int32_t n, const flo
   const size_t o_score = 256, o_scored = o_score + nn * 4, o_off = up256(o_scored + nn), o_pts = o_off + up256((nn + 1) * 4),
                o_rec = o_pts + up256(nn * 4), o_own = o_rec + up256(nn * rec_floats * 4), o_other = o_own + up256(nn * 4),
                total = o_other + up256(nn * 4);
+  const size_t back = mean ? o_scored + nn : sizeof(CsrInfo);
   clue_status st = post_reserve(ws, total, o_scored + nn);
   if (st != CLUE_OK) return st;
   char* base = static_cast<char*>(ws.post);
@@ -315,19 +322,18 @@ clue_status clue_silhouette(clue_context ctx, int32_t ndim, int32_t n, const flo
   if (st == CLUE_OK) {
 #define CLUE_SIL(N)                                                                                              \
   case N:                                                                                                        \
-    launch_silhouette<N>(n, coords, cluster_index, offsets, points, info, rec, own_mean, other, score, scored, s); \
+    launch_silhouette<N>(n, coords, cluster_index, offsets, points, info, rec, own_mean, other, per_point,       \
+                         score, scored, s);                                                                      \
     break;
     switch (ndim) {
       CLUE_SIL(1) CLUE_SIL(2) CLUE_SIL(3) CLUE_SIL(4) CLUE_SIL(5) CLUE_SIL(6) CLUE_SIL(7) CLUE_SIL(8) CLUE_SIL(9)
-      default: launch_silhouette<10>(n, coords, cluster_index, offsets, points, info, rec, own_mean, other, score,
-                                     scored, s);
+      default: launch_silhouette<10>(n, coords, cluster_index, offsets, points, info, rec, own_mean, other, per_point,
+                                     score, scored, s);
     }
 #undef CLUE_SIL
     ws.launches += 3;
     e = cudaGetLastError();
-    if (e == cudaSuccess && per_point) e = cudaMemcpyAsync(per_point, score, nn * 4, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(ws.post_host, base, mean ? o_scored + nn : sizeof(CsrInfo), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ws.post_host, base, back, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   }
   cudaSetDevice(prev);

@@ -302,7 +302,7 @@ clue_status clue_silhouette(clue_context ctx, int32_t ndim, int32_t n, const flo
                o_rec = o_pts + up256(nn * 4), o_own = o_rec + up256(nn * rec_floats * 4), o_other = o_own + up256(nn * 4),
                total = o_other + up256(nn * 4);
   const size_t back = mean ? o_scored + nn : sizeof(CsrInfo);
-  clue_status st = post_reserve(ws, total, o_scored + nn);
+  clue_status st = post_reserve(ws, total, back);
   if (st != CLUE_OK) return st;
   char* base = static_cast<char*>(ws.post);
   CsrInfo* info = reinterpret_cast<CsrInfo*>(base);

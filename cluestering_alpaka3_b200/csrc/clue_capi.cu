@@ -193,12 +193,18 @@ static void wait_idle(Workspace& ws) {
 clue_status workspace_reserve(Workspace& ws, int ndim, size_t n, size_t ntiles, size_t n_events) {
   const size_t words = (size_t)((ndim + 1 + 3) / 4);
   ws.reused = false;
+  ws.ask_n = std::max(ws.ask_n, n);
+  ws.ask_tiles = std::max(ws.ask_tiles, ntiles);
+  ws.ask_words = std::max(ws.ask_words, words);
+  ws.ask_events = std::max(ws.ask_events, n_events);
   if (n <= ws.cap_n && ntiles <= ws.cap_tiles && words <= ws.cap_words && n_events <= ws.cap_events && ws.arena)
     return CLUE_OK;
-  n = std::max(n, ws.cap_n);
-  ntiles = std::max(ntiles, ws.cap_tiles);
-  n_events = std::max(n_events, ws.cap_events);
-  const size_t w = std::max(words, ws.cap_words);
+  // (not max with the capacities: those of an idle context are another program part's, and the product
+  // of its record words and this one's points would be memory that nobody asked for)
+  n = ws.ask_n;
+  ntiles = ws.ask_tiles;
+  n_events = ws.ask_events;
+  const size_t w = ws.ask_words;
   Workspace nw = ws;
   void* evtab = nullptr;
   const std::vector<ArenaItem> items = arena_items(nw, &evtab, n, ntiles, n_events, w);
@@ -217,6 +223,7 @@ clue_status workspace_reserve(Workspace& ws, int ndim, size_t n, size_t ntiles, 
     cudaGetLastError();
     cudaSetDevice(prev);
     ws.cap_n = ws.cap_tiles = ws.cap_words = ws.cap_events = 0;
+    ws.ask_n = ws.ask_tiles = ws.ask_words = ws.ask_events = 0;
     set_error(std::string("workspace allocation of ") + std::to_string(total) + " bytes failed: " +
               cudaGetErrorString(e));
     return CLUE_ERR_OUT_OF_MEMORY;
@@ -512,6 +519,7 @@ static bool idle_put(clue_context ctx) {
   ws.near_from_host = false;
   ws.timing = false;
   ws.launches = 0;
+  ws.ask_n = ws.ask_tiles = ws.ask_words = ws.ask_events = 0;
   ws.reused = true;
   clue_context drop = nullptr;
   {

@@ -108,6 +108,8 @@ struct Workspace {
   // current capacities
   size_t cap_n = 0, cap_tiles = 0, cap_words = 0;
   size_t cap_events = 0;
+  // the largest that the context's owner asked for (capacities may be an earlier owner's, see idle_put)
+  size_t ask_n = 0, ask_tiles = 0, ask_words = 0, ask_events = 0;
   void* arena = nullptr;
   size_t arena_bytes = 0;
 

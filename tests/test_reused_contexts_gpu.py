@@ -1,0 +1,53 @@
+"""Contexts made from an idle one (clue_context_destroy keeps small ones): what they hold, what they say
+of themselves and what a program can rely on is as with a new one."""
+import numpy as np
+import pytest
+
+from parity_util import gpu_args, random_blobs
+
+pytestmark = pytest.mark.gpu
+
+
+def _leave_idle(ndim, n):
+    """Leaves two idle contexts that ran n points of ndim dimensions."""
+    from cluestering_alpaka3_b200 import capi
+    c, w = random_blobs(np.random.default_rng(1), n, ndim, nblobs=max(4, n // 1000), extent=30.0 * max(1, n / 4000) ** 0.5)
+    ctxs = [capi.Context(0) for _ in range(2)]
+    for ctx in ctxs:
+        ctx.make_clusters_host(c, w, *gpu_args(dc=0.5, rhoc=2.0, dm=0.8))
+    for ctx in ctxs:
+        ctx.close()
+
+
+def _drop_idle():
+    """Takes the idle contexts and closes them too large to be kept."""
+    from cluestering_alpaka3_b200 import capi
+    ctxs = [capi.Context(0) for _ in range(2)]
+    for ctx in ctxs:
+        ctx.reserve(2, 3_000_000)
+    for ctx in ctxs:
+        ctx.close()
+
+
+@pytest.mark.parametrize("last,own", [((10, 3000), (2, 4_000_000)), ((2, 300_000), (10, 20_000))])
+@pytest.mark.parametrize("first", [0, 200])
+def test_larger_allocation_ignores_the_last_owner(last, own, first):
+    """An earlier owner's record words do not multiply a later one's points, nor its points their words."""
+    from cluestering_alpaka3_b200 import capi
+    c, w = random_blobs(np.random.default_rng(2), 200, 2, nblobs=2, extent=30.0)
+
+    def held():
+        ctx = capi.Context(0)
+        if first:  # a call that fits what is there
+            ctx.make_clusters_host(c, w, *gpu_args(dc=1.0, rhoc=2.0, dm=1.5))
+        ctx.reserve(*own)
+        b = ctx.workspace_bytes
+        ctx.close()
+        return b
+
+    _drop_idle()
+    new = held()
+    _drop_idle()
+    _leave_idle(*last)
+    assert held() <= new + (12 << 20)  # (staging buffers of the last owner, 9.6 MB, are not the workspace's)
+    _drop_idle()

@@ -556,6 +556,12 @@ static clue_context idle_take(int device) {
   return nullptr;
 }
 
+clue_context context_new(int32_t device) {
+  auto* c = new (std::nothrow) clue_context_s;
+  if (c) c->ws.device = device;
+  return c;
+}
+
 cudaError_t device_malloc(void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaErrorMemoryAllocation) return e;
@@ -835,9 +841,8 @@ clue_status clue_context_create(int32_t device, clue_context* ctx) {
     return CLUE_ERR_CUDA;
   }
   auto* c = idle_take(device);
-  if (!c) c = new (std::nothrow) clue_context_s;
+  if (!c) c = context_new(device);
   if (!c) return CLUE_ERR_OUT_OF_MEMORY;
-  c->ws.device = device;
   *ctx = c;
   return CLUE_OK;
 }

@@ -209,6 +209,10 @@ inline void stage_mark(Workspace& ws, int k, cudaStream_t s) {
 
 Workspace& context_workspace(clue_context ctx);
 
+// A context with no buffers, never an idle one: whose owner answers for the memory it holds (null:
+// out of memory).
+clue_context context_new(int32_t device);
+
 // Grows the post-processing temporaries to at least these sizes.
 clue_status post_reserve(Workspace& ws, size_t device_bytes, size_t host_bytes);
 

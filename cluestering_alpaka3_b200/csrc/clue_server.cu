@@ -112,9 +112,9 @@ void free_slot(Slot& s) {
 
 clue_status alloc_slot(clue_server_s* S, Slot& s) {
   const int nd = S->cfg.ndim;
-  clue_status st = clue_context_create(S->cfg.device, &s.ctx);
-  if (st != CLUE_OK) return st;
-  st = clue_context_reserve_batch(s.ctx, nd, S->cap_points, S->cap_tiles, S->cap_events);
+  s.ctx = context_new(S->cfg.device);  // (an idle one may hold more than the slot's budget)
+  if (!s.ctx) return CLUE_ERR_OUT_OF_MEMORY;
+  clue_status st = clue_context_reserve_batch(s.ctx, nd, S->cap_points, S->cap_tiles, S->cap_events);
   if (st != CLUE_OK) return st;
   CLUE_CUDA_TRY(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
   CLUE_CUDA_TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));

@@ -51,3 +51,23 @@ def test_larger_allocation_ignores_the_last_owner(last, own, first):
     _leave_idle(*last)
     assert held() <= new + (12 << 20)  # (staging buffers of the last owner, 9.6 MB, are not the workspace's)
     _drop_idle()
+
+
+def test_server_stays_inside_its_budget():
+    """Slots hold what was reserved for them, not a larger idle context's buffers."""
+    import torch
+    from cluestering_alpaka3_b200 import capi
+    _drop_idle()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    _leave_idle(2, 300_000)
+    budget = 24 << 20
+    cfg = capi.ServerConfig(ndim=2, n_slots=2, max_batch_events=16, max_event_points=20000, device_budget_bytes=budget)
+    srv = capi.Server(cfg, *gpu_args(dc=1.0, rhoc=2.0, dm=1.5))
+    try:
+        _drop_idle()  # those that the server did not take
+        held = free - torch.cuda.mem_get_info()[0]
+        assert srv.stats()["device_bytes"] <= budget
+        assert held <= budget + (24 << 20)  # (allocations of the driver, 2 MB each)
+    finally:
+        srv.close()

@@ -38,6 +38,7 @@ CLUE_DECLARE_DIM(9)
 CLUE_DECLARE_DIM(10)
 
 clue_status run_pipeline_dispatch(Workspace& ws, const RunArgs& a, cudaStream_t s) {
+  ws.reused = false;
   switch (a.ndim) {
     case 1: return run_pipeline<1>(ws, a, s);
     case 2: return run_pipeline<2>(ws, a, s);
@@ -192,7 +193,6 @@ static void wait_idle(Workspace& ws) {
 
 clue_status workspace_reserve(Workspace& ws, int ndim, size_t n, size_t ntiles, size_t n_events) {
   const size_t words = (size_t)((ndim + 1 + 3) / 4);
-  ws.reused = false;
   ws.ask_n = std::max(ws.ask_n, n);
   ws.ask_tiles = std::max(ws.ask_tiles, ntiles);
   ws.ask_words = std::max(ws.ask_words, words);
@@ -873,7 +873,10 @@ clue_status clue_context_reserve_batch(clue_context ctx, int32_t ndim, int64_t n
   return workspace_reserve(ctx->ws, ndim, (size_t)n_points, (size_t)n_tiles, (size_t)n_events);
 }
 
-size_t clue_context_workspace_bytes(clue_context ctx) { return ctx ? ctx->ws.arena_bytes + ctx->ws.dstage_bytes + ctx->ws.post_bytes : 0; }
+size_t clue_context_workspace_bytes(clue_context ctx) {
+  if (!ctx || ctx->ws.ask_n == 0) return 0;  // (an idle context's buffers before its owner's first call)
+  return ctx->ws.arena_bytes + ctx->ws.dstage_bytes + ctx->ws.post_bytes;
+}
 
 }  // extern "C"
 

@@ -71,3 +71,31 @@ def test_server_stays_inside_its_budget():
         assert held <= budget + (24 << 20)  # (allocations of the driver, 2 MB each)
     finally:
         srv.close()
+
+
+def test_no_status_and_no_bytes_before_a_call():
+    """The last owner's run is nobody's business, also after calls that are not runs."""
+    import torch
+    from cluestering_alpaka3_b200 import capi
+    _leave_idle(2, 3000)
+    ctx = capi.Context(0)
+    try:
+        assert ctx.workspace_bytes == 0
+        for call in ("none", "reserve", "get_clusters"):
+            if call == "reserve":
+                ctx.reserve(2, 100)
+                assert ctx.workspace_bytes > 0
+            elif call == "get_clusters":
+                lab = torch.zeros(64, dtype=torch.int32, device="cuda")
+                off, pts = torch.empty(65, dtype=torch.int32, device="cuda"), torch.empty_like(lab)
+                torch.cuda.synchronize()
+                assert ctx.get_clusters(lab.data_ptr(), 64, off.data_ptr(), pts.data_ptr()) == (1, 64)
+            with pytest.raises(capi.ClueError):
+                ctx.read_info()
+            with pytest.raises(capi.ClueError):
+                ctx.near_counts()
+        c, w = random_blobs(np.random.default_rng(2), 200, 2, nblobs=2, extent=30.0)
+        got = ctx.make_clusters_host(c, w, *gpu_args(dc=1.0, rhoc=2.0, dm=1.5))
+        assert ctx.read_info().n_clusters == got.info.n_clusters
+    finally:
+        ctx.close()

@@ -1,4 +1,5 @@
 // clue_capi.cu -- the extern "C" entry points of libclue_b200.so (include/clue_b200.h).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -191,6 +192,21 @@ static void wait_idle(Workspace& ws) {
   if (ws.busy) cudaDeviceSynchronize();
 }
 
+// The number of the current device's primary context, another one after every reset of the device
+// (which ends the buffers, streams and graphs of all contexts); 0: unknown.
+static unsigned long long device_life() {
+  using GetId = CUresult (*)(CUcontext, unsigned long long*);
+  static const GetId get_id = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found{};
+    const cudaError_t e = cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &found);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<GetId>(f) : nullptr;
+  }();
+  unsigned long long id = 0;
+  return get_id && get_id(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 clue_status workspace_reserve(Workspace& ws, int ndim, size_t n, size_t ntiles, size_t n_events) {
   const size_t words = (size_t)((ndim + 1 + 3) / 4);
   ws.ask_n = std::max(ws.ask_n, n);
@@ -237,6 +253,7 @@ clue_status workspace_reserve(Workspace& ws, int ndim, size_t n, size_t ntiles, 
   event_table_carve(evtab, n_events, &nw.ev, &nw.ev_pt, &nw.ev_tile);
   nw.arena = arena;
   nw.arena_bytes = total;
+  nw.life = device_life();
   nw.cap_n = n;
   nw.cap_tiles = ntiles;
   nw.cap_words = w;
@@ -504,6 +521,12 @@ static bool idle_put(clue_context ctx) {
   if (!ws.arena || ws.busy || ctx->alt || ws.arena_bytes + ws.dstage_bytes + ws.post_bytes > kIdleBytes ||
       ws.pipe_pinned)
     return false;
+  int prev = 0;
+  cudaGetDevice(&prev);
+  cudaSetDevice(ws.device);
+  const bool alive = ws.life != 0 && ws.life == device_life();
+  cudaSetDevice(prev);
+  if (!alive) return false;
   for (auto& t : ws.tev)
     if (t) cudaEventDestroy(t);
   // as a new context, with the buffers, streams, events and executable graphs
@@ -535,25 +558,54 @@ static bool idle_put(clue_context ctx) {
         }
     idle.list.push_back(ctx);
   }
-  if (drop) context_free(drop);
+  if (drop) {
+    if (drop->ws.life == ws.life)
+      context_free(drop);
+    else
+      delete drop;  // (from before a reset of the device)
+  }
   return true;
 }
 
-// The most recent idle context of the device, or null.
+// The most recent idle context of the device, or null.  Contexts from before a reset of the device
+// have lost their buffers and are forgotten: their addresses may be the program's by now.
 static clue_context idle_take(int device) {
+  int prev = 0;
+  cudaGetDevice(&prev);
+  cudaSetDevice(device);
+  const unsigned long long life = device_life();
+  cudaSetDevice(prev);
   IdleContexts& idle = idle_contexts();
   std::lock_guard<std::mutex> lock(idle.mutex);
   for (size_t k = idle.list.size(); k-- > 0;) {
     clue_context c = idle.list[k];
     if (c->ws.device != device) continue;
     idle.list.erase(idle.list.begin() + (ptrdiff_t)k);
-    // a device reset by the program took its buffers along: forget it
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, c->ws.arena) == cudaSuccess && at.type == cudaMemoryTypeDevice) return c;
-    cudaGetLastError();
+    if (c->ws.life == life) return c;
     delete c;
   }
   return nullptr;
+}
+
+// Frees all idle contexts; whether there was one.
+static bool idle_release() {
+  std::vector<clue_context_s*> all;
+  {
+    IdleContexts& idle = idle_contexts();
+    std::lock_guard<std::mutex> lock(idle.mutex);
+    all.swap(idle.list);
+  }
+  int prev = 0;
+  cudaGetDevice(&prev);
+  for (auto* c : all) {
+    cudaSetDevice(c->ws.device);
+    if (c->ws.life == device_life())
+      context_free(c);
+    else
+      delete c;  // as in idle_take
+  }
+  if (!all.empty()) cudaSetDevice(prev);
+  return !all.empty();
 }
 
 clue_context context_new(int32_t device) {
@@ -565,16 +617,8 @@ clue_context context_new(int32_t device) {
 cudaError_t device_malloc(void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaErrorMemoryAllocation) return e;
-  std::vector<clue_context_s*> all;
-  {
-    IdleContexts& idle = idle_contexts();
-    std::lock_guard<std::mutex> lock(idle.mutex);
-    all.swap(idle.list);
-  }
-  if (all.empty()) return e;
   cudaGetLastError();
-  for (auto* c : all) context_free(c);
-  return cudaMalloc(p, bytes);
+  return idle_release() ? cudaMalloc(p, bytes) : e;
 }
 }  // namespace clue_b200
 

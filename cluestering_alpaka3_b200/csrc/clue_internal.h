@@ -104,6 +104,7 @@ cudaError_t device_malloc(void** p, size_t bytes);
 struct Workspace {
   int device = 0;
   bool reused = false;  // buffers (and a status) of an idle context, no run of this one yet
+  unsigned long long life = 0;  // of the device when the arena was allocated (device_life)
   bool busy = false;    // work may be in flight: set by every call, cleared by one that waited for its end
   // current capacities
   size_t cap_n = 0, cap_tiles = 0, cap_words = 0;

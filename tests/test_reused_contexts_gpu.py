@@ -99,3 +99,58 @@ def test_no_status_and_no_bytes_before_a_call():
         assert ctx.read_info().n_clusters == got.info.n_clusters
     finally:
         ctx.close()
+
+
+RESET = r'''
+import ctypes, sys
+import numpy as np
+sys.path[:0] = [ROOT, ROOT + "/tests"]
+from cluestering_alpaka3_b200 import capi
+from parity_util import gpu_args, random_blobs
+c, w = random_blobs(np.random.default_rng(1), 3000, 2, nblobs=4, extent=30.0)
+args = gpu_args(dc=1.0, rhoc=2.0, dm=1.5)
+vp, n = ctypes.c_void_p, 8 << 20
+first = capi.Context(0)
+want = first.make_clusters_host(c, w, *args)
+second = capi.Context(0)
+second.make_clusters_host(c, w, *args)
+first.close()
+second.close()
+assert ctypes.CDLL("libcuda.so.1").cuDevicePrimaryCtxReset_v2(0) == 0  # what cudaDeviceReset does
+# the program's own memory, perhaps where the contexts' was
+bufs, data = [], np.arange(n, dtype=np.uint8)
+for _ in range(6):
+    p = vp()
+    capi.check(capi.lib.clue_device_alloc(0, n, ctypes.byref(p)))
+    capi.check(capi.lib.clue_memcpy_htod(p, data.ctypes.data, n, None))
+    bufs.append(p)
+if WHAT == "failing allocation":  # gives the idle contexts back
+    p = vp()
+    assert capi.lib.clue_device_alloc(0, 1 << 45, ctypes.byref(p)) != 0
+for _ in range(3):
+    ctx = capi.Context(0)
+    got = ctx.make_clusters_host(c, w, *args)
+    assert np.array_equal(got.cluster_index, want.cluster_index)
+    assert np.array_equal(got.rho.view(np.uint32), want.rho.view(np.uint32))
+    ctx.close()
+back = np.empty_like(data)
+for p in bufs:
+    capi.check(capi.lib.clue_memcpy_dtoh(back.ctypes.data, p, n, None))
+    capi.check(capi.lib.clue_stream_synchronize(None))
+    assert np.array_equal(back, data)
+    capi.check(capi.lib.clue_device_free(p))
+print("ok")
+'''
+
+
+@pytest.mark.parametrize("what", ["create", "failing allocation"])
+def test_device_reset_forgets_idle_contexts(what):
+    """A program that resets its device between contexts (in a child process: the reset ends all that
+    the process has on the device)."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", f"ROOT = {root!r}\nWHAT = {what!r}\n" + RESET], capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr

@@ -46,7 +46,7 @@ EXPORTED = [
     "clue_server_create", "clue_server_destroy", "clue_server_submit", "clue_server_wait",
     "clue_server_stats_read", "clue_server_replay", "clue_tuning_defaults", "clue_context_set_tuning",
     "clue_context_get_tuning", "clue_autotune_batch", "clue_silhouette", "clue_context_read_near_counts",
-    "clue_cluster_centroids",
+    "clue_cluster_centroids", "clue_idle_contexts_release",
 ]
 
 
@@ -150,6 +150,7 @@ def _load() -> ctypes.CDLL:
         "clue_stream_synchronize": ([vp], ctypes.c_int),
         "clue_context_create": ([i32, ctypes.POINTER(vp)], ctypes.c_int),
         "clue_context_destroy": ([vp], ctypes.c_int),
+        "clue_idle_contexts_release": ([], ctypes.c_int),
         "clue_context_reserve": ([vp, i32, i32, i32], ctypes.c_int),
         "clue_context_workspace_bytes": ([vp], sz),
         "clue_make_clusters": ([vp, ctypes.POINTER(_Params), ctypes.POINTER(_Kernel),
@@ -330,6 +331,12 @@ def device_count() -> int:
     c = ctypes.c_int32()
     st = lib.clue_device_count(ctypes.byref(c))
     return c.value if st == OK else 0
+
+
+def release_idle_contexts() -> None:
+    """Gives back the memory of the closed contexts that are kept for the next ones (at most two per
+    GPU, 64 MiB each)."""
+    check(lib.clue_idle_contexts_release())
 
 
 class Context:

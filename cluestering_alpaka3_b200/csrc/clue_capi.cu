@@ -501,8 +501,9 @@ static void context_free(clue_context ctx) {
 // Destroyed contexts kept for the next clue_context_create on their device: a program that makes a
 // Clusterer (or a Python clusterer) per table paid for the workspace, pinned buffers, stream and
 // executable graph of a new context on every call (4.0 ms of a 2000-point Python call, 0.28 ms with a
-// kept one).  At most kIdleContexts per device, each holding at most kIdleBytes of device memory; all
-// are freed when an allocation of the library fails (device_malloc).
+// kept one).  At most kIdleContexts per device, each holding at most kIdleBytes of device and pinned
+// memory; all are freed by clue_idle_contexts_release and when an allocation of the library fails
+// (device_malloc).
 constexpr size_t kIdleContexts = 2;
 constexpr size_t kIdleBytes = 64u << 20;
 struct IdleContexts {
@@ -518,8 +519,8 @@ static IdleContexts& idle_contexts() {
 static bool idle_put(clue_context ctx) {
   Workspace& ws = ctx->ws;
   // (nothing of this context may be in flight when its buffers get their next owner)
-  if (!ws.arena || ws.busy || ctx->alt || ws.arena_bytes + ws.dstage_bytes + ws.post_bytes > kIdleBytes ||
-      ws.pipe_pinned)
+  const size_t held = ws.arena_bytes + ws.dstage_bytes + ws.post_bytes + ws.pinned_bytes + ws.post_host_bytes;
+  if (!ws.arena || ws.busy || ctx->alt || ws.pipe_pinned || held > kIdleBytes)
     return false;
   int prev = 0;
   cudaGetDevice(&prev);
@@ -894,6 +895,11 @@ clue_status clue_context_create(int32_t device, clue_context* ctx) {
 clue_status clue_context_destroy(clue_context ctx) {
   if (!ctx) return CLUE_OK;
   if (!idle_put(ctx)) context_free(ctx);
+  return CLUE_OK;
+}
+
+clue_status clue_idle_contexts_release(void) {
+  idle_release();
   return CLUE_OK;
 }
 

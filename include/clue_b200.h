@@ -188,14 +188,21 @@ clue_status clue_stream_synchronize(void* stream);
  * label buffers) on one device; buffers only grow.  Not thread-safe: one caller
  * at a time, like a reference Clusterer. */
 clue_status clue_context_create(int32_t device, clue_context* ctx);
+/* A small context that no call is in flight on is kept for the next clue_context_create on its
+ * device, which finds its buffers, stream and graphs but none of its settings: at most two per
+ * device, each of at most 64 MiB of device and pinned memory.  They are given back by
+ * clue_idle_contexts_release, or when an allocation of this library fails; an allocator of the
+ * program's own does not see them. */
 clue_status clue_context_destroy(clue_context ctx);
+/* Frees what clue_context_destroy has kept, on every device. */
+clue_status clue_idle_contexts_release(void);
 /* Pre-size the workspace for up to n points of ndim dimensions (optional). */
 clue_status clue_context_reserve(clue_context ctx, int32_t ndim, int32_t n, int32_t points_per_tile);
-/* Bytes of device workspace the context currently holds. */
 /* Pre-sizes the workspace for batched calls of up to n_points points, n_tiles tiles (the sum of
  * the events' reference grids) and n_events events, so that such calls allocate nothing. */
 clue_status clue_context_reserve_batch(clue_context ctx, int32_t ndim, int64_t n_points, int64_t n_tiles,
                                        int32_t n_events);
+/* Bytes of device workspace the context currently holds (0 before its first call). */
 size_t clue_context_workspace_bytes(clue_context ctx);
 
 /*

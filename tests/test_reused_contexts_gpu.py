@@ -154,3 +154,21 @@ def test_device_reset_forgets_idle_contexts(what):
     r = subprocess.run([sys.executable, "-c", f"ROOT = {root!r}\nWHAT = {what!r}\n" + RESET], capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
+def test_release_gives_the_memory_back():
+    import torch
+    from cluestering_alpaka3_b200 import capi
+    _leave_idle(2, 3000)  # (kernels loaded, streams made)
+    capi.release_idle_contexts()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    _leave_idle(2, 300_000)
+    assert free - torch.cuda.mem_get_info()[0] > 60 << 20
+    capi.release_idle_contexts()
+    capi.release_idle_contexts()  # nothing left
+    assert free - torch.cuda.mem_get_info()[0] < 8 << 20
+    ctx = capi.Context(0)
+    c, w = random_blobs(np.random.default_rng(2), 200, 2, nblobs=2, extent=30.0)
+    ctx.make_clusters_host(c, w, *gpu_args(dc=1.0, rhoc=2.0, dm=1.5))
+    ctx.close()

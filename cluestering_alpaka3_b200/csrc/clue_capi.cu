@@ -506,13 +506,38 @@ static void context_free(clue_context ctx) {
 // (device_malloc).
 constexpr size_t kIdleContexts = 2;
 constexpr size_t kIdleBytes = 64u << 20;
+constexpr size_t kIdleDevices = 64;
+// Nothing here allocates, so the entry points that use it throw nothing.  (The contexts are not freed
+// at exit: the driver may be gone by then.)
 struct IdleContexts {
   std::mutex mutex;
-  std::vector<clue_context_s*> list;  // oldest first
+  clue_context list[kIdleContexts * kIdleDevices];  // oldest first
+  size_t count;
+
+  void remove(size_t k) {
+    std::copy(list + k + 1, list + count, list + k);
+    --count;
+  }
 };
-static IdleContexts& idle_contexts() {
-  static IdleContexts* p = new IdleContexts;  // (not destroyed: the driver may be gone at exit)
-  return *p;
+static IdleContexts g_idle;
+
+// Whether the device still is in the life that the context's buffers belong to.
+static bool idle_alive(clue_context c) {
+  int prev = 0;
+  cudaGetDevice(&prev);
+  cudaSetDevice(c->ws.device);
+  const unsigned long long life = device_life();
+  cudaSetDevice(prev);
+  return life != 0 && life == c->ws.life;
+}
+
+// Frees an idle context.  One from before a reset of the device has lost its buffers and is forgotten:
+// their addresses may be the program's by now.
+static void idle_free(clue_context c) {
+  if (idle_alive(c))
+    context_free(c);
+  else
+    delete c;
 }
 
 // Keeps ctx if it is small; false: the caller frees it.
@@ -522,12 +547,7 @@ static bool idle_put(clue_context ctx) {
   const size_t held = ws.arena_bytes + ws.dstage_bytes + ws.post_bytes + ws.pinned_bytes + ws.post_host_bytes;
   if (!ws.arena || ws.busy || ctx->alt || ws.pipe_pinned || held > kIdleBytes)
     return false;
-  int prev = 0;
-  cudaGetDevice(&prev);
-  cudaSetDevice(ws.device);
-  const bool alive = ws.life != 0 && ws.life == device_life();
-  cudaSetDevice(prev);
-  if (!alive) return false;
+  if (!idle_alive(ctx)) return false;
   for (auto& t : ws.tev)
     if (t) cudaEventDestroy(t);
   // as a new context, with the buffers, streams, events and executable graphs
@@ -547,66 +567,52 @@ static bool idle_put(clue_context ctx) {
   ws.reused = true;
   clue_context drop = nullptr;
   {
-    IdleContexts& idle = idle_contexts();
-    std::lock_guard<std::mutex> lock(idle.mutex);
-    size_t same = 0;
-    for (auto* c : idle.list) same += c->ws.device == ws.device;
-    if (same >= kIdleContexts)
-      for (size_t k = 0; k < idle.list.size() && !drop; ++k)
-        if (idle.list[k]->ws.device == ws.device) {
-          drop = idle.list[k];
-          idle.list.erase(idle.list.begin() + (ptrdiff_t)k);
-        }
-    idle.list.push_back(ctx);
+    std::lock_guard<std::mutex> lock(g_idle.mutex);
+    size_t same = 0, oldest = 0;
+    for (size_t k = g_idle.count; k-- > 0;)
+      if (g_idle.list[k]->ws.device == ws.device) {
+        ++same;
+        oldest = k;
+      }
+    if (same >= kIdleContexts || g_idle.count == kIdleContexts * kIdleDevices) {
+      drop = g_idle.list[oldest];
+      g_idle.remove(oldest);
+    }
+    g_idle.list[g_idle.count++] = ctx;
   }
-  if (drop) {
-    if (drop->ws.life == ws.life)
-      context_free(drop);
-    else
-      delete drop;  // (from before a reset of the device)
-  }
+  if (drop) idle_free(drop);
   return true;
 }
 
-// The most recent idle context of the device, or null.  Contexts from before a reset of the device
-// have lost their buffers and are forgotten: their addresses may be the program's by now.
+// The most recent idle context of the device, or null (contexts from before a reset are forgotten).
 static clue_context idle_take(int device) {
-  int prev = 0;
-  cudaGetDevice(&prev);
-  cudaSetDevice(device);
-  const unsigned long long life = device_life();
-  cudaSetDevice(prev);
-  IdleContexts& idle = idle_contexts();
-  std::lock_guard<std::mutex> lock(idle.mutex);
-  for (size_t k = idle.list.size(); k-- > 0;) {
-    clue_context c = idle.list[k];
-    if (c->ws.device != device) continue;
-    idle.list.erase(idle.list.begin() + (ptrdiff_t)k);
-    if (c->ws.life == life) return c;
+  for (;;) {
+    clue_context c = nullptr;
+    {
+      std::lock_guard<std::mutex> lock(g_idle.mutex);
+      for (size_t k = g_idle.count; k-- > 0 && !c;)
+        if (g_idle.list[k]->ws.device == device) {
+          c = g_idle.list[k];
+          g_idle.remove(k);
+        }
+    }
+    if (!c || idle_alive(c)) return c;
     delete c;
   }
-  return nullptr;
 }
 
 // Frees all idle contexts; whether there was one.
 static bool idle_release() {
-  std::vector<clue_context_s*> all;
+  clue_context all[kIdleContexts * kIdleDevices];
+  size_t count = 0;
   {
-    IdleContexts& idle = idle_contexts();
-    std::lock_guard<std::mutex> lock(idle.mutex);
-    all.swap(idle.list);
+    std::lock_guard<std::mutex> lock(g_idle.mutex);
+    count = g_idle.count;
+    std::copy(g_idle.list, g_idle.list + count, all);
+    g_idle.count = 0;
   }
-  int prev = 0;
-  cudaGetDevice(&prev);
-  for (auto* c : all) {
-    cudaSetDevice(c->ws.device);
-    if (c->ws.life == device_life())
-      context_free(c);
-    else
-      delete c;  // as in idle_take
-  }
-  if (!all.empty()) cudaSetDevice(prev);
-  return !all.empty();
+  for (size_t k = 0; k < count; ++k) idle_free(all[k]);
+  return count > 0;
 }
 
 clue_context context_new(int32_t device) {

@@ -127,7 +127,6 @@ enum : uint32_t {
   kChkFinalizeNh = 5,    // k_nearest_higher: a nearest higher
   kChkDensityTile = 6,   // k_density_sym: a tile of the search box
   kChkDensityMirror = 7, // k_density_sym: the mirrored term's point
-  kChkBuildCluster = 8,  // k_build: the cluster's size (in every build)
 };
 inline const char* check_site_name(uint32_t site) {
   switch (site) {
@@ -137,7 +136,6 @@ inline const char* check_site_name(uint32_t site) {
     case kChkFinalizeRoot: return "labels (root)";
     case kChkFinalizeNh: return "outputs (nearest higher)";
     case kChkDensityTile: return "symmetric density (search-box tile)";
-    case kChkBuildCluster: return "build (cluster size)";
     case kChkDensityMirror: return "symmetric density (mirrored point)";
   }
   return "unknown";

@@ -27,6 +27,10 @@
 // of the warp's homes; the spatial sweeps take one 32-record Morton block at a time, skip blocks
 // whose bounding box is out of reach, and read the candidates from shared memory (nearest higher)
 // or from their owner lanes by shuffle (symmetric density).
+#include <atomic>
+#include <cstdlib>
+#include <cstring>
+
 #include "clue_internal.h"
 
 #ifndef CLUE_NDIM
@@ -1045,19 +1049,12 @@ struct BuildBufs {
   DevStatus* st;
 };
 
+// Event e by one cluster of `ranks` CTAs.
 template <int N, int W>
-__global__ void __launch_bounds__(32 * W) k_build(const KParams kp, InPtrs in, EvGrid* eg, BuildBufs o, bool two,
-                                                  int mbits, int tile_passes, int passes, int want_ranks) {
-  __shared__ BuildSmem<N, W> sm;
-  uint32_t rank, ranks;
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
-  if ((int)ranks != want_ranks) {  // not the launch that was asked for: nothing is touched
-    if (blockIdx.x == 0 && threadIdx.x == 0) o.st->check_site = kChkBuildCluster, o.st->check_index = (int)ranks;
-    return;
-  }
+__device__ __forceinline__ void build_event(BuildSmem<N, W>& sm, const KParams& kp, const InPtrs& in, EvGrid* eg,
+                                            const BuildBufs& o, bool two, int mbits, int tile_passes, int passes, int e,
+                                            uint32_t rank, uint32_t ranks) {
   const int lane = lane_id(), warp = threadIdx.x >> 5;
-  const int e = blockIdx.x / ranks;
   EvGrid* g = eg + e;
   const bool single = kp.n_events == 1;
   const int n = single ? kp.n : g->pt_count, pt = single ? 0 : g->pt_base;
@@ -1271,6 +1268,22 @@ __global__ void __launch_bounds__(32 * W) k_build(const KParams kp, InPtrs in, E
     write_block_box<N>(o.tblk, (int)__ldcg(o.tblk_off + t) + b, x, w);
   }
   cluster_barrier();  // sm.scan[0] of the first CTA is read by all
+}
+
+// An event per cluster.  The clusters of a launch share its events by the sizes that the hardware
+// reports, whatever was asked for (an executable graph updated in place has kept an older launch's).
+template <int N, int W>
+__global__ void __launch_bounds__(32 * W) k_build(const KParams kp, InPtrs in, EvGrid* eg, BuildBufs o, bool two,
+                                                  int mbits, int tile_passes, int passes) {
+  __shared__ BuildSmem<N, W> sm;
+  uint32_t rank, ranks;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+  const int clusters = gridDim.x / ranks;
+  for (int e = blockIdx.x / ranks; e < kp.n_events; e += clusters) {
+    build_event<N, W>(sm, kp, in, eg, o, two, mbits, tile_passes, passes, e, rank, ranks);
+    if (e + clusters < kp.n_events) cluster_barrier();  // the next event takes the same shared memory
+  }
 }
 
 // ---- chunks ---------------------------------------------------------------------
@@ -2588,32 +2601,96 @@ inline int build_ranks(int n_events, int n) {
   return n_events <= 64 ? 8 : (n_events <= 128 ? 4 : (n_events <= 256 ? 2 : 1));
 }
 
+#if CLUE_DEVICE_CHECKS
+// The checked build can be told to find a device's limits: CLUE_BUILD_CLUSTERS = "fit N" (no clusters
+// above N CTAs, 0: none), "refuse" (launches fail), "half", "double" (clusters of another size than
+// asked for).
+inline const char* build_clusters_env() {
+  const char* v = getenv("CLUE_BUILD_CLUSTERS");
+  return v ? v : "";
+}
+inline bool build_cluster_allowed(int ranks) {
+  const char* v = build_clusters_env();
+  return strncmp(v, "fit ", 4) != 0 || ranks <= atoi(v + 4);
+}
+inline cudaError_t build_launch_fault(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr) {
+  const char* v = build_clusters_env();
+  if (!strcmp(v, "refuse")) return cudaErrorInvalidConfiguration;
+  unsigned& c = attr.val.clusterDim.x;
+  if (!strcmp(v, "half")) c = std::max(1u, c / 2);
+  if (!strcmp(v, "double")) c = std::min(8u, c * 2);
+  cfg.gridDim.x = (cfg.gridDim.x + c - 1) / c * c;
+  return cudaSuccess;
+}
+#else
+inline bool build_cluster_allowed(int) { return true; }
+inline cudaError_t build_launch_fault(cudaLaunchConfig_t&, cudaLaunchAttribute&) { return cudaSuccess; }
+#endif
+
+// The launch of k_build with clusters of `ranks` CTAs.
 template <int N, int W>
-void launch_build_cluster(const KParams& kp, const InPtrs& in, EvGrid* eg, const BuildBufs& o, bool two, int mbits,
-                          int tile_passes, int passes, int ranks, cudaStream_t s) {
+struct BuildLaunch {
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)ranks;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(kp.n_events * ranks));
-  cfg.blockDim = dim3(32 * W);
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (ranks > 8) cudaFuncSetAttribute(k_build<N, W>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaLaunchKernelEx(&cfg, k_build<N, W>, kp, in, eg, o, two, mbits, tile_passes, passes, ranks);
+  BuildLaunch(int n_events, int ranks, cudaStream_t s) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ranks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(n_events * ranks));
+    cfg.blockDim = dim3(32 * W);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+};
+
+// Whether the current device can hold a cluster of `ranks` CTAs (a partitioned one may not); asked once
+// per device and size.
+template <int N, int W>
+bool build_cluster_fits(int ranks) {
+  constexpr int kDevices = 64;
+  static std::atomic<uint32_t> known[kDevices];  // bit ranks: fits, bit 31 - ranks / 2: asked
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const uint32_t fits = 1u << ranks, asked = 1u << (31 - ranks / 2);
+  if (dev < kDevices) {
+    const uint32_t k = known[dev].load(std::memory_order_relaxed);
+    if (k & asked) return k & fits;
+  }
+  BuildLaunch<N, W> l(1, ranks, nullptr);
+  int count = 0;
+  cudaError_t e = cudaSuccess;
+  if (ranks > 8) e = cudaFuncSetAttribute(k_build<N, W>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&count, k_build<N, W>, &l.cfg);
+  if (e != cudaSuccess) cudaGetLastError();
+  const bool ok = build_cluster_allowed(ranks) && e == cudaSuccess && count > 0;
+  if (dev < kDevices) known[dev].fetch_or(asked | (ok ? fits : 0u), std::memory_order_relaxed);
+  return ok;
 }
 
-// Stage 1 through k_build; returns the launches.
+template <int N, int W>
+cudaError_t launch_build_cluster(const KParams& kp, const InPtrs& in, EvGrid* eg, const BuildBufs& o, bool two,
+                                 int mbits, int tile_passes, int passes, int ranks, cudaStream_t s) {
+  BuildLaunch<N, W> l(kp.n_events, ranks, s);
+  cudaError_t e = build_launch_fault(l.cfg, l.attr[0]);
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&l.cfg, k_build<N, W>, kp, in, eg, o, two, mbits, tile_passes, passes);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
+// Stage 1 through k_build with the largest clusters up to build_ranks that the device holds; returns
+// the launches, 0 if there was none: the separate launches then take its place.
 template <int N>
 int launch_build(const KParams& kp, const InPtrs& in, Workspace& ws, bool two, int mbits, int tile_bits,
                  cudaStream_t s) {
   const int passes = (tile_bits + mbits + kRadixBits - 1) / kRadixBits;
   const int tile_passes = std::max(1, (tile_bits + kRadixBits - 1) / kRadixBits);
   const bool odd = passes & 1;
-  const int ranks = build_ranks(kp.n_events, kp.n);
+  const bool single = kp.n_events == 1;
+  int ranks = build_ranks(kp.n_events, kp.n);
+  while (ranks > 0 && !(single ? build_cluster_fits<N, 32>(ranks) : build_cluster_fits<N, 16>(ranks))) ranks /= 2;
   ws.build_ranks = ranks;
+  if (ranks == 0) return 0;
   BuildBufs o{};
   o.k0 = ws.keys[0];
   o.k1 = ws.keys[1];
@@ -2638,14 +2715,17 @@ int launch_build(const KParams& kp, const InPtrs& in, Workspace& ws, bool two, i
   o.st = ws.status;
   ws.perm = two ? ws.mq_alt : (odd ? ws.vals[0] : ws.vals[1]);
   ws.mq = two ? (odd ? ws.vals[1] : ws.vals[0]) : nullptr;
-  if (kp.n_events > 1) {
+  if (!single)
     k_init<N><<<grid_for(std::max(kp.n_events, kp.n / 128), 256), 256, 0, s>>>(kp, events_of(ws), ws.ev_pt, ws.ev_tile,
                                                                                ws.seed_bits, ws.chunk_total, ws.status);
-    launch_build_cluster<N, 16>(kp, in, ws.ev, o, two, mbits, tile_passes, passes, ranks, s);
-    return 2;
+  const cudaError_t e =
+      single ? launch_build_cluster<N, 32>(kp, in, ws.ev, o, two, mbits, tile_passes, passes, ranks, s)
+             : launch_build_cluster<N, 16>(kp, in, ws.ev, o, two, mbits, tile_passes, passes, ranks, s);
+  if (e != cudaSuccess) {
+    ws.build_ranks = 0;
+    return 0;
   }
-  launch_build_cluster<N, 32>(kp, in, ws.ev, o, two, mbits, tile_passes, passes, ranks, s);
-  return 1;
+  return single ? 1 : 2;
 }
 
 #define CLUE_METRIC_SWITCH(mt, FN, ...)                                           \
@@ -2697,12 +2777,12 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
   const int max_slots = kChunkWarps * (n / kChunk + kp.ntiles + 1);
   const int pts_max = kp.n_events == 1 ? n : a.max_points;
   const int ev_bits = bits_for((uint32_t)((kp.n_events == 1 ? kp.ntiles : a.max_tiles) - 1));
-  bool composite = false;
-  if (build_takes(kp, pts_max, ev_bits, mbits)) {
-    composite = symmetric;
-    launches += launch_build<N>(kp, in, ws, !symmetric, mbits, ev_bits, s);
-  } else {
-    ws.build_ranks = 0;
+  bool composite = symmetric;
+  ws.build_ranks = 0;
+  const int built =
+      build_takes(kp, pts_max, ev_bits, mbits) ? launch_build<N>(kp, in, ws, !symmetric, mbits, ev_bits, s) : 0;
+  launches += built;
+  if (built == 0) {
     launches += 4;  // init, bbox, grid, bin
     k_init<N><<<grid_for(std::max(kp.n_events, n / 128), 256), 256, 0, s>>>(kp, ev, ws.ev_pt, ws.ev_tile, ws.seed_bits,
                                                                             nullptr, ws.status);

@@ -2582,13 +2582,30 @@ void launch_near_ties(const KParams& kp, Workspace& ws, cudaStream_t s) {
 // points 134 against 180 us, 40k 173 / 233, 65k 183 / 233, 131k 261 / 283 (a 3-D one with the symmetric
 // density 293 / 304); 24 events of 3300 4-D points 167 / 246, 64 events 269 / 318, 100 2-D events of
 // 3300 points 293 / 333, 300 events 798 / 756.
+// Many events: a CTA of 512 threads takes one through all passes, however small, so the stage grows
+// with the events beside the points.  2-D batches, exponential kernel: 1000 events of 10 points 203 against
+// 259 us, 2500 361 / 354; 1500 of 100 points 269 / 277, 2500 385 / 349; 1500 of 250 points 356 / 358, 2000
+// 435 / 423 (100000 events of 5 points: 11.5 against 6.5 ms).
+// Many tiles: one CTA scans all tiles of an event and a batch's unused slots are launched, which the
+// separate launches of the symmetric density (one sort) do not make up for beyond a line in points and
+// tiles.  Single events: 16k points and 8192 tiles 203 / 223 us, 16384 tiles 261 / 249; 65k and 5461 202 /
+// 210, 8192 238 / 228; 131k and 1024 203 / 201, 8192 287 / 249, 32768 592 / 396.  Batches: 8 events of 30000
+// points and 1875 tiles each 323 / 336, 3750 461 / 441, 7500 713 / 613; 50 of 10000 points and 625 tiles 459 /
+// 465, 1250 706 / 691, 2500 1105 / 1049; 24 of 3300 points and 1650 tiles 421 / 466.  The three sorts of the
+// other calls take more with as many tiles (131k points and 65536 tiles, tile stage: 226 / 291 us).
 constexpr int kBuildPoints = 131072;       // of a single event
 constexpr int kBuildBatchPoints = 1 << 19;  // of a batch, each event at most kBuildEventPoints
 constexpr int kBuildEventPoints = 32768;
+constexpr int kBuildEvents = 2304;         // events + points / 512 of a batch
 constexpr int kBuildTileBits = 16;
-inline bool build_takes(const KParams& kp, int max_points, int tile_bits, int mbits) {
+constexpr int kBuildSymTiles = 13000;      // symmetric density: tiles + points / 11 of a single event,
+constexpr int kBuildSymEventTiles = 2048;  // tiles of a batch's event and
+constexpr int kBuildSymBatchTiles = 49152;  // of a batch
+inline bool build_takes(const KParams& kp, int max_points, int max_tiles, int tile_bits, int mbits, bool symmetric) {
   if (tile_bits > kBuildTileBits || tile_bits + mbits > 32) return false;
-  if (kp.n_events == 1) return kp.n <= kBuildPoints;
+  if (kp.n_events == 1) return kp.n <= kBuildPoints && (!symmetric || kp.ntiles + kp.n / 11 <= kBuildSymTiles);
+  if (kp.n_events + kp.n / 512 > kBuildEvents) return false;
+  if (symmetric && (max_tiles > kBuildSymEventTiles || kp.ntiles > kBuildSymBatchTiles)) return false;
   // a batch's chunks and blocks have slots per event (k_build): they must fit the buffers
   return kp.n <= kBuildBatchPoints && max_points <= kBuildEventPoints && kp.n / 32 + kp.ntiles + 1 <= kp.n;
 }
@@ -2776,11 +2793,13 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
   const int nsb = (n + 1023) >> 10;
   const int max_slots = kChunkWarps * (n / kChunk + kp.ntiles + 1);
   const int pts_max = kp.n_events == 1 ? n : a.max_points;
-  const int ev_bits = bits_for((uint32_t)((kp.n_events == 1 ? kp.ntiles : a.max_tiles) - 1));
+  const int tiles_max = kp.n_events == 1 ? kp.ntiles : a.max_tiles;
+  const int ev_bits = bits_for((uint32_t)(tiles_max - 1));
   bool composite = symmetric;
   ws.build_ranks = 0;
-  const int built =
-      build_takes(kp, pts_max, ev_bits, mbits) ? launch_build<N>(kp, in, ws, !symmetric, mbits, ev_bits, s) : 0;
+  int built = 0;
+  if (build_takes(kp, pts_max, tiles_max, ev_bits, mbits, symmetric))
+    built = launch_build<N>(kp, in, ws, !symmetric, mbits, ev_bits, s);
   launches += built;
   if (built == 0) {
     launches += 4;  // init, bbox, grid, bin

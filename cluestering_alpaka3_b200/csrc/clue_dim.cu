@@ -1870,13 +1870,14 @@ struct PairSmem {
   static constexpr int kRows = (N + 2) / 2;
   static constexpr int kFloats = kRows * 64;
 };
-// All components of a pair at shared-memory address `a` (row 0's word).
+// All components of a pair at shared-memory address `a` (row 0's word); "memory", since ordinary stores
+// of the warp put them there.
 template <int N>
 __device__ __forceinline__ void load_pairs(uint32_t a, unsigned long long* c) {
 #pragma unroll
   for (int f = 0; f < (N + 1) / 2; ++f)
-    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(c[2 * f]), "=l"(c[2 * f + 1]) : "r"(a + 256u * f));
-  if constexpr ((N + 1) & 1) asm volatile("ld.shared.u64 %0, [%1];" : "=l"(c[N]) : "r"(a + 256u * (N / 2)));
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(c[2 * f]), "=l"(c[2 * f + 1]) : "r"(a + 256u * f) : "memory");
+  if constexpr ((N + 1) & 1) asm volatile("ld.shared.u64 %0, [%1];" : "=l"(c[N]) : "r"(a + 256u * (N / 2)) : "memory");
 }
 
 // VAR selects measured alternatives of the pair step (clue_tuning.density_gate / density_exp2):

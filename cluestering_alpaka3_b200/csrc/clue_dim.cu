@@ -1657,9 +1657,10 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
       unsigned om = __ballot_sync(0xffffffffu, ok);
       if (om == 0) continue;
       if (om & (om - 1)) {
-        // of several, those that a strictly denser one is not strictly nearer than
+        // Of several, those that a strictly denser one is not strictly nearer than.  (The metric value is
+        // negative for a negative weight: times slack would be nearer than itself.)
         const float near = warp_min_f(ok && r > rho_h ? s : INFINITY);
-        om = __ballot_sync(0xffffffffu, ok && s <= near * slack);
+        om = __ballot_sync(0xffffffffu, ok && s <= fmaxf(near, near * slack));
       }
       do {
         const int j = __ffs(om) - 1;

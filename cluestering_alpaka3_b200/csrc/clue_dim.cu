@@ -1493,6 +1493,42 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4)) k_density(
 // (or than dm) or holds no density reaching the lane's.  TIE == CLUE_TIE_RHO_INDEX resolves equal
 // distances by higher rho, then lower index.
 
+// The two functions below are for equal distances: points on a lattice, or of one place.  Calls and not
+// inlined, which keeps them out of the usual path's registers (4096-event batch 2.07 ms, 2.11 inlined).
+
+// Homes `nm` of a block that still need a search home by home.  Not those with nothing higher, all
+// densities being equal and the indices lower, nor those whose best so far is as near as the block's
+// nearest, of this tile and of a lower index than any: pos_best (else -1).  pos, rho: the lane's candidate,
+// pos_home, rho_home: the lane's home.  (16k points of one place: 0.85 ms, 13 without it.)
+__device__ __noinline__ unsigned tie_block(unsigned nm, int pos_best, const int32_t* perm, int pos, float rho,
+                                           float rho_home, int pos_home) {
+  const int orig = __ldg(perm + pos);
+  const int orig_min = warp_min_i(orig), orig_max = warp_max_i(orig);
+  const float rho_max = warp_max_f(rho);
+  bool skip = pos_best >= 0 && orig_min >= __ldg(perm + pos_best);
+  if (rho_max <= rho_home) skip = skip || orig_max <= __ldg(perm + pos_home);
+  return nm & ~__ballot_sync(0xffffffffu, skip);
+}
+
+// Of one home's candidates `om` (a lane each), the least by rounded distance, then by density (RHO_INDEX),
+// then by original index, which orders the points of a tile as the iteration rank does; 0 if none is
+// higher.
+template <int TIE>
+__device__ __noinline__ unsigned tie_least(unsigned om, float dist, float rho, float rho_home, const int32_t* perm,
+                                           int pos, int pos_home) {
+  const int lane = threadIdx.x & 31;
+  const int orig = __ldg(perm + pos), orig_home = __ldg(perm + pos_home);
+  const bool higher = ((om >> lane) & 1u) && (rho > rho_home || (rho > 0.0f && orig > orig_home));
+  const float dist_min = warp_min_f(higher ? dist : INFINITY);
+  bool least = higher && dist == dist_min;
+  if (TIE != CLUE_TIE_REFERENCE) {
+    const float rho_max = warp_max_f(least ? rho : -INFINITY);
+    least = least && rho == rho_max;
+  }
+  const int first = warp_min_i(least ? orig : INT_MAX);
+  return __ballot_sync(0xffffffffu, least && orig == first);
+}
+
 // A block is visited in one of two forms.  Where few lanes need it, it is taken home by home with
 // a candidate per lane: one distance per lane, one vote, and the few candidates that pass settle
 // the home's update.  Otherwise it is taken candidate by candidate with a home per lane, without
@@ -1636,7 +1672,7 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
         for (int d = 0; d < N; ++d) cj[d] = reinterpret_cast<const float*>(s_blk[warp][d])[j];
         const float s = M::partial(x, cj, kp.mpar);
         if ((k2 >> 5) - (k1 >> 5) <= 1u)
-          slow = true;
+          slow = __uint_as_float(k1 & ~31u) <= bnd;  // (the shortened value is not above the least)
         else if (s <= bnd) {
           if (reinterpret_cast<const float*>(s_blk[warp][N])[j] > rho_i && s * slack < s_best)
             take(j, s);
@@ -1645,6 +1681,12 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
         }
       }
       nm = __ballot_sync(0xffffffffu, slow);
+      if (nm) {
+        const bool tied = TIE == CLUE_TIE_REFERENCE && slow && nh >= 0 && rank == rank_best &&
+                          __uint_as_float(k1 & ~31u) >= s_best;
+        nm = tie_block(nm, tied ? order_at(mq, nh) : -1, perm, order_at(mq, lane < cnt ? p0 + lane : p0), r, rho_i,
+                       order_at(mq, h.p));
+      }
     }
     while (nm) {
       const int hl = __ffs(nm) - 1;
@@ -1662,17 +1704,19 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
         const float near = warp_min_f(ok && r > rho_h ? s : INFINITY);
         om = __ballot_sync(0xffffffffu, ok && s <= fmaxf(near, near * slack));
       }
-      do {
-        const int j = __ffs(om) - 1;
-        om &= om - 1;
-        const float sj = __shfl_sync(0xffffffffu, s, j), rj = __shfl_sync(0xffffffffu, r, j);
-        if (lane == hl) {
-          if (rj > rho_i && sj * slack < s_best)
-            take(j, sj);
-          else
-            consider(j, sj, rj);
-        }
-      } while (om);
+      if (om & (om - 1)) {  // still several
+        om = tie_least<TIE>(om, s < 0.0f ? s : M::finish(s), r, rho_h, perm, order_at(mq, lane < cnt ? p0 + lane : p0),
+                            order_at(mq, pw + hl));
+        if (om == 0) continue;
+      }
+      const int j = __ffs(om) - 1;
+      const float sj = __shfl_sync(0xffffffffu, s, j), rj = __shfl_sync(0xffffffffu, r, j);
+      if (lane == hl) {
+        if (rj > rho_i && sj * slack < s_best)
+          take(j, sj);
+        else
+          consider(j, sj, rj);
+      }
     }
   });
   // Seeds (KernelFindClusters) and every output but the label, while all of it is at hand.  d(i, nh)

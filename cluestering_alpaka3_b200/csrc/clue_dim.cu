@@ -2365,76 +2365,92 @@ constexpr int kSeedBlockPoints = 4096, kSeedBlocks = 64;
 
 // Pointer jumping on the forest: every parent pointer is replaced by its grandparent until it
 // names a root.  All writes move a pointer to an ancestor, so concurrent updates are safe.
-// At most `iters` jumps per point per launch; a launch that leaves a point unresolved records
-// it in st->unresolved[round] and the next launch continues.  With LABELS every point that
-// reaches its root gets its label.
+// With LABELS every point that reaches its root gets its label.
+// A thread makes up to `passes` passes over its chains, at most `hops` jumps a chain in each.  The grid
+// is one that the GPU holds at once (label_blocks), so the chains of all points move on together and a
+// pass finds the parents of the one before far ahead.  A chain climbed to its end at once goes point by
+// point through those whose threads have not begun: a ramp of 1M points took 16.2 ms with up to 4096 jumps
+// at once, 0.06 with 16 a pass (8: 0.06, 32: 0.17, 64: 0.42), one of 4M points 13 and 0.15 ms.  What is
+// unresolved after the last pass is recorded in st->unresolved[round] and left to the next launch.
+struct JumpLimits {
+  int hops, passes;
+};
 template <bool LABELS, int K>
 __device__ __forceinline__ void jump(int32_t* par, const int32_t* __restrict__ perm, int32_t* __restrict__ label,
-                                     int n, int iters, DevStatus* st, int round) {
-  bool unres = false;
+                                     int n, JumpLimits limits, DevStatus* st, int round) {
   const int stride = gridDim.x * blockDim.x;
-  // K chains per thread walked in lockstep: each step's parent loads are independent, so they are in
-  // flight together (the walk is bound by load latency, not bandwidth)
-  for (int64_t pos0 = blockIdx.x * blockDim.x + threadIdx.x; pos0 < n; pos0 += (int64_t)K * stride) {
-    int p[K], i[K];
-    bool act[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int64_t pos = pos0 + (int64_t)k * stride;
-      p[k] = pos < n ? par[pos] : -1;
-      if (LABELS) i[k] = pos < n ? perm[pos] : -1;
-      act[k] = p[k] >= 0;
-    }
-    for (int it = 0; it < iters; ++it) {
-      bool any = false;
+  uint32_t todo = ~0u;  // groups of K chains with an unresolved one (the last bit: of all from the 32nd on)
+  for (int pass = 0; pass < limits.passes && todo; ++pass) {
+    uint32_t left = 0, bit = 1u;
+    // K chains per thread walked in lockstep: each step's parent loads are independent, so they are in
+    // flight together (the walk is bound by load latency, not bandwidth)
+    for (int64_t pos0 = blockIdx.x * blockDim.x + threadIdx.x; pos0 < n; pos0 += (int64_t)K * stride) {
+      const uint32_t group = bit;
+      if (bit != 0x80000000u) bit <<= 1;
+      if (!(todo & group)) continue;
+      int p[K], i[K];
+      bool act[K];
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        if (act[k] && dcheck_bad(st, p[k], n, kChkJumpParent)) act[k] = false;
-        if (act[k]) {
-          const int pp = __ldcg(par + p[k]);
-          if (pp < 0) {
-            act[k] = false;
-            if (LABELS) p[k] = pp;  // the root's value
-          } else {
-            p[k] = pp;
-            par[pos0 + (int64_t)k * stride] = pp;
-          }
-        }
-        any |= act[k];
+        const int64_t pos = pos0 + (int64_t)k * stride;
+        p[k] = pos < n ? par[pos] : -1;
+        if (LABELS) i[k] = pos < n ? perm[pos] : -1;
+        act[k] = p[k] >= 0;
       }
-      if (!any) break;
-    }
+      for (int it = 0; it < limits.hops; ++it) {
+        bool any = false;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (act[k]) {  // still climbing after `iters` jumps
-        const int pp = __ldcg(par + p[k]);
-        if (pp >= 0)
-          unres = true;
-        else if (LABELS)
-          p[k] = pp;
+        for (int k = 0; k < K; ++k) {
+          if (act[k] && dcheck_bad(st, p[k], n, kChkJumpParent)) act[k] = false;
+          if (act[k]) {
+            const int pp = __ldcg(par + p[k]);
+            if (pp < 0) {
+              act[k] = false;
+              if (LABELS) p[k] = pp;  // the root's value
+            } else {
+              p[k] = pp;
+              par[pos0 + (int64_t)k * stride] = pp;
+            }
+          }
+          any |= act[k];
+        }
+        if (!any) break;
       }
-      if (LABELS && p[k] < 0 && i[k] >= 0) label[i[k]] = p[k] < -1 ? -2 - p[k] : -1;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        if (act[k]) {  // still climbing after the pass's jumps
+          const int pp = __ldcg(par + p[k]);
+          if (pp >= 0)
+            left |= group;
+          else if (LABELS)
+            p[k] = pp;
+        }
+        if (LABELS && p[k] < 0 && i[k] >= 0) label[i[k]] = p[k] < -1 ? -2 - p[k] : -1;
+      }
     }
+    todo = left;
   }
-  if (__any_sync(0xffffffffu, unres) && (threadIdx.x & 31) == 0) atomicAdd(&st->unresolved[round], 1u);
+  if (__any_sync(0xffffffffu, todo != 0) && (threadIdx.x & 31) == 0) atomicAdd(&st->unresolved[round], 1u);
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(&st->label_rounds, (uint32_t)round + 1);
 }
 
 // First round: the climb that ends most chains writes the labels as well.  Four chains per thread from
 // 2M points on, one below, where there are threads enough (label stage: 4M points 0.075 ms against
-// 0.091 with one; 1M points 0.056 ms with four, 0.048 with one).
+// 0.091 with one; 1M points 0.056 ms with four, 0.048 with one).  Eight blocks an SM, so that the grid of
+// label_blocks is resident: the 4096-event batch's label stage 0.200 -> 0.169 ms, 4M points 0.075 -> 0.071 (two
+// chains 0.194 and 0.073, three 0.177 and 0.071; five blocks of 40 registers 0.212 and 0.081).
 constexpr int kLabelChainPoints = 1 << 21;
 template <int K>
-__global__ void __launch_bounds__(256) k_labels(int32_t* par, const int32_t* __restrict__ perm,
-                                                int32_t* __restrict__ label, int n, int iters, int rounds,
+__global__ void __launch_bounds__(256, 8) k_labels(int32_t* par, const int32_t* __restrict__ perm,
+                                                int32_t* __restrict__ label, int n, JumpLimits limits, int rounds,
                                                 DevStatus* st) {
   if (blockIdx.x == 0 && threadIdx.x == 0) st->label_enqueued = (uint32_t)rounds;
-  jump<true, K>(par, perm, label, n, iters, st, 0);
+  jump<true, K>(par, perm, label, n, limits, st, 0);
 }
 
-__global__ void __launch_bounds__(256) k_jump(int32_t* par, int n, int iters, DevStatus* st, int round) {
+__global__ void __launch_bounds__(256, 8) k_jump(int32_t* par, int n, JumpLimits limits, DevStatus* st, int round) {
   if (st->unresolved[round - 1] == 0) return;
-  jump<false, 4>(par, nullptr, nullptr, n, iters, st, round);
+  jump<false, 4>(par, nullptr, nullptr, n, limits, st, round);
 }
 
 // All labels again, from parents that name roots, when the first round left a chain unresolved.
@@ -2813,10 +2829,18 @@ int launch_build(const KParams& kp, const InPtrs& in, Workspace& ws, bool two, i
 }  // namespace
 
 // Pointer-jumping rounds of a run whose caller does not read the status back (rounds past the first
-// do nothing unless the round before left a chain unresolved), and hops per round: events of a few
-// thousand points have chains of some hundred hops, and 64 hops sent every round over all of them.
+// do nothing unless the round before left a chain unresolved), and a round's passes.
 constexpr int kJumpLaunches = 4;
-constexpr int kJumpIters = 4096;
+constexpr JumpLimits kJumpLimits = {16, 256};
+inline JumpLimits jump_limits() {
+#if CLUE_DEVICE_CHECKS
+  // (the checked build can be told to leave chains to later rounds)
+  if (const char* v = getenv("CLUE_LABEL_HOPS")) return {std::max(1, atoi(v)), 1};
+#endif
+  return kJumpLimits;
+}
+// Blocks of the label climbs: no more than the GPU holds at once (see jump).
+inline int label_blocks(int n) { return std::min(grid_for(n, 256), 148 * 8); }
 
 template <int N>
 clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
@@ -2984,11 +3008,11 @@ clue_status run_pipeline(Workspace& ws, const RunArgs& a, cudaStream_t s) {
                                      l);
     launches += scan_launches(n) + kBfsLevels + 3;  // count, scan, fill, seeds, levels
   }
-  (n < kLabelChainPoints ? k_labels<1> : k_labels<4>)<<<grid_for(n, 256), 256, 0, s>>>(
-      ws.par, ws.perm, a.out.cluster_index, n, kJumpIters, a.blocking ? 1 : kJumpLaunches, ws.status);
+  (n < kLabelChainPoints ? k_labels<1> : k_labels<4>)<<<label_blocks(n), 256, 0, s>>>(
+      ws.par, ws.perm, a.out.cluster_index, n, jump_limits(), a.blocking ? 1 : kJumpLaunches, ws.status);
   if (!a.blocking) {
     for (int r = 1; r < kJumpLaunches; ++r)
-      k_jump<<<grid_for(n, 256), 256, 0, s>>>(ws.par, n, kJumpIters, ws.status, r);
+      k_jump<<<label_blocks(n), 256, 0, s>>>(ws.par, n, jump_limits(), ws.status, r);
     k_labels_again<<<grid_for(n, 256), 256, 0, s>>>(ws.par, ws.perm, a.out.cluster_index, n, kJumpLaunches, ws.status);
   }
   stage_mark(ws, 4, s);
@@ -3005,7 +3029,7 @@ clue_status finish_labels(Workspace& ws, const RunArgs& a, cudaStream_t s, int f
   const int n = a.kp.n;
   int r = first_round;
   for (uint32_t unres = 1; unres != 0 && r < 64; ++r) {
-    k_jump<<<grid_for(n, 256), 256, 0, s>>>(ws.par, n, kJumpIters, ws.status, r);
+    k_jump<<<label_blocks(n), 256, 0, s>>>(ws.par, n, jump_limits(), ws.status, r);
     ++ws.launches;
     CLUE_CUDA_TRY(cudaMemcpyAsync(&unres, &ws.status->unresolved[r], 4, cudaMemcpyDeviceToHost, s));
     CLUE_CUDA_TRY(cudaStreamSynchronize(s));

@@ -25,8 +25,8 @@
 // for the spatial sweeps.  A CTA processes a chunk of 128 home points of one tile (four warps
 // of 32).  The reference-order density reads whole candidate tiles and sums what lies within reach
 // of the warp's homes; the spatial sweeps take one 32-record Morton block at a time, skip blocks
-// whose bounding box is out of reach, and read the candidates from shared memory (nearest higher)
-// or from their owner lanes by shuffle (symmetric density).
+// whose bounding box is out of reach, and read the candidates from shared memory (nearest higher) or,
+// as neighbouring pairs, from a shared-memory copy by component (symmetric density).
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -1842,10 +1842,10 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
 // Blocks are 32 consecutive Morton-ordered records counted from their tile's start (so the
 // result does not depend on where a tile lies in a batch): block slot 4 c + w is warp w of
 // chunk c.  The warp of block A evaluates A against itself one-sidedly and every block B of its
-// tile after A and of the later tiles of its search-box union both ways: the candidate records
-// rotate through the lanes, each lane adding K(d) w_j to its own sum and K(d) w_i to the
-// travelling candidate's sum, which is then added in fixed point (exact integer adds, so the
-// order of arrival does not matter) to the candidate's accumulator.
+// tile after A and of the later tiles of its search-box union both ways: at step k lane l reads
+// candidate l ^ k from shared memory, adds K(d) w_j to its own sum and hands K(d) w_i to the
+// candidate's lane by shuffle; that lane's sum is then added in fixed point (exact integer adds, so
+// the order of arrival does not matter) to the candidate's accumulator.
 
 // Block boxes in compact order: block b of tile u is entry bo[u] + b (bo = exclusive scan of
 // the tiles' block counts).  One thread per (chunk, warp) slot; slots past a tile's end write
@@ -2064,8 +2064,9 @@ __global__ void __launch_bounds__(kTileThreads, (N <= 4 ? 8 : 4) * 128 / kTileTh
           const int cntB = min(32, pe - first);
           const bool cv = lane < cntB;
           // lane m owns candidate m of the block; at step k lane l meets candidate l ^ k and the
-          // candidate's owner collects the term from lane m ^ k = l (butterfly shuffles with
-          // immediate lane masks), so no value is carried from one step to the next
+          // candidate's owner collects the term from lane m ^ k = l (shuffles with immediate lane
+          // masks), so no value is carried from one step to the next; the candidates themselves are
+          // read from shared memory, two steps at a time (PairSmem)
           {
             float ox[N + 1];
             load_rec<N>(rec_m, first + (cv ? lane : 0), ox, ox[N]);
@@ -2288,7 +2289,7 @@ __device__ __forceinline__ int64_t seed_cap(const KParams& kp, const EvGrid* g) 
 // hides the scatter, seeds are ranked by a scan over one bit per point, and a point reads its parent
 // chain and its index and writes its label.  A pass for the seeds with a flag word per point, its
 // scan, four jump launches and an output pass over all arrays took 0.605 ms on the 4096-event batch
-// and 0.253 ms on 4M 3-D points; this takes 0.20 and 0.079 ms, and 0.10 ms and 0.02 ms more in the
+// and 0.253 ms on 4M 3-D points; this takes 0.17 and 0.071 ms, and 0.10 ms and 0.02 ms more in the
 // search.
 
 // Seeds before point i of the original order.

@@ -115,7 +115,7 @@ struct Workspace {
   size_t arena_bytes = 0;
 
   // event tables, one contiguous block: EvGrid[cap_events], ev_pt[cap_events + 1],
-  // ev_tile[cap_events + 1] (uploaded in one copy for batched calls)
+  // ev_tile[cap_events + 1] (uploaded in three copies for batched calls, see upload_events)
   EvGrid* ev = nullptr;
   int32_t* ev_pt = nullptr;
   int32_t* ev_tile = nullptr;

@@ -33,8 +33,8 @@ struct SilRec {
   static constexpr int kFloats = N <= 2 ? N : (N + 3) / 4 * 4;
 };
 
-// The clustered points in (cluster, index) order: coordinates as records, and every point's state
-// for k_silhouette (own mean -1: not set; smallest other mean FLT_MAX).
+// The clustered points in (cluster, index) order: coordinates as records, and every point's smallest
+// other mean, FLT_MAX before k_silhouette (which writes every point's own mean in exactly one run).
 template <int N>
 __global__ void __launch_bounds__(256) k_sil_gather(int n, const float* __restrict__ coords,
                                                     const int32_t* __restrict__ points, const CsrInfo* info,

@@ -161,7 +161,7 @@ void deliver(clue_server_s* S, Slot& s, clue_status st) {
   const int64_t P = s.points;
   if (st == CLUE_OK) {
     clue_run_info ri;
-    st = clue_context_read_info(s.ctx, s.stream, &ri);  // bounded-wait timeouts, non-finite input
+    st = clue_context_read_info(s.ctx, s.stream, &ri);  // unresolved label chains, non-finite input
   }
   for (size_t e = 0; e < s.reqs.size(); ++e) {
     Request* r = s.reqs[e];

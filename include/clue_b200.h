@@ -48,7 +48,8 @@ typedef enum clue_status {
   CLUE_ERR_INVALID_ARG = 1,    /* std::invalid_argument in the reference */
   CLUE_ERR_OUT_OF_MEMORY = 2,  /* device allocation failed */
   CLUE_ERR_CAPACITY = 3,       /* request larger than a fixed capacity */
-  CLUE_ERR_TIMEOUT = 4,        /* a bounded device wait gave up */
+  CLUE_ERR_TIMEOUT = 4,        /* label chains outlast the enqueued rounds (status reads of calls that
+                                  do not wait), or a request is not done in time (clue_server_wait) */
   CLUE_ERR_CUDA = 5,           /* CUDA runtime error (message holds the CUDA error string) */
   CLUE_ERR_NOT_SUPPORTED = 6,  /* option not available in this build */
   CLUE_ERR_NONFINITE = 7,      /* NaN or Inf in coordinates or weights */

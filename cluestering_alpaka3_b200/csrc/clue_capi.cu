@@ -930,7 +930,8 @@ clue_status clue_context_reserve_batch(clue_context ctx, int32_t ndim, int64_t n
 }
 
 size_t clue_context_workspace_bytes(clue_context ctx) {
-  if (!ctx || ctx->ws.ask_n == 0) return 0;  // (an idle context's buffers before its owner's first call)
+  // (an idle context's buffers are not its next owner's before a call)
+  if (!ctx || (ctx->ws.reused && ctx->ws.ask_n == 0)) return 0;
   return ctx->ws.arena_bytes + ctx->ws.dstage_bytes + ctx->ws.post_bytes;
 }
 
